@@ -29,21 +29,41 @@ constexpr int cls_X()
 constexpr int kX = cls_X();
 constexpr int kY = QCG_CLASS - kX * (kX + 1) / 2;
 
-// Warps per CTA, every warp a consumer of its own ket component per pass.  At most 8: the SM's registers are
-// split among its four schedulers, and 8 warps (two per scheduler) leave each thread up to 255 registers,
-// which the (dd|dd) steps need without spilling (a ninth warp caps every thread at 168).  Each component
-// has its own straight-line ket code, and the code of the components in flight must fit the instruction
-// cache.  Measured on a B200: on (dd|dd) 8 warps on 8 components ran at half the speed of 4 (and 3.4x slower
-// than 8 warps sharing one component's code), 2 warps were slower than 4, and 4 warps also beat 8 on (dd|dp),
-// (dd|pp) and (dp|dp), whose largest components have 220-570 instructions.  So: 8 warps where the largest
-// component has at most kSmallKet instructions, else 4.
-constexpr int kSmallKet = 150;
+// Pieces of ket code per pass (kNG; each runs on three warps, one per rotation).  A thread keeps Y_f and acc_f
+// in registers, and the SM's 65 536 registers are split among four schedulers, so ceil(3 g / 4) warps per
+// scheduler leave each thread 512 / ceil(3 g / 4) registers (255 at most): g is the largest for which Y_f, acc_f
+// and kTemps further registers fit, and the pieces are then spread evenly over the passes.
+constexpr int kTemps = 36;
 
-constexpr int team_warps(int nf, int ket_instr)
+constexpr int warp_regs(int g)
 {
-    const int maxw = ket_instr <= kSmallKet ? 8 : 4;
-    const int npass = (nf + maxw - 1) / maxw;
-    return (nf + npass - 1) / npass;
+    const int per = (3 * g + 3) / 4, r = 512 / per / 8 * 8;
+    return r > 255 ? 255 : r;
+}
+constexpr int team_pieces(int ncode, int nh, int ne)
+{
+    int g = 1;
+    for (int x = 2; x <= 8 && x <= ncode; ++x)
+        if (warp_regs(x) >= 2 * (nh + ne) + kTemps) g = x;
+    const int npass = (ncode + g - 1) / g;
+    return (ncode + npass - 1) / npass;
+}
+// Doubles of the stage space: three stages, and at least 18 primitive pairs (contractions of three).
+constexpr int team_stage_space(int stage)
+{
+    const int pairs = 18 * kTeamPairDoubles;
+    return (3 * stage > pairs ? 3 * stage : pairs) * 32;
+}
+constexpr size_t team_smem(int stage)
+{
+    return (size_t)(team_stage_space(stage) + kBoysRows * kBoysColumns) * sizeof(double);
+}
+// CTAs per SM to compile for: about twelve warps, as far as their shared memory fits
+constexpr int team_min_blocks(int ng, int stage)
+{
+    const int fit = (int)((227 * 1024) / (team_smem(stage) + 1024)), want = 12 / (3 * ng);
+    const int m = fit < want ? fit : want;
+    return m < 1 ? 1 : m;
 }
 
 struct Cls
@@ -51,23 +71,30 @@ struct Cls
     static constexpr int LA = kPairLA[kX], LB = kPairLB[kX], LC = kPairLA[kY], LD = kPairLB[kY];
     static constexpr int kNF = gen::QCG_CAT(kTeamNF, QCG_CLASS), kNE = gen::QCG_CAT(kTeamNE, QCG_CLASS);
     static constexpr int kNH = gen::QCG_CAT(kTeamNH, QCG_CLASS), kStage = gen::QCG_CAT(kTeamStage, QCG_CLASS);
-#ifdef QCG_TEAM_NW
-    static constexpr int kNW = QCG_TEAM_NW;
-#else
-    static constexpr int kNW = team_warps(kNF, gen::QCG_CAT(kTeamKetInstr, QCG_CLASS));
-#endif
-    static __device__ __forceinline__ void produce(double* st, const PrimPairData& ab, const PrimPairData& cd,
-                                                   const double* __restrict__ bt, bool bra_e)
+    static constexpr int kNCode = gen::QCG_CAT(kTeamNCode, QCG_CLASS);
+    static constexpr int kKetStage = gen::QCG_CAT(kTeamKetStage, QCG_CLASS);
+    static constexpr int kNG = team_pieces(kNCode, kNH, kNE), kNW = 3 * kNG;
+    static constexpr int kMinBlocks = team_min_blocks(kNG, kStage);
+    using View = gen::QCG_CAT(TeamView, QCG_CLASS)<double>;
+    static __device__ __forceinline__ constexpr int fslot(int jc) { return gen::QCG_CAT(team_fslot_, QCG_CLASS)(jc); }
+    static __device__ __forceinline__ constexpr bool fixed(int jc) { return gen::QCG_CAT(team_ffixed_, QCG_CLASS)(jc); }
+    static constexpr int kStageSpace = team_stage_space(kStage), kPairSlots = kStageSpace / (32 * kTeamPairDoubles);
+    static __device__ __forceinline__ void produce(double* st, const TeamPair& ab, const TeamPair& cd,
+                                                   const BoysColumns& bt, bool bra_e)
     {
         gen::QCG_CAT(team_produce_, QCG_CLASS)<double>(st, ab, cd, bt, bra_e);
     }
-    static __device__ __forceinline__ void ket(int jf, const double* st, double (&Y)[kNH])
+    static __device__ __forceinline__ void ket(int jc, const View& v, double (&Y)[kNH])
     {
-        gen::QCG_CAT(team_ket_, QCG_CLASS)<double>(jf, st, Y);
+        gen::QCG_CAT(team_ket_piece_, QCG_CLASS)<double>(jc, v, Y);
     }
-    static __device__ __forceinline__ void bra(const double* st, const double (&Y)[kNH], double (&acc)[kNE])
+    static __device__ __forceinline__ void bra(const View& v, const double (&Y)[kNH], double (&acc)[kNE])
     {
-        gen::QCG_CAT(team_bra_, QCG_CLASS)<double>(st, Y, acc);
+        gen::QCG_CAT(team_bra_view_, QCG_CLASS)<double>(v, Y, acc);
+    }
+    static __device__ __forceinline__ void store(const double (&acc)[kNE], double* hA, int rot)
+    {
+        gen::QCG_CAT(team_store_, QCG_CLASS)<double>(acc, hA, rot);
     }
     static __device__ __forceinline__ void hrr_ket(const double* p, double* y, double CDx, double CDy, double CDz)
     {
@@ -82,7 +109,7 @@ struct Cls
 
 constexpr int kThreads = Cls::kNW * 32;
 constexpr int kNCD = ncart(Cls::LC) * ncart(Cls::LD);
-constexpr size_t kSmem = 3 * (size_t)Cls::kStage * 32 * sizeof(double);   // three stages
+constexpr size_t kSmem = team_smem(Cls::kStage);   // the stages and the Boys columns
 std::atomic<unsigned long long> g_smem_ready{0};
 }   // namespace
 

@@ -12,15 +12,16 @@
 //     consumers to halve the stage (1.4x slower on (dd|dd): the contraction is bound by instruction issue),
 //     and walking the group one bra primitive pair at a time so that the cache stays in L2 (1.3x slower: a
 //     barrier, a pipeline restart and an accumulator save per window cost more than the HBM traffic saved).
-//  2. Contraction.  Warp w owns one component f of the ket range of the horizontal-recurrence form (f over
-//     L = LC..LC+LD on centre C) per pass; each component has its own straight-line ket code, and the warp
-//     count is sized so that the code of the components in flight fits the SM's instruction cache.  It keeps in registers Y_f -- the ket step summed over the ket
-//     primitives of the current bra primitive pair -- and acc_f = [e0|f] for every e, adding the bra step
-//     of Y_f to acc_f after the bra pair's last ket primitive (team_ket_<k>, team_bra_<k>).  The stages
-//     stream from the R cache into shared memory, three deep, by bulk copies (cp.async.bulk, the Tensor
-//     Memory Accelerator's untiled form) that one thread issues on an mbarrier; one barrier per primitive
-//     quartet.  With more ket components than warps the group is walked in passes, each pass reading the
-//     stages again (from L2 or HBM) instead of recomputing them.
+//  2. Contraction.  A warp works on one component f of the ket range of the horizontal-recurrence form (f over
+//     L = LC..LC+LD on centre C) per pass.  Components that are cyclic rotations of one another run the same
+//     code in rotated frames (gen_md.py, team form): warp 3 g + r takes piece pass * kNG + g of the ket code in
+//     rotation r, so the three warps of a piece walk one instruction stream over one stage.  It keeps in
+//     registers Y_f -- the ket step summed over the ket primitives of the current bra primitive pair -- and
+//     acc_f = [e0|f] for every e, adding the bra step of Y_f to acc_f after the bra pair's last ket primitive
+//     (team_ket_piece_<k>, team_bra_view_<k>).  The stages stream from the R cache into shared memory, three
+//     deep, by bulk copies (cp.async.bulk, the Tensor Memory Accelerator's untiled form) that one warp issues
+//     on an mbarrier, without a gap between passes; one barrier per primitive quartet.  With more pieces than
+//     a pass holds, each pass reads the stages again (from L2 or HBM) instead of recomputing them.
 //  3. Recurrences.  acc_f goes to the CTA's scratch as [e0|f0] (lane-minor, so every access of a warp is
 //     one coalesced line); the ket recurrence per e row gives [e0|cd] there, and the bra recurrence per
 //     (c d) column writes (ab|cd) into the quartet's output block (generated team_hrr_ket_<k>,
@@ -40,16 +41,157 @@ namespace qcg {
 
 extern __shared__ __align__(128) double qcg_team_smem[];
 
+// Shared memory of both kernels: three stages, whose space holds the group's primitive pairs while the stage
+// tables are made (slot t of lane l: entry k at [(t * kTeamPairDoubles + k) * 32 + l]), then the Boys columns.
 template <class Cls>
-__global__ void __launch_bounds__(Cls::kNW * 32, 1)
+__device__ __forceinline__ BoysColumns team_boys(const double* __restrict__ table)
+{
+    double* const s = qcg_team_smem + Cls::kStageSpace;
+    for (int i = threadIdx.x; i < kBoysRows * kBoysColumns; i += blockDim.x)
+    {
+        const int k = i / kBoysRows, it = i - k * kBoysRows;
+        const double f[kBoysColumns] = {1.0, 1.0, 0.5, 1.0 / 6.0, 1.0 / 24.0, 1.0 / 120.0, 1.0 / 720.0};
+        double c = f[0];
+#pragma unroll
+        for (int j = 1; j < kBoysColumns; ++j) c = k == j ? f[j] : c;
+        s[i] = table[it * 23 + Cls::LA + Cls::LB + Cls::LC + Cls::LD + k] * c;
+    }
+    return BoysColumns{s};
+}
+__device__ __forceinline__ void team_pair_store(int t, int lane, const TeamPair& d)
+{
+    double* const s = qcg_team_smem + t * kTeamPairDoubles * 32 + lane;
+    s[0] = d.p; s[32] = d.Px; s[64] = d.Py; s[96] = d.Pz;
+    s[128] = d.PAx; s[160] = d.PAy; s[192] = d.PAz; s[224] = d.kp; s[256] = d.h;
+}
+__device__ __forceinline__ TeamPair team_pair_load(int t, int lane)
+{
+    const double* const s = qcg_team_smem + t * kTeamPairDoubles * 32 + lane;
+    return TeamPair{s[0], s[32], s[64], s[96], s[128], s[160], s[192], s[224], s[256]};
+}
+
+// Phase 1 of both kernels: the stage tables of the group's primitive quartets into rc.  bra(i) and ket(i) give
+// this lane's primitive pairs; each is formed once, by the warps in turn, and read back from shared memory by the
+// stages that use it (a contraction too long for that space forms them stage by stage).
+template <class Cls, class Bra, class Ket>
+__device__ __forceinline__ void team_stages(double* __restrict__ rc, const int Kab, const int Kcd, const int Kg,
+                                            const BoysColumns& bt, Bra bra, Ket ket)
+{
+    constexpr int NW = Cls::kNW, STAGE = Cls::kStage * 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int K = Kab * Kcd;
+    const int npair = __reduce_max_sync(0xffffffffu, Kab + Kcd);
+    const bool kept = npair <= Cls::kPairSlots;   // CTA-uniform: every warp sees the same lanes
+    if (kept)
+        for (int t = warp; t < npair; t += NW)
+        {
+            if (t < Kab) team_pair_store(t, lane, team_pair(bra(t)));
+            else if (t < Kab + Kcd) team_pair_store(t, lane, team_pair(ket(t - Kab)));
+        }
+    __syncthreads();
+    for (int x = warp; x < Kg; x += NW)
+        if (x < K)
+        {
+            const int ij = x / Kcd, kl = x - ij * Kcd;
+            const TeamPair ab = kept ? team_pair_load(ij, lane) : team_pair(bra(ij));
+            const TeamPair cd = kept ? team_pair_load(Kab + kl, lane) : team_pair(ket(kl));
+            Cls::produce(rc + (long long)x * STAGE + lane, ab, cd, bt, kl == Kcd - 1);
+        }
+    team::fence_async();   // the stages (global) and the pairs (shared) before the copies into the stage space
+    __syncthreads();
+}
+
+// Phase 2 of both kernels: [e0|f0] of the group (lane-minor, rows and columns in slot order) from the Kg stages
+// in rc; K and Kcd are this lane's primitive-quartet and ket-pair counts (0 for an absent quartet), G the
+// number of steps streamed so far.  False, CTA-uniform, when a bulk copy did not arrive.
+template <class Cls>
+__device__ __forceinline__ bool team_contract(const double* __restrict__ rc, double* __restrict__ hA, const int K,
+                                              const int Kcd, const int Kg, unsigned long long& G, uint64_t* full,
+                                              int* err)
+{
+    constexpr int NG = Cls::kNG, NF = Cls::kNF, NE = Cls::kNE, NH = Cls::kNH, NC = Cls::kNCode;
+    constexpr int NPASS = (NC + NG - 1) / NG;
+    constexpr int STAGE = Cls::kStage * 32;        // doubles per stage (entry-major, lane-minor)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int piece = warp / 3, rot = warp - 3 * piece;
+    const bool leader = threadIdx.x == 0;
+    const int nsteps = NPASS * Kg;
+    // step t = pass * Kg + x reads stage x; warp 0 issues its copy, without the bra tables when no lane needs them
+    int ix = 0, ikl = 0;   // the next issued step's stage and its ket primitive in this lane
+    auto issue = [&](int t) {
+        const bool bra = __any_sync(0xffffffffu, ix < K && ikl == Kcd - 1);
+        if (leader)
+        {
+            const unsigned long long gs = G + t;
+            team::bulk_load(qcg_team_smem + (gs % 3) * STAGE, rc + (long long)ix * STAGE,
+                            (bra ? Cls::kStage : Cls::kKetStage) * 32 * (uint32_t)sizeof(double), &full[gs % 3]);
+        }
+        ikl = ikl == Kcd - 1 ? 0 : ikl + 1;
+        if (++ix == Kg) ix = ikl = 0;
+    };
+    if (warp == 0)
+    {
+        issue(0);
+        if (nsteps > 1) issue(1);
+    }
+    int t = 0;
+    for (int pass = 0; pass < NPASS; ++pass)
+    {
+        const int jc = pass * NG + piece;
+        const bool on = jc < NC && !(rot != 0 && Cls::fixed(jc));
+        double Y[NH], acc[NE];
+#pragma unroll
+        for (int h = 0; h < NH; ++h) Y[h] = 0.0;
+#pragma unroll
+        for (int e = 0; e < NE; ++e) acc[e] = 0.0;
+        int kl = 0;
+        for (int x = 0; x < Kg; ++x, ++t)
+        {
+            const unsigned long long gs = G + t;
+            bool late = false;
+            if (leader) late = !team::mbar_wait(&full[gs % 3], (uint32_t)((gs / 3) & 1));
+            // stage x is in shared memory; every warp has left the step before
+            if (__syncthreads_or(late))
+            {
+                // a copy did not arrive: let the ones in flight land and record it
+                if (leader)
+                {
+                    team::drain(full, G, t, nsteps);
+                    atomicOr(err, 1);
+                }
+                return false;
+            }
+            if (warp == 0 && t + 2 < nsteps) issue(t + 2);   // into the stage the step before used
+            if (on && x < K)
+            {
+                const typename Cls::View v(qcg_team_smem + (gs % 3) * STAGE + lane, rot);
+                Cls::ket(jc, v, Y);
+                if (kl == Kcd - 1)
+                {
+                    Cls::bra(v, Y, acc);
+#pragma unroll
+                    for (int h = 0; h < NH; ++h) Y[h] = 0.0;
+                    kl = 0;
+                }
+                else
+                    ++kl;
+            }
+        }
+        if (on) Cls::store(acc, hA + (Cls::fslot(jc) + rot) * 32 + lane, rot);
+    }
+    G += nsteps;
+    __syncthreads();   // the stages are no longer read; [e0|f0] is written
+    return true;
+}
+
+template <class Cls>
+__global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     eri_batch_team_kernel(BasisDev bs, const int4* __restrict__ quartets, const int* __restrict__ order, long long nq,
                           double* __restrict__ out, const double* __restrict__ boys_table, TeamScratchDev scr)
 {
-    constexpr int NW = Cls::kNW;                   // warps; warp w owns ket component pass * NW + w
-    constexpr int NF = Cls::kNF, NE = Cls::kNE, NH = Cls::kNH;
-    constexpr int NPASS = (NF + NW - 1) / NW;
+    constexpr int NW = Cls::kNW;
+    constexpr int NF = Cls::kNF, NE = Cls::kNE;
     constexpr int STAGE = Cls::kStage * 32;        // doubles per stage (entry-major, lane-minor)
-    constexpr uint32_t STAGE_BYTES = STAGE * sizeof(double);
     constexpr int NCD = ncart(Cls::LC) * ncart(Cls::LD);
     constexpr long long BLK = (long long)ncart(Cls::LA) * ncart(Cls::LB) * NCD;
     static_assert(NE <= ncart(Cls::LA) * ncart(Cls::LB) && NF <= NCD, "[e0|f0] fits the output block");
@@ -61,6 +203,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, 1)
         for (int s = 0; s < 3; ++s) team::mbar_init(&full[s]);
         team::mbar_init_fence();
     }
+    const BoysColumns bt = team_boys<Cls>(boys_table);
     __syncthreads();
     double* const rc = scr.rcache + (long long)blockIdx.x * scr.kmax * STAGE;   // this CTA's stage slots
     double* const hA = scr.hrr + (long long)blockIdx.x * (NE * NF + NE * NCD) * 32;
@@ -90,76 +233,11 @@ __global__ void __launch_bounds__(Cls::kNW * 32, 1)
             continue;
         }
         // 1. stage tables of every primitive quartet, written once to the R cache
-        for (int x = warp; x < Kg; x += NW)
-            if (x < K)
-            {
-                const int ij = x / Kcd, kl = x - ij * Kcd;
-                const PrimPairData ab = shell_prim_pair(bs, s.x, ij / nj, s.y, ij % nj);
-                const PrimPairData cd = shell_prim_pair(bs, s.z, kl / nl, s.w, kl % nl);
-                Cls::produce(rc + (long long)x * STAGE + lane, ab, cd, boys_table, kl == Kcd - 1);
-            }
-        team::fence_async_global();
-        __syncthreads();
+        team_stages<Cls>(
+            rc, ni * nj, Kcd, Kg, bt, [&](int ij) { return shell_prim_pair(bs, s.x, ij / nj, s.y, ij % nj); },
+            [&](int kl) { return shell_prim_pair(bs, s.z, kl / nl, s.w, kl % nl); });
         // 2. contraction, the stages streamed back through shared memory three deep
-        for (int pass = 0; pass < NPASS; ++pass)
-        {
-            const int jf = pass * NW + warp;
-            auto issue = [&](int x) {
-                const unsigned long long gs = G + x;
-                team::bulk_load(qcg_team_smem + (gs % 3) * STAGE, rc + (long long)x * STAGE, STAGE_BYTES,
-                                &full[gs % 3]);
-            };
-            if (leader)
-            {
-                issue(0);
-                if (Kg > 1) issue(1);
-            }
-            double Y[NH], acc[NE];
-#pragma unroll
-            for (int h = 0; h < NH; ++h) Y[h] = 0.0;
-#pragma unroll
-            for (int e = 0; e < NE; ++e) acc[e] = 0.0;
-            int kl = 0;
-            for (int i = 0; i < Kg; ++i)
-            {
-                const unsigned long long gs = G + i;
-                bool late = false;
-                if (leader) late = !team::mbar_wait(&full[gs % 3], (uint32_t)((gs / 3) & 1));
-                // stage i is in shared memory; every warp has left step i - 1
-                if (__syncthreads_or(late))
-                {
-                    // a copy did not arrive: let the ones in flight land, record it and end the CTA
-                    if (leader)
-                    {
-                        team::drain(full, G, i, Kg);
-                        atomicOr(scr.err, 1);
-                    }
-                    return;
-                }
-                if (leader && i + 2 < Kg) issue(i + 2);   // into the stage step i - 1 used
-                if (jf < NF && i < K)
-                {
-                    const double* st = qcg_team_smem + (gs % 3) * STAGE + lane;
-                    Cls::ket(jf, st, Y);
-                    if (kl == Kcd - 1)
-                    {
-                        Cls::bra(st, Y, acc);
-#pragma unroll
-                        for (int h = 0; h < NH; ++h) Y[h] = 0.0;
-                        kl = 0;
-                    }
-                    else
-                        ++kl;
-                }
-            }
-            G += Kg;
-            if (jf < NF)
-            {
-#pragma unroll
-                for (int e = 0; e < NE; ++e) hA[(e * NF + jf) * 32 + lane] = acc[e];
-            }
-            __syncthreads();   // the pass's stages are no longer read; its [e0|f] columns are written
-        }
+        if (!team_contract<Cls>(rc, hA, K, Kcd, Kg, G, full, scr.err)) return;
         // 3. recurrences: ket per e row into [e0|cd], bra per (c d) column into the output block
         const double* A = bs.cen + 3 * s.x;
         const double* B = bs.cen + 3 * s.y;
@@ -193,16 +271,14 @@ __global__ void __launch_bounds__(Cls::kNW * 32, 1)
 // Internal/Imp/ERI4.C:10-17) without storing the integrals.
 // ------------------------------------------------------------------------------------------------
 template <class Cls, bool DET>
-__global__ void __launch_bounds__(Cls::kNW * 32, 1)
+__global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     jk_team_kernel(JKWorkDev w, PairListDev bra, PairListDev ket, PrimPairsDev P, const int* __restrict__ shell_f0,
                    const double* __restrict__ D, double* __restrict__ J, double* __restrict__ K, int n,
                    const double* __restrict__ boys_table, TeamScratchDev scr)
 {
     constexpr int NW = Cls::kNW;
-    constexpr int NF = Cls::kNF, NE = Cls::kNE, NH = Cls::kNH;
-    constexpr int NPASS = (NF + NW - 1) / NW;
+    constexpr int NF = Cls::kNF, NE = Cls::kNE;
     constexpr int STAGE = Cls::kStage * 32;
-    constexpr uint32_t STAGE_BYTES = STAGE * sizeof(double);
     constexpr int NB = ncart(Cls::LB), ND = ncart(Cls::LD);
     constexpr int NAB = ncart(Cls::LA) * NB, NCD = ncart(Cls::LC) * ND;
     static_assert(NE <= NAB && NF <= NCD, "[e0|f0] fits the blocks");
@@ -214,6 +290,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, 1)
         for (int s = 0; s < 3; ++s) team::mbar_init(&full[s]);
         team::mbar_init_fence();
     }
+    const BoysColumns bt = team_boys<Cls>(boys_table);
     __syncthreads();
     double* const rc = scr.rcache + (long long)blockIdx.x * scr.kmax * STAGE;
     double* const hA = scr.hrr + (long long)blockIdx.x * (NE * NF + NE * NCD + NAB * NCD) * 32;
@@ -253,74 +330,11 @@ __global__ void __launch_bounds__(Cls::kNW * 32, 1)
             continue;
         }
         // 1. stage tables, from the primitive-pair table
-        for (int x = warp; x < Kg; x += NW)
-            if (x < Kq)
-            {
-                const int ij = x / Kcd, kl = x - ij * Kcd;
-                const PrimPairData ab = load_pp(P, bra.ppo[i] + ij);
-                const PrimPairData cd = load_pp(P, ket.ppo[j] + kl);
-                Cls::produce(rc + (long long)x * STAGE + lane, ab, cd, boys_table, kl == Kcd - 1);
-            }
-        team::fence_async_global();
-        __syncthreads();
+        team_stages<Cls>(
+            rc, Kab, Kcd, Kg, bt, [&](int ij) { return load_pp(P, bra.ppo[i] + ij); },
+            [&](int kl) { return load_pp(P, ket.ppo[j] + kl); });
         // 2. contraction (as in eri_batch_team_kernel)
-        for (int pass = 0; pass < NPASS; ++pass)
-        {
-            const int jf = pass * NW + warp;
-            auto issue = [&](int x) {
-                const unsigned long long gs = G + x;
-                team::bulk_load(qcg_team_smem + (gs % 3) * STAGE, rc + (long long)x * STAGE, STAGE_BYTES,
-                                &full[gs % 3]);
-            };
-            if (leader)
-            {
-                issue(0);
-                if (Kg > 1) issue(1);
-            }
-            double Y[NH], acc[NE];
-#pragma unroll
-            for (int h = 0; h < NH; ++h) Y[h] = 0.0;
-#pragma unroll
-            for (int e = 0; e < NE; ++e) acc[e] = 0.0;
-            int kl = 0;
-            for (int x = 0; x < Kg; ++x)
-            {
-                const unsigned long long gs = G + x;
-                bool late = false;
-                if (leader) late = !team::mbar_wait(&full[gs % 3], (uint32_t)((gs / 3) & 1));
-                if (__syncthreads_or(late))
-                {
-                    if (leader)
-                    {
-                        team::drain(full, G, x, Kg);
-                        atomicOr(scr.err, 1);
-                    }
-                    return;
-                }
-                if (leader && x + 2 < Kg) issue(x + 2);
-                if (jf < NF && x < Kq)
-                {
-                    const double* st = qcg_team_smem + (gs % 3) * STAGE + lane;
-                    Cls::ket(jf, st, Y);
-                    if (kl == Kcd - 1)
-                    {
-                        Cls::bra(st, Y, acc);
-#pragma unroll
-                        for (int h = 0; h < NH; ++h) Y[h] = 0.0;
-                        kl = 0;
-                    }
-                    else
-                        ++kl;
-                }
-            }
-            G += Kg;
-            if (jf < NF)
-            {
-#pragma unroll
-                for (int e = 0; e < NE; ++e) hA[(e * NF + jf) * 32 + lane] = acc[e];
-            }
-            __syncthreads();
-        }
+        if (!team_contract<Cls>(rc, hA, Kq, Kcd, Kg, G, full, scr.err)) return;
         // 3. recurrences into the scratch: [e0|cd] in hB, (ab|cd) in hC (lane-minor)
         // C - D = (P - D) - (P - C) and A - B = (P - B) - (P - A), from the shell pairs' first primitive pairs
         if (valid)

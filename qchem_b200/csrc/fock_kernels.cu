@@ -94,21 +94,20 @@ __global__ void pattern_key_kernel(BasisDev bs, const int4* __restrict__ quartet
         if (h[i]) atomicAdd(&hist[i], h[i]);
 }
 
-// exclusive scan of the 256 bucket counts (one block of 256 threads)
+// First position of every bucket (one block of 256 threads).  Buckets go by decreasing primitive-quartet count:
+// the batch kernels hand out groups of neighbouring quartets round robin, so the long primitive loops start
+// first and the short ones fill the last wave.
 __global__ void pattern_scan_kernel(const int* __restrict__ hist, int* __restrict__ cursor)
 {
-    __shared__ int v[256];
+    __shared__ int n[256], w[256];
     const int t = threadIdx.x;
-    v[t] = hist[t];
+    n[t] = hist[t];
+    w[t] = ((t >> 6) + 1) * (((t >> 4) & 3) + 1) * (((t >> 2) & 3) + 1) * ((t & 3) + 1);
     __syncthreads();
-    for (int off = 1; off < 256; off <<= 1)
-    {
-        const int x = t >= off ? v[t - off] : 0;
-        __syncthreads();
-        v[t] += x;
-        __syncthreads();
-    }
-    cursor[t] = v[t] - hist[t];
+    int before = 0;
+    for (int u = 0; u < 256; ++u)
+        if (w[u] > w[t] || (w[u] == w[t] && u < t)) before += n[u];
+    cursor[t] = before;
 }
 
 __global__ void pattern_scatter_kernel(const unsigned char* __restrict__ key, long long nq, int* __restrict__ cursor,

@@ -121,8 +121,9 @@ def e_names(prefix, la, lb):
 
 def r_prologue(L, rsm, w):
     HL = nherm(L)
-    w("    const double p = ab.p, q = cd.p, pq = p + q;")
-    w("    const double alpha = p * q / pq;")
+    # one division (1 / (p q (p + q))) serves alpha, lambda, 1/(2p) and 1/(2q)
+    w("    const double p = ab.p, q = cd.p, pq = p * q, s = p + q, inv = 1.0 / (pq * s);")
+    w("    const double alpha = pq * (pq * inv);")
     w("    const double Xd = ab.Px - cd.Px, Yd = ab.Py - cd.Py, Zd = ab.Pz - cd.Pz;")
     w(f"    RT F[{L + 1}];")
     w(f"    boys<{L}>(alpha * (Xd * Xd + Yd * Yd + Zd * Zd), bt, F);")
@@ -157,8 +158,8 @@ def r_prologue(L, rsm, w):
                             e += f" + RT({v - 1}) * RR({hidx(L, 0, 0, v - 2)})"
                     w(f"    RR({hidx(L, t, u, v)}) = {e};")
         w(f"    RR(0) = pwn[{n}] * F[{n}];")
-    w("    const RT lambda = RT(34.986836655249725693 / (p * q * sqrt(pq)) * ab.K * cd.K);")
-    w("    const RT a12b = RT(0.5 / ab.p), a12k = RT(0.5 / cd.p);")
+    w("    const RT lambda = RT(34.986836655249725693 * inv * sqrt(s) * ab.K * cd.K);")
+    w("    const RT a12b = RT(0.5 * (q * s) * inv), a12k = RT(0.5 * (p * s) * inv);")
 
 
 def ket_blocks(LA, LB, LC, LD, cds, w):
@@ -497,18 +498,66 @@ def main_hrr(outdir):
 
 
 # ------------------------------------------------------------------------------------------------------
-# Team form (main_team): the code of the warp-specialised ERI-batch kernel (eri_team.cuh).  A CTA holds 32
-# contracted quartets, one per lane.  Per primitive quartet a producer warp writes a shared-memory stage
-# per lane: R^0_{tuv} scaled by the prefactor lambda, and the single-centre Hermite tables E^{i0}_t of the
-# ket pair (and, after the last ket primitive of a bra primitive pair, of the bra pair).  Consumer warp w
-# owns one ket component f of the HRR form ([e0|f0], f over L = LC..LC+LD on centre C) and keeps in
-# registers
+# Team form (main_team): the code of the ERI-batch kernel that shares a quartet's work among warps
+# (eri_team.cuh).  A CTA holds 32 contracted quartets, one per lane.  Per primitive quartet a stage holds, per
+# lane, R^0_{tuv} scaled by the prefactor lambda, and the single-centre Hermite tables E^{i0}_t of the ket
+# pair (and, at the last ket primitive of a bra primitive pair, of the bra pair).  A warp works on one
+# component f of the HRR form's ket range ([e0|f0], f over L = LC..LC+LD on centre C) and keeps in registers
 #     Y_f[h] = sum over the ket primitives of sum_{h' in supp(f)} (-1)^{|h'|} E^{f0}_{h'} R_{h+h'}
 # for h over the bra's Hermite indices, and, once per bra primitive pair, adds
 #     acc_f[e] += sum_t E^{ex 0}_t sum_u E^{ey 0}_u sum_v E^{ez 0}_v Y_f[tuv]
 # so the bra contraction runs once per bra primitive pair instead of once per primitive quartet.  The
 # ket and bra horizontal recurrences of the HRR form then give (ab|cd).  All indices are literals.
+#
+# Components that are cyclic rotations of one another (x -> y -> z -> x) share ONE piece of code, run in a
+# frame whose axis a is the molecule's axis (a + r) % 3.  Nothing is computed for it: entries indexed by an
+# axis triple are stored orbit by orbit (the three rotations of a triple in consecutive slots 3k, 3k + 1,
+# 3k + 2, the fixed triples (n, n, n) after them), so member j of orbit k in the frame is slot
+# 3k + (j + r) % 3, and three base pointers (one per j) make every access of the rotated code the same
+# literal offset from one of them.  The 1-D Hermite tables are stored axis by axis and get three pointers the
+# same way.  (dd|dd) then has 11 pieces of ket code instead of 31, three warps run each of them side by side
+# on the same stage, and the code in flight per warp is a third.
 # ------------------------------------------------------------------------------------------------------
+def rotated(c, r):
+    """the frame triple c seen from the molecule: its axis a is the molecule's axis (a + r) % 3"""
+    return tuple(c[(a - r) % 3] for a in range(3))
+
+
+def orbits(items, weight=lambda c: 0):
+    """The items (a set closed under rotation) as orbits under rotation, heaviest first, then the fixed
+    triples: (representatives of the three-fold orbits, fixed triples)."""
+    reps, fixed, seen = [], [], set()
+    for c in items:
+        if c in seen:
+            continue
+        if c[0] == c[1] == c[2]:
+            fixed.append(c)
+        else:
+            reps.append(c)
+        seen.update(rotated(c, r) for r in range(3))
+    reps.sort(key=lambda c: -weight(c))
+    return reps, fixed
+
+
+def orbit_order(items, weight=lambda c: 0):
+    """items in slot order"""
+    reps, fixed = orbits(items, weight)
+    return [rotated(c, r) for c in reps for r in range(3)] + fixed
+
+
+def orbit_member(order, c):
+    """(slot of its orbit's first member, member number) of triple c; (slot, None) for a fixed triple"""
+    k = order.index(c)
+    return (k, None) if c[0] == c[1] == c[2] else (k - k % 3, k % 3)
+
+
+def ket_weight(LAB, f):
+    """instructions of the ket step of component f, estimated (loads, products, fused multiply-adds)"""
+    supp = [(a, b, c) for a in range(f[0] + 1) for b in range(f[1] + 1) for c in range(f[2] + 1)]
+    loads = set((h[0] + a, h[1] + b, h[2] + c) for h in herm_list(LAB) for (a, b, c) in supp)
+    return nherm(LAB) * len(supp) + len(loads) + 2 * len(supp) + sum(f) + 3
+
+
 def ne1(Lmax):
     """stored 1-D entries E^{i0}_t, 1 <= i <= Lmax, t <= i (E^{00}_0 = 1 is not stored)"""
     return (Lmax + 1) * (Lmax + 2) // 2 - 1
@@ -519,18 +568,19 @@ def e1_slot(i, t):
 
 
 def r_stream(L, w, store):
-    """Boys -> R^0_{tuv} for t+u+v <= L, each stored once through store(H, name) as soon as it exists.
+    """Boys -> R^0_{tuv} for t+u+v <= L, each stored once through store((t, u, v), name) as soon as it exists.
     Same recursion and branch order as r_prologue (x first, then y, then z), evaluated column by column
     (v, then u, then t) so that only the columns the next ones need stay live; lambda is folded into
     R^n_{000}, so every R value carries it."""
-    w("    const double p = ab.p, q = cd.p, pq = p + q;")
-    w("    const double alpha = p * q / pq;")
+    # one division (1 / (p + q)) per primitive quartet; 1/p and 1/q come with the pairs
+    w("    const double p = ab.p, q = cd.p, inv = 1.0 / (p + q);")
+    w("    const double alpha = p * q * inv;")
     w("    const double Xd = ab.Px - cd.Px, Yd = ab.Py - cd.Py, Zd = ab.Pz - cd.Pz;")
     w(f"    RT F[{L + 1}];")
     w(f"    boys<{L}>(alpha * (Xd * Xd + Yd * Yd + Zd * Zd), bt, F);")
     w("    const RT X = RT(Xd), Y = RT(Yd), Z = RT(Zd);")
     w("    const RT m2a = RT(-2.0 * alpha);")
-    w("    const RT lambda = RT(34.986836655249725693 / (p * q * sqrt(pq)) * ab.K * cd.K);")
+    w("    const RT lambda = RT(34.986836655249725693 * (pair_k_over_p(ab) * pair_k_over_p(cd)) * sqrt(inv));")
     w("    const RT g0 = lambda;")
     for n in range(1, L + 1):
         w(f"    const RT g{n} = g{n - 1} * m2a;")
@@ -561,17 +611,26 @@ def r_stream(L, w, store):
                         if t > 1:
                             e += f" + RT({t - 1}) * {nm(n + 1, t - 2, u, v)}"
                         w(f"    const RT {nm(n, t, u, v)} = {e};")
-                w(store(hidx(L, t, u, v), nm(0, t, u, v)))
+                w(store((t, u, v), nm(0, t, u, v)))
 
 
 def gen_class_team(LA, LB, LC, LD, idx):
     L = LA + LB + LC + LD
     LAB, LCD = LA + LB, LC + LD
-    E, F = comps_range(LA, LAB), comps_range(LC, LCD)
-    HAB = herm_list(LAB)
+    HR, HAB = orbit_order(herm_list(L)), orbit_order(herm_list(LAB))
+    E = orbit_order(comps_range(LA, LAB))
+    codes, fixed = orbits(comps_range(LC, LCD), lambda f: ket_weight(LAB, f))
+    F = orbit_order(comps_range(LC, LCD), lambda f: ket_weight(LAB, f))
+    # the pieces of ket code in the order the passes take them: heaviest first, so that the pieces of one
+    # pass take about the same time
+    passes = sorted([(f, 3 * k, False) for k, f in enumerate(codes)]
+                    + [(f, 3 * len(codes) + k, True) for k, f in enumerate(fixed)],
+                    key=lambda p: -ket_weight(LAB, p[0]))
     NR, NH = nherm(L), nherm(LAB)
     NEB, NEK = 3 * ne1(LAB), 3 * ne1(LCD)
-    BOFF, KOFF = NR, NR + NEB
+    KOFF, BOFF = NR, NR + NEK
+    rslot = {h: k for k, h in enumerate(HR)}
+    hslot = {h: k for k, h in enumerate(HAB)}
     o = []
     w = o.append
     w(f"// class {idx} in team form: R has {NR} entries, Y_f {NH}, [e0|f0] {len(E)} x {len(F)}")
@@ -579,26 +638,49 @@ def gen_class_team(LA, LB, LC, LD, idx):
     w(f"constexpr int kTeamNH{idx} = {NH};")
     w(f"constexpr int kTeamNE{idx} = {len(E)};")
     w(f"constexpr int kTeamNF{idx} = {len(F)};")
-    w(f"constexpr int kTeamStage{idx} = {NR + NEB + NEK};   // stage entries per lane")
-    # ket-step instruction estimate (loads, products, fused multiply-adds) of the largest component: the
-    # launcher sizes its warp count so that the ket code running at once fits the instruction cache
-    sizes = []
-    for f in F:
-        supp = (f[0] + 1) * (f[1] + 1) * (f[2] + 1)
-        idxs = set((h[0] + a, h[1] + b, h[2] + c) for h in HAB for a in range(f[0] + 1) for b in range(f[1] + 1)
-                   for c in range(f[2] + 1))
-        sizes.append(len(HAB) * supp + len(idxs) + 2 * supp + sum(f) + 3)
-    w(f"constexpr int kTeamKetInstr{idx} = {max(sizes)};")
+    w(f"constexpr int kTeamNCode{idx} = {len(passes)};   // pieces of ket code")
+    w(f"constexpr int kTeamStage{idx} = {NR + NEB + NEK};   // stage entries per lane: R, ket tables, bra tables")
+    w(f"constexpr int kTeamKetStage{idx} = {NR + NEK};   // ... of which the ket step reads these")
+    w("// slot of piece jc's component in rotation 0 (rotation r: + r), and whether it is its own rotation")
+    w(f"__device__ __forceinline__ constexpr int team_fslot_{idx}(const int jc)")
+    w("{")
+    w("    return " + "".join(f"jc == {k} ? {p[1]} : " for k, p in enumerate(passes)) + "0;")
+    w("}")
+    w(f"__device__ __forceinline__ constexpr bool team_ffixed_{idx}(const int jc)")
+    w("{")
+    w("    (void)jc;")
+    w("    return " + (" || ".join(f"jc == {k}" for k, p in enumerate(passes) if p[2]) or "false") + ";")
+    w("}")
+    # a stage seen in rotation r
+    w("// a stage of one lane seen in rotation r: orbit members of R, axes of the ket and of the bra tables")
+    w("template <class RT>")
+    w(f"struct TeamView{idx}")
+    w("{")
+    w("    const RT *st, *r0, *r1, *r2, *kx, *ky, *kz, *bx, *by, *bz;")
+    w(f"    __device__ __forceinline__ TeamView{idx}(const RT* stage, const int r) : st(stage)")
+    w("    {")
+    w("        const int a0 = r, a1 = r == 2 ? 0 : r + 1, a2 = r == 0 ? 2 : r - 1;   // (j + r) % 3")
+    w("        r0 = st + a0 * 32; r1 = st + a1 * 32; r2 = st + a2 * 32;")
+    for n, off, cnt in (("k", KOFF, ne1(LCD)), ("b", BOFF, ne1(LAB))):
+        w(f"        {n}x = st + ({off} + a0 * {cnt}) * 32; {n}y = st + ({off} + a1 * {cnt}) * 32; "
+          f"{n}z = st + ({off} + a2 * {cnt}) * 32;")
+    w("    }")
+    w("};")
+
+    def r_at(h):
+        k, j = orbit_member(HR, h)
+        return f"v.st[{k * 32}]" if j is None else f"v.r{j}[{k * 32}]"
+
     # producer
     w("// one lane's stage for one primitive quartet: entry i at st[i * 32]; the bra tables only when bra_e")
-    w("template <class RT>")
-    w(f"__device__ __forceinline__ void team_produce_{idx}(RT* __restrict__ st, const PrimPairData& ab,")
-    w("    const PrimPairData& cd, const double* __restrict__ bt, const bool bra_e)")
+    w("template <class RT, class Pair, class Table>")
+    w(f"__device__ __forceinline__ void team_produce_{idx}(RT* __restrict__ st, const Pair& ab, const Pair& cd,")
+    w("    const Table& bt, const bool bra_e)")
     w("{")
-    r_stream(L, w, lambda H, name: f"    st[{H} * 32] = {name};")
+    r_stream(L, w, lambda t, name: f"    st[{rslot[t]} * 32] = {name};")
     if LCD > 0:
         w("    {")
-        w("    const RT a12k = RT(0.5 / cd.p);")
+        w("    const RT a12k = RT(pair_half_over_p(cd));")
         w("    const RT kPAx = RT(cd.PAx), kPAy = RT(cd.PAy), kPAz = RT(cd.PAz);")
         for d, (dn, PA) in enumerate((("ekx", "kPAx"), ("eky", "kPAy"), ("ekz", "kPAz"))):
             for s_ in gen_E(dn, LCD, 0, PA, "0", "a12k"):
@@ -610,7 +692,7 @@ def gen_class_team(LA, LB, LC, LD, idx):
     if LAB > 0:
         w("    if (bra_e)")
         w("    {")
-        w("    const RT a12b = RT(0.5 / ab.p);")
+        w("    const RT a12b = RT(pair_half_over_p(ab));")
         w("    const RT bPAx = RT(ab.PAx), bPAy = RT(ab.PAy), bPAz = RT(ab.PAz);")
         for d, (dn, PA) in enumerate((("ebx", "bPAx"), ("eby", "bPAy"), ("ebz", "bPAz"))):
             for s_ in gen_E(dn, LAB, 0, PA, "0", "a12b"):
@@ -622,21 +704,22 @@ def gen_class_team(LA, LB, LC, LD, idx):
     else:
         w("    (void)bra_e;")
     w("}")
-    # consumer: ket step of component jf
-    w("// Y_f[h] += sum_{h' in supp(f)} (-1)^{|h'|} E^{f0}_{h'} R_{h+h'} for ket component jf (warp-uniform)")
+    # ket step of piece jc
+    w("// Y[h] += sum_{h' in supp(f)} (-1)^{|h'|} E^{f0}_{h'} R_{h+h'} for the component f of piece jc in the")
+    w("// view's frame (jc warp-uniform)")
     w("template <class RT>")
-    w(f"__device__ __forceinline__ void team_ket_{idx}(const int jf, const RT* __restrict__ st, RT (&Yf)[{NH}])")
+    w(f"__device__ __forceinline__ void team_ket_piece_{idx}(const int jc, const TeamView{idx}<RT>& v, RT (&Yf)[{NH}])")
     w("{")
-    w("    switch (jf)")
+    w("    switch (jc)")
     w("    {")
-    for jf, f in enumerate(F):
-        w(f"    case {jf}: {{ // f = {f}")
-        for d, dn in enumerate(("ekx", "eky", "ekz")):
+    for jc, (f, _, _) in enumerate(passes):
+        w(f"    case {jc}: {{ // f = {f}")
+        for d, (dn, ptr) in enumerate((("ekx", "kx"), ("eky", "ky"), ("ekz", "kz"))):
             for t in range(f[d] + 1):
                 if f[d] == 0:
                     w(f"    const RT {dn}_0_0_0 = RT(1);")
                 else:
-                    w(f"    const RT {dn}_{f[d]}_0_{t} = st[{KOFF + d * ne1(LCD) + e1_slot(f[d], t)} * 32];")
+                    w(f"    const RT {dn}_{f[d]}_0_{t} = v.{ptr}[{e1_slot(f[d], t)} * 32];")
         supp = [(tp, up, vp) for tp in range(f[0] + 1) for up in range(f[1] + 1) for vp in range(f[2] + 1)]
         for (tp, up, vp) in supp:
             sgn = "-" if (tp + up + vp) & 1 else ""
@@ -644,55 +727,88 @@ def gen_class_team(LA, LB, LC, LD, idx):
         contrib = {}
         for h in HAB:
             for hp in supp:
-                H = hidx(L, h[0] + hp[0], h[1] + hp[1], h[2] + hp[2])
-                contrib.setdefault(H, []).append((hidx(LAB, *h), hp))
+                contrib.setdefault((h[0] + hp[0], h[1] + hp[1], h[2] + hp[2]), []).append((hslot[h], hp))
         for H in sorted(contrib):
             body = " ".join(f"Yf[{xi}] = qfma(s{hp[0]}{hp[1]}{hp[2]}, r, Yf[{xi}]);" for (xi, hp) in contrib[H])
-            w(f"    {{ const RT r = st[{H} * 32]; {body} }}")
+            w(f"    {{ const RT r = {r_at(H)}; {body} }}")
         w("    } break;")
     w("    default: break;")
     w("    }")
     w("}")
-    # consumer: bra step (the same for every f)
-    w("// acc[e] += sum_t E^{ex 0}_t sum_u E^{ey 0}_u sum_v E^{ez 0}_v Y_f[tuv], bra tables from the stage")
+    # bra step (the same for every f)
+    w("// acc[e] += sum_t E^{ex 0}_t sum_u E^{ey 0}_u sum_v E^{ez 0}_v Y[tuv], e and tuv in the view's frame")
     w("template <class RT>")
-    w(f"__device__ __forceinline__ void team_bra_{idx}(const RT* __restrict__ st, const RT (&Yf)[{NH}],")
+    w(f"__device__ __forceinline__ void team_bra_view_{idx}(const TeamView{idx}<RT>& v, const RT (&Yf)[{NH}],")
     w(f"    RT (&acc)[{len(E)}])")
     w("{")
-    for d, dn in enumerate(("ebx", "eby", "ebz")):
+    for dn, ptr in (("ebx", "bx"), ("eby", "by"), ("ebz", "bz")):
         w(f"    const RT {dn}_0_0_0 = RT(1);")
         for i in range(1, LAB + 1):
             for t in range(i + 1):
-                w(f"    const RT {dn}_{i}_0_{t} = st[{BOFF + d * ne1(LAB) + e1_slot(i, t)} * 32];")
+                w(f"    const RT {dn}_{i}_0_{t} = v.{ptr}[{e1_slot(i, t)} * 32];")
     for je, e in enumerate(E):
         w("    {")
         w("      RT sx = RT(0);")
         for t in range(e[0] + 1):
             w("      { RT sy = RT(0);")
             for u in range(e[1] + 1):
-                zs = f"ebz_{e[2]}_0_0 * Yf[{hidx(LAB, t, u, 0)}]"
-                for v in range(1, e[2] + 1):
-                    zs = f"qfma(ebz_{e[2]}_0_{v}, Yf[{hidx(LAB, t, u, v)}], {zs})"
+                zs = f"ebz_{e[2]}_0_0 * Yf[{hslot[(t, u, 0)]}]"
+                for vv in range(1, e[2] + 1):
+                    zs = f"qfma(ebz_{e[2]}_0_{vv}, Yf[{hslot[(t, u, vv)]}], {zs})"
                 w(f"        sy = qfma(eby_{e[1]}_0_{u}, {zs}, sy);")
             w(f"        sx = qfma(ebx_{e[0]}_0_{t}, sy, sx); }}")
         w(f"      acc[{je}] += sx;")
         w("    }")
     w("}")
+    # acc, in the frame of rotation r, to column fslot of [e0|f0] (row = slot of e)
+    w("// acc (frame of rotation r) to rows e of [e0|f0]: hA points at this lane's entry of row 0, column f")
+    w("template <class RT>")
+    w(f"__device__ __forceinline__ void team_store_{idx}(const RT (&acc)[{len(E)}], RT* __restrict__ hA, const int r)")
+    w("{")
+    row = len(F) * 32
+    w(f"    RT* const h0 = hA + r * {row};")
+    w(f"    RT* const h1 = hA + (r == 2 ? 0 : r + 1) * {row};")
+    w(f"    RT* const h2 = hA + (r == 0 ? 2 : r - 1) * {row};")
+    w("    (void)h0; (void)h1; (void)h2;")
+    for je, e in enumerate(E):
+        k, j = orbit_member(E, e)
+        w(f"    {'hA' if j is None else f'h{j}'}[{k * row}] = acc[{je}];")
+    w("}")
+    # one component at a time, Y and acc in the molecule's own frame
+    w("// the ket step of component jf (slot order) and the bra step with every index in the molecule's frame")
+    w("template <class RT>")
+    w(f"__device__ __forceinline__ void team_ket_{idx}(const int jf, const RT* __restrict__ st, RT (&Yf)[{NH}])")
+    w("{")
+    nrot = 3 * len(codes)
+    w(f"    const int r = jf < {nrot} ? jf % 3 : 0;")
+    w("    int jc = 0;")
+    w(f"    while (team_fslot_{idx}(jc) != jf - r) ++jc;")
+    w(f"    RT Y[{NH}] = {{}};")
+    w(f"    team_ket_piece_{idx}<RT>(jc, TeamView{idx}<RT>(st, r), Y);")
+    nhrot = 3 * len(orbits(herm_list(LAB))[0])
+    w(f"    for (int k = 0; k < {NH}; ++k) Yf[k < {nhrot} ? k - k % 3 + (k + r) % 3 : k] += Y[k];")
+    w("}")
+    w("template <class RT>")
+    w(f"__device__ __forceinline__ void team_bra_{idx}(const RT* __restrict__ st, const RT (&Yf)[{NH}], RT (&acc)[{len(E)}])")
+    w("{")
+    w(f"    team_bra_view_{idx}<RT>(TeamView{idx}<RT>(st, 0), Yf, acc);")
+    w("}")
     # the recurrences on the per-CTA scratch, whose layout is lane-minor (element k of lane l at [k * 32 + l]):
     # ket of one e row: p[f] -> y[c * ND + d]; bra of one (c d) column: y[e * NCD] -> o[(a * NB + b) * os]
     nd, nb, ncd = len(comps(LD)), len(comps(LB)), len(comps(LC)) * len(comps(LD))
+    Fn, En = comps_range(LC, LCD), comps_range(LA, LAB)
     w("template <class RT>")
     w(f"__device__ __forceinline__ void team_hrr_ket_{idx}(const RT* p, RT* y, const RT CDx, const RT CDy,")
     w("    const RT CDz)")
     w("{")
-    hrr_code(LC, LD, lambda k: f"p[{k} * 32]", lambda ix, iy, v, nrm: f"    y[{ix * nd + iy} * 32] = {v} * RT({lit(nrm)});",
-             ("CDx", "CDy", "CDz"), w, "t")
+    hrr_code(LC, LD, lambda k: f"p[{F.index(Fn[k])} * 32]",
+             lambda ix, iy, v, nrm: f"    y[{ix * nd + iy} * 32] = {v} * RT({lit(nrm)});", ("CDx", "CDy", "CDz"), w, "t")
     w("}")
     w("template <class RT>")
     w(f"__device__ __forceinline__ void team_hrr_bra_{idx}(const RT* y, RT* o, const int os, const RT ABx,")
     w("    const RT ABy, const RT ABz)")
     w("{")
-    hrr_code(LA, LB, lambda k: f"y[{k * ncd} * 32]",
+    hrr_code(LA, LB, lambda k: f"y[{E.index(En[k]) * ncd} * 32]",
              lambda ix, iy, v, nrm: f"    o[{ix * nb + iy} * os] = {v} * RT({lit(nrm)});", ("ABx", "ABy", "ABz"), w, "t")
     w("}")
     return o

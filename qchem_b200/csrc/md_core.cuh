@@ -78,48 +78,51 @@ __host__ __device__ constexpr double comp_norm(int L, int k)
 // ------------------------------------------------------------------------------------------------
 // Boys function.  Three branches as in AuxillaryFJ.C:13-48.  The T<12 table (121 x 23, step 0.1) is
 // generated from the series definition by gen_boys_table.py and read through the read-only path.
+//
+// An FP64 division is a sequence of some ten dependent instructions, so the constants of the Taylor sum and of
+// the downward recursion are multiplied by their reciprocals, the upward branch divides once (1/T) and takes
+// its fit coefficients by selection instead of branching (lanes of a warp fall into different intervals).
 // ------------------------------------------------------------------------------------------------
+// F_{JMAX+k} at table row `it`, over k!
 template <int JMAX>
-__device__ __forceinline__ void boys(double T, const double* __restrict__ table, double (&F)[JMAX + 1])
+__device__ __forceinline__ double boys_taylor(const double* __restrict__ table, int it, int k)
+{
+    constexpr double inv_fact[7] = {1.0, 1.0, 0.5, 1.0 / 6.0, 1.0 / 24.0, 1.0 / 120.0, 1.0 / 720.0};
+    return __ldg(table + it * 23 + JMAX + k) * inv_fact[k];
+}
+
+struct BoysColumns;
+template <int JMAX>
+__device__ __forceinline__ double boys_taylor(const BoysColumns& t, int it, int k);
+
+template <int JMAX, class Table>
+__device__ __forceinline__ void boys(double T, const Table& table, double (&F)[JMAX + 1])
 {
     const double et = exp(-T);
     if (T < 12.0)
     {
         const int it = (int)(T * 10.0 + 0.5);
         const double dt = (double)it * 0.1 - T;
-        const double* FT = table + it * 23 + JMAX;
         // Taylor: F_j(T) = sum_k F_{j+k}(T*) dt^k / k!
-        double f0 = __ldg(FT), f1 = __ldg(FT + 1), f2 = __ldg(FT + 2), f3 = __ldg(FT + 3), f4 = __ldg(FT + 4),
-               f5 = __ldg(FT + 5), f6 = __ldg(FT + 6);
-        double dt2 = dt * dt, dt3 = dt2 * dt, dt4 = dt3 * dt, dt5 = dt4 * dt, dt6 = dt5 * dt;
-        double f = f0;
-        f += f1 * dt / 1.0;
-        f += f2 * dt2 / 2.0;
-        f += f3 * dt3 / 6.0;
-        f += f4 * dt4 / 24.0;
-        f += f5 * dt5 / 120.0;
-        f += f6 * dt6 / 720.0;
-        F[JMAX] = f;
+        double f = boys_taylor<JMAX>(table, it, 6);
 #pragma unroll
-        for (int j = JMAX - 1; j >= 0; --j) F[j] = (2 * T * F[j + 1] + et) / (2 * j + 1);
+        for (int k = 5; k >= 0; --k) f = fma(f, dt, boys_taylor<JMAX>(table, it, k));
+        F[JMAX] = f;
+        const double T2 = 2.0 * T;
+#pragma unroll
+        for (int j = JMAX - 1; j >= 0; --j) F[j] = fma(T2, F[j + 1], et) * (1.0 / (2 * j + 1));
     }
     else
     {
-        const double pi = 3.14159265358979323846;
-        double F0;
-        if (T < 30.0)
-        {
-            double g;
-            if (T < 15.0) g = 0.4999489092 - 0.2473631686 / T + 0.321180909 / (T * T) - 0.3811559346 / (T * T * T);
-            else if (T < 18.0) g = 0.4998436875 - 0.24249438 / T + 0.24642845 / (T * T);
-            else if (T < 24.0) g = 0.499093162 - 0.2152832 / T;
-            else g = 0.49;
-            F0 = 0.5 * sqrt(pi / T) - et * g / T;
-        }
-        else
-            F0 = 0.5 * sqrt(pi / T);
-        F[0] = F0;
-        const double inv2T = 1.0 / (2 * T);
+        const double iT = 1.0 / T;
+        double c0 = 0.49, c1 = 0.0, c2 = 0.0, c3 = 0.0;
+        if (T < 24.0) { c0 = 0.499093162; c1 = -0.2152832; }
+        if (T < 18.0) { c0 = 0.4998436875; c1 = -0.24249438; c2 = 0.24642845; }
+        if (T < 15.0) { c0 = 0.4999489092; c1 = -0.2473631686; c2 = 0.321180909; c3 = -0.3811559346; }
+        if (!(T < 30.0)) c0 = 0.0;
+        const double g = fma(fma(fma(c3, iT, c2), iT, c1), iT, c0);
+        F[0] = 0.5 * sqrt(3.14159265358979323846 * iT) - et * g * iT;
+        const double inv2T = 0.5 * iT;
 #pragma unroll
         for (int j = 0; j < JMAX; ++j) F[j + 1] = ((2 * j + 1) * F[j] - et) * inv2T;
     }
@@ -127,8 +130,8 @@ __device__ __forceinline__ void boys(double T, const double* __restrict__ table,
 
 // FP32 form of the Boys function.  FP64 is kept where the table and the downward recursion live (T < 12);
 // above, the asymptotic branches are evaluated in FP32.
-template <int JMAX>
-__device__ __forceinline__ void boys(double T, const double* __restrict__ table, float (&F)[JMAX + 1])
+template <int JMAX, class Table>
+__device__ __forceinline__ void boys(double T, const Table& table, float (&F)[JMAX + 1])
 {
     if (T < 12.0)
     {
@@ -192,6 +195,38 @@ __device__ __forceinline__ PrimPairData make_prim_pair(double a, double ax, doub
     const double abx = ax - bx, aby = ay - by, abz = az - bz;
     d.K = ca * cb * exp(-a * b * ip * (abx * abx + aby * aby + abz * abz));
     return d;
+}
+
+// What the Hermite integrals and the single-centre E tables of a primitive quartet need of a pair, with its
+// divisions done: the team kernels form it once per pair and group, not once per primitive quartet.
+struct TeamPair
+{
+    double p, Px, Py, Pz, PAx, PAy, PAz, kp, h;   // kp = K / p, h = 1 / (2 p)
+};
+constexpr int kTeamPairDoubles = 9;
+
+__device__ __forceinline__ TeamPair team_pair(const PrimPairData& d)
+{
+    const double ip = 1.0 / d.p;
+    return TeamPair{d.p, d.Px, d.Py, d.Pz, d.PAx, d.PAy, d.PAz, d.K * ip, 0.5 * ip};
+}
+__device__ __forceinline__ double pair_k_over_p(const TeamPair& d) { return d.kp; }
+__device__ __forceinline__ double pair_half_over_p(const TeamPair& d) { return d.h; }
+__device__ __forceinline__ double pair_k_over_p(const PrimPairData& d) { return d.K / d.p; }
+__device__ __forceinline__ double pair_half_over_p(const PrimPairData& d) { return 0.5 / d.p; }
+
+// The columns of the Boys table that a kernel of one class reads, F_{JMAX} .. F_{JMAX+6} over k!, in shared
+// memory (column-major): the lanes' rows differ, and a gather from shared memory costs the few cycles of its
+// bank conflicts where one from the global table costs a tag lookup per lane.
+constexpr int kBoysRows = 121, kBoysColumns = 7;
+struct BoysColumns
+{
+    const double* s;
+};
+template <int JMAX>
+__device__ __forceinline__ double boys_taylor(const BoysColumns& t, int it, int k)
+{
+    return t.s[k * kBoysRows + it];
 }
 
 // how a sink is handed to a __noinline__ chunk function: by reference unless the sink says it is a

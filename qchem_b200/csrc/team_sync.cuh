@@ -74,10 +74,10 @@ __device__ __forceinline__ void mbar_inval(uint64_t* bar)
     asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-// this thread's generic-proxy writes to global memory become visible to later bulk copies (async proxy)
-__device__ __forceinline__ void fence_async_global()
+// this thread's generic-proxy accesses to global and shared memory come before later bulk copies (async proxy)
+__device__ __forceinline__ void fence_async()
 {
-    asm volatile("fence.proxy.async.global;" ::: "memory");
+    asm volatile("fence.proxy.async;" ::: "memory");
 }
 
 }   // namespace team
