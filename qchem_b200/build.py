@@ -118,7 +118,7 @@ def _jobs():
     for k in range(NCLASS):
         defs = [f"-DQCG_CLASS={k}"]
         parts = [_read(team_src), _read(os.path.join(GEN, f"md_team_{k}.cuh"))]
-        key = _hash(parts + core + _headers(["eri_kernels.cuh", "eri_team.cuh", "eri_team_iface.h", "team_sync.cuh", "smem_attr.h"])
+        key = _hash(parts + core + _headers(["eri_kernels.cuh", "eri_team.cuh", "jk_group.cuh", "eri_team_iface.h", "team_sync.cuh", "smem_attr.h"])
                     + FLAGS + defs)
         jobs.append((team_src, defs, os.path.join(BUILD, f"eri_team_{k}_{key}.o")))
     extra = {"runtime.cu": _headers(["boys_table.h", "eri_team_iface.h"]) + [_read(os.path.join(INCLUDE, "qchem_b200.h"))],

@@ -1,6 +1,7 @@
 // eri_team.cu -- the team form of the FP64 ERI batches (eri_team.cuh) for ONE quartet class; compiled with
 // -DQCG_CLASS=k for every class, defining launch_eri_team_k and team_shape_k.  The generated code comes from
 // gen/md_team_<k>.cuh (stage tables, ket and bra steps, recurrences).
+#include <algorithm>
 #include <atomic>
 
 #include "eri_kernels.cuh"
@@ -75,6 +76,21 @@ struct Cls
     static constexpr int kKetStage = gen::QCG_CAT(kTeamKetStage, QCG_CLASS);
     static constexpr int kNG = team_pieces(kNCode, kNH, kNE), kNW = 3 * kNG;
     static constexpr int kMinBlocks = team_min_blocks(kNG, kStage);
+    // jk_group_kernel: groups of 32 quartets per round (two sets of stages within the shared memory), its warps --
+    // eight where Y_f, acc_f or the digestion of a (dd| bra need more registers than twelve leave -- and CTAs per SM
+    static constexpr int kGroups = [] {
+        const int g = (int)((227 * 1024 - 8192 - (int)(kBoysRows * kBoysColumns * sizeof(double))) /
+                            (2 * kStage * 32 * sizeof(double)));
+        return g < 1 ? 1 : (g > 4 ? 4 : g);
+    }();
+    static constexpr int kJKWarps = LA + LB == 4 ? 8 : 12, kJKBlocks = 1;
+    static __device__ __forceinline__ unsigned long long column(int cd) { return gen::QCG_CAT(kTeamColumn, QCG_CLASS)[cd]; }
+    static __device__ __forceinline__ double column_norm(int cd) { return gen::QCG_CAT(kTeamColumnNorm, QCG_CLASS)[cd]; }
+    template <class Sink>
+    static __device__ __forceinline__ void bra_out(const double (&y)[kNE], double ABx, double ABy, double ABz, Sink sink)
+    {
+        gen::QCG_CAT(team_bra_out_, QCG_CLASS)<double>(y, ABx, ABy, ABz, sink);
+    }
     using View = gen::QCG_CAT(TeamView, QCG_CLASS)<double>;
     static __device__ __forceinline__ constexpr int fslot(int jc) { return gen::QCG_CAT(team_fslot_, QCG_CLASS)(jc); }
     static __device__ __forceinline__ constexpr bool fixed(int jc) { return gen::QCG_CAT(team_ffixed_, QCG_CLASS)(jc); }
@@ -110,6 +126,8 @@ struct Cls
 constexpr int kThreads = Cls::kNW * 32;
 constexpr int kNCD = ncart(Cls::LC) * ncart(Cls::LD);
 constexpr size_t kSmem = team_smem(Cls::kStage);   // the stages and the Boys columns
+constexpr size_t kGroupSmem =
+    (2 * (size_t)Cls::kGroups * Cls::kStage * 32 + kBoysRows * kBoysColumns) * sizeof(double);
 std::atomic<unsigned long long> g_smem_ready{0};
 }   // namespace
 
@@ -123,9 +141,11 @@ TeamShape QCG_CAT(team_shape_, QCG_CLASS)(int nsm)
     TeamShape sh;
     sh.grid = nsm * per_sm;
     sh.threads = kThreads;
+    sh.nsm = nsm;
     sh.slot_doubles = (long long)Cls::kStage * 32;
-    // [e0|f0], [e0|cd] and, for the J/K form, (ab|cd): lane-minor blocks of the group's 32 quartets
-    sh.hrr_doubles = (long long)(Cls::kNE * Cls::kNF + Cls::kNE * kNCD + ncart(Cls::LA) * ncart(Cls::LB) * kNCD) * 32;
+    // [e0|f0] and [e0|cd]: lane-minor blocks of the group's 32 quartets (the J/K form: [e0|f0] of its groups)
+    sh.hrr_doubles = (long long)Cls::kNE * (Cls::kNF + kNCD) * 32;
+    sh.group_doubles = (long long)Cls::kGroups * Cls::kNE * Cls::kNF * 32 * nsm * Cls::kJKBlocks;
     return sh;
 }
 
@@ -150,10 +170,21 @@ void QCG_CAT(launch_jk_team_, QCG_CLASS)(const JKWorkDev& w, const PairListDev& 
 {
     const long long span = w.gend - w.gbeg;
     if (span <= 0) return;
+    const long long ngroups = (span + 31) / 32;
+    if (scr.kmax == 1)
+    {
+        // one primitive quartet per quartet throughout: jk_group_kernel, one wave of CTAs
+        auto k = w.det_lo ? jk_group_kernel<Cls, true> : jk_group_kernel<Cls, false>;
+        static std::atomic<unsigned long long> ready{0}, ready_det{0};
+        ensure_smem(k, kGroupSmem, w.det_lo ? ready_det : ready);
+        const long long rounds = (ngroups + Cls::kGroups - 1) / Cls::kGroups;
+        const long long blocks = std::min<long long>(rounds, (long long)sh.nsm * Cls::kJKBlocks);
+        k<<<(unsigned)blocks, Cls::kJKWarps * 32, kGroupSmem, st>>>(w, bra, ket, P, f0, D, J, K, n, boys, scr.hrr);
+        return;
+    }
     auto k = w.det_lo ? jk_team_kernel<Cls, true> : jk_team_kernel<Cls, false>;
     static std::atomic<unsigned long long> ready{0}, ready_det{0};
     ensure_smem(k, kSmem, w.det_lo ? ready_det : ready);
-    const long long ngroups = (span + 31) / 32;
     const long long blocks = ngroups < sh.grid ? ngroups : sh.grid;
     k<<<(unsigned)blocks, kThreads, kSmem, st>>>(w, bra, ket, P, f0, D, J, K, n, boys, scr);
 }

@@ -44,9 +44,8 @@ extern __shared__ __align__(128) double qcg_team_smem[];
 // Shared memory of both kernels: three stages, whose space holds the group's primitive pairs while the stage
 // tables are made (slot t of lane l: entry k at [(t * kTeamPairDoubles + k) * 32 + l]), then the Boys columns.
 template <class Cls>
-__device__ __forceinline__ BoysColumns team_boys(const double* __restrict__ table)
+__device__ __forceinline__ BoysColumns team_boys(double* __restrict__ s, const double* __restrict__ table)
 {
-    double* const s = qcg_team_smem + Cls::kStageSpace;
     for (int i = threadIdx.x; i < kBoysRows * kBoysColumns; i += blockDim.x)
     {
         const int k = i / kBoysRows, it = i - k * kBoysRows;
@@ -203,7 +202,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         for (int s = 0; s < 3; ++s) team::mbar_init(&full[s]);
         team::mbar_init_fence();
     }
-    const BoysColumns bt = team_boys<Cls>(boys_table);
+    const BoysColumns bt = team_boys<Cls>(qcg_team_smem + Cls::kStageSpace, boys_table);
     __syncthreads();
     double* const rc = scr.rcache + (long long)blockIdx.x * scr.kmax * STAGE;   // this CTA's stage slots
     double* const hA = scr.hrr + (long long)blockIdx.x * (NE * NF + NE * NCD) * 32;
@@ -260,14 +259,18 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     }
 }
 
+}   // namespace qcg
+
+#include "jk_group.cuh"
+
+namespace qcg {
+
 // ------------------------------------------------------------------------------------------------
-// The team form of the direct J/K build.  The same three phases on 32 quartets of a class's screened work
-// list at a time (lane l: quartet gbeg + 32 g + l, its bra pair found by binary search, its kets from the
-// Q-sorted list), the stages built from the primitive-pair table; the bra recurrence writes (ab|cd) into a
-// third lane-minor block of the CTA's scratch, and a fourth phase digests it into J' and K' with the
-// thread-per-quartet kernel's sink (JKSink: the eight permutational images, symmetry weights, registers for
-// the partial sums, atomics or the deterministic integer pairs), warp w taking ket components w, w + nwarps,
-// ....  This replaces qchem's MakeDirect/MakeExchange + ERI4::MatMul (Molecule/IrrepBasisSet.C:138-183,
+// The team form of the direct J/K build (contracted classes; uncontracted ones: jk_group.cuh).  The same stages
+// and contraction on 32 quartets of a class's screened work list at a time (lane l: quartet gbeg + 32 g + l, its
+// bra pair found by binary search, its kets from the Q-sorted list), the stages built from the primitive-pair
+// table; then the digestion of [e0|f0] into J' and K' (team_digest), the (c d) columns split over the warps.
+// This replaces qchem's MakeDirect/MakeExchange + ERI4::MatMul (Molecule/IrrepBasisSet.C:138-183,
 // Internal/Imp/ERI4.C:10-17) without storing the integrals.
 // ------------------------------------------------------------------------------------------------
 template <class Cls, bool DET>
@@ -279,9 +282,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     constexpr int NW = Cls::kNW;
     constexpr int NF = Cls::kNF, NE = Cls::kNE;
     constexpr int STAGE = Cls::kStage * 32;
-    constexpr int NB = ncart(Cls::LB), ND = ncart(Cls::LD);
-    constexpr int NAB = ncart(Cls::LA) * NB, NCD = ncart(Cls::LC) * ND;
-    static_assert(NE <= NAB && NF <= NCD, "[e0|f0] fits the blocks");
+    constexpr int NCD = ncart(Cls::LC) * ncart(Cls::LD);
     __shared__ uint64_t full[3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool leader = threadIdx.x == 0;
@@ -290,12 +291,10 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         for (int s = 0; s < 3; ++s) team::mbar_init(&full[s]);
         team::mbar_init_fence();
     }
-    const BoysColumns bt = team_boys<Cls>(boys_table);
+    const BoysColumns bt = team_boys<Cls>(qcg_team_smem + Cls::kStageSpace, boys_table);
     __syncthreads();
     double* const rc = scr.rcache + (long long)blockIdx.x * scr.kmax * STAGE;
-    double* const hA = scr.hrr + (long long)blockIdx.x * (NE * NF + NE * NCD + NAB * NCD) * 32;
-    double* const hB = hA + NE * NF * 32;
-    double* const hC = hB + NE * NCD * 32;
+    double* const hA = scr.hrr + (long long)blockIdx.x * NE * NF * 32;
     unsigned long long G = 0;
     const long long ngroups = (w.gend - w.gbeg + 31) >> 5;
     for (long long g = blockIdx.x; g < ngroups; g += gridDim.x)
@@ -335,57 +334,11 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
             [&](int kl) { return load_pp(P, ket.ppo[j] + kl); });
         // 2. contraction (as in eri_batch_team_kernel)
         if (!team_contract<Cls>(rc, hA, Kq, Kcd, Kg, G, full, scr.err)) return;
-        // 3. recurrences into the scratch: [e0|cd] in hB, (ab|cd) in hC (lane-minor)
-        // C - D = (P - D) - (P - C) and A - B = (P - B) - (P - A), from the shell pairs' first primitive pairs
-        if (valid)
-        {
-            const PrimPairData cd0 = load_pp(P, ket.ppo[j]);
-            const double CDx = cd0.PBx - cd0.PAx, CDy = cd0.PBy - cd0.PAy, CDz = cd0.PBz - cd0.PAz;
-            for (int e = warp; e < NE; e += NW)
-                Cls::hrr_ket(hA + e * NF * 32 + lane, hB + e * NCD * 32 + lane, CDx, CDy, CDz);
-        }
-        __syncthreads();
-        if (valid)
-        {
-            const PrimPairData ab0 = load_pp(P, bra.ppo[i]);
-            const double ABx = ab0.PBx - ab0.PAx, ABy = ab0.PBy - ab0.PAy, ABz = ab0.PBz - ab0.PAz;
-            for (int cd = warp; cd < NCD; cd += NW)
-                Cls::hrr_bra(hB + cd * 32 + lane, hC + cd * 32 + lane, NCD * 32, ABx, ABy, ABz);
-        }
-        __syncthreads();
-        // 4. digestion of this lane's quartet, ket components cd = warp, warp + NW, ...
-        if (valid)
-        {
-            JKSink<double, Cls::LA, Cls::LB, Cls::LC, Cls::LD, DET> sink;
-            sink.D = D;
-            sink.J = J;
-            sink.K = K;
-            sink.n = n;
-            if constexpr (DET) sink.det_lo = w.det_lo;
-            if (bra.mol)
-            {
-                const int m = bra.mol[i];
-                const long long o = w.mols.off[m];
-                sink.D = D + o;
-                sink.J = J + o;
-                sink.K = K + o;
-                sink.n = w.mols.n[m];
-            }
-            sink.set_bra(shell_f0[sa], shell_f0[sb]);
-            sink.fc = shell_f0[sc];
-            sink.fd = shell_f0[sd];
-            sink.s = (sa == sb ? 0.5 : 1.0) * (sc == sd ? 0.5 : 1.0) * ((w.same_class && i == j) ? 0.5 : 1.0);
-            for (int cd = warp; cd < NCD; cd += NW)
-            {
-                const int ic = cd / ND, id = cd - ic * ND;
-                sink.ket_begin(ic, id);
-#pragma unroll
-                for (int ab = 0; ab < NAB; ++ab) sink(ab / NB, ab % NB, ic, id, hC[(ab * NCD + cd) * 32 + lane]);
-                sink.ket_end(ic, id);
-                sink.flush_k_row();
-            }
-            sink.flush_bra();
-        }
+        // 3. recurrences and digestion, the (c d) columns in runs of neighbours over the warps
+        constexpr int PER = (NCD + NW - 1) / NW;
+        const int cd0 = warp * PER, cd1 = cd0 + PER < NCD ? cd0 + PER : NCD;
+        if (cd0 < NCD)
+            team_digest<Cls, DET>(w, bra, ket, P, shell_f0, D, J, K, n, hA + lane, valid, i, j, cd0, cd1, lane);
         __syncthreads();   // the scratch and the R cache are free for the next group
     }
 }

@@ -9,8 +9,7 @@ namespace qcg {
 // Device memory a team launch works in, beside its inputs and outputs (the handle owns it):
 //   rcache -- per CTA, kmax stage slots: the primitive quartets' R tables and Hermite tables, written once
 //             per group of quartets and streamed back into shared memory once per pass;
-//   hrr    -- per CTA, the [e0|f0], [e0|cd] and (for the J/K form) (ab|cd) blocks of the group's 32 quartets,
-//             lane-minor;
+//   hrr    -- per CTA, the [e0|f0] and [e0|cd] blocks of the group's 32 quartets, lane-minor;
 //   err    -- bit 0: a wait for a bulk copy gave up (the results of the launch are not valid);
 //             bit 1: a group needed more stage slots than kmax.
 struct TeamScratchDev
@@ -24,9 +23,10 @@ struct TeamScratchDev
 // The launch shape of class k on nsm SMs and the scratch it needs per CTA, in doubles.
 struct TeamShape
 {
-    int grid, threads;
-    long long slot_doubles;   // one stage slot of the R cache
-    long long hrr_doubles;
+    int grid, threads, nsm;
+    long long slot_doubles;    // one stage slot of the R cache
+    long long hrr_doubles;     // recurrence blocks
+    long long group_doubles;   // all CTAs' blocks of the J/K build of an uncontracted class
 };
 
 using EriTeamLauncher = void (*)(const BasisDev&, const int4*, const int*, long long, double*, const double*,

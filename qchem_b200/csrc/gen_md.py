@@ -811,6 +811,34 @@ def gen_class_team(LA, LB, LC, LD, idx):
     hrr_code(LA, LB, lambda k: f"y[{E.index(En[k]) * ncd} * 32]",
              lambda ix, iy, v, nrm: f"    o[{ix * nb + iy} * os] = {v} * RT({lit(nrm)});", ("ABx", "ABy", "ABz"), w, "t")
     w("}")
+    # the J/K digestion's forms: a (c d) column as terms of [e0|f0] columns, and the bra recurrence from registers
+    # into a sink.  (c, d) = sum over k <= d of binom(d, k) CD^(d - k) [c + k]; a term is a 16-bit field: the slot of
+    # c + k in the low byte, the code of its factor (column_factor) in the high byte
+    factor = {(0, 0, 0): {1: 1}, (1, 0, 0): {1: 2, 2: 5}, (0, 1, 0): {1: 3, 2: 6}, (0, 0, 1): {1: 4, 2: 7},
+              (2, 0, 0): {1: 8}, (0, 2, 0): {1: 9}, (0, 0, 2): {1: 10}, (1, 1, 0): {1: 11}, (0, 1, 1): {1: 12},
+              (1, 0, 1): {1: 13}}
+    cols, norms = [], []
+    for c in comps(LC):
+        for d in comps(LD):
+            v = 0
+            terms = [(a, b, e) for a in range(d[0] + 1) for b in range(d[1] + 1) for e in range(d[2] + 1)]
+            for t, k in enumerate(reversed(terms)):
+                rest = tuple(d[x] - k[x] for x in range(3))
+                binom = math.prod(math.comb(d[x], k[x]) for x in range(3))
+                v |= (F.index(tuple(c[x] + k[x] for x in range(3))) | factor[rest][binom] << 8) << (16 * t)
+            cols.append(v)
+            norms.append(comp_norm(c) * comp_norm(d))
+    w("#ifdef __CUDACC__")
+    w(f"static __constant__ unsigned long long kTeamColumn{idx}[{len(cols)}] = {{{', '.join('0x%xull' % v for v in cols)}}};")
+    w(f"static __constant__ double kTeamColumnNorm{idx}[{len(cols)}] = {{{', '.join(lit(v) for v in norms)}}};")
+    w("#endif")
+    w("template <class RT, class Sink>")
+    w(f"__device__ __forceinline__ void team_bra_out_{idx}(const RT (&y)[{len(E)}], const RT ABx, const RT ABy,")
+    w("    const RT ABz, Sink sink)")
+    w("{")
+    hrr_code(LA, LB, lambda k: f"y[{E.index(En[k])}]",
+             lambda ix, iy, v, nrm: f"    sink({ix}, {iy}, {v} * RT({lit(nrm)}));", ("ABx", "ABy", "ABz"), w, "t")
+    w("}")
     return o
 
 

@@ -2557,7 +2557,8 @@ bool team_scratch(qcg_handle* h, int k, TeamScratchDev& scr, TeamShape& sh)
     long long kmax = 1;
     for (int l : Ls) kmax *= h->maxnp[l];
     sh = kEriTeamShapes[k](h->nsm);
-    const long long need = (long long)sh.grid * (kmax * sh.slot_doubles + sh.hrr_doubles);
+    long long need = (long long)sh.grid * (kmax * sh.slot_doubles + sh.hrr_doubles);
+    if (kmax == 1) need = std::max(need, (long long)sh.grid * sh.slot_doubles + sh.group_doubles);
     if (need * (long long)sizeof(double) > kTeamScratchMax) return false;
     if (need > h->team_cap)
     {
