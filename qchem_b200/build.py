@@ -64,11 +64,10 @@ def _eri_hrr(k: int) -> bool:
     return k in HRR_CLASSES
 
 
-# FP64 ERI-batch classes that run in the team form (eri_team.cu) by default: every class whose ket pair is not
-# (ss).  Measured on a B200 at 10^6 quartets per class, the team form was 1.15-6.8x faster on these 15 classes
-# ((dd|dd) 2.8x, (dd|pp) 6.8x); on the (xx|ss) classes, whose single ket component gives a one-warp CTA, it was
-# 0.6-1.0x.  Every class has a team launcher; QCG_ERI_TEAM_MASK in the environment selects others at run time.
-TEAM_CLASSES = tuple(k for k in range(NCLASS) if k not in (0, 1, 3, 6, 10, 15))
+# FP64 ERI-batch classes that run in the team form (eri_team.cu) by default: every class.  The (xx|ss) ones run
+# eri_ss_kernel there (a thread per quartet with its sums in registers).  QCG_ERI_TEAM_MASK in the environment
+# selects others at run time.
+TEAM_CLASSES = tuple(range(NCLASS))
 
 
 def _team_mask() -> int:
@@ -118,7 +117,7 @@ def _jobs():
     for k in range(NCLASS):
         defs = [f"-DQCG_CLASS={k}"]
         parts = [_read(team_src), _read(os.path.join(GEN, f"md_team_{k}.cuh"))]
-        key = _hash(parts + core + _headers(["eri_kernels.cuh", "eri_team.cuh", "jk_group.cuh", "eri_team_iface.h", "team_sync.cuh", "smem_attr.h"])
+        key = _hash(parts + core + _headers(["eri_kernels.cuh", "eri_team.cuh", "eri_ss.cuh", "jk_group.cuh", "eri_team_iface.h", "team_sync.cuh", "smem_attr.h"])
                     + FLAGS + defs)
         jobs.append((team_src, defs, os.path.join(BUILD, f"eri_team_{k}_{key}.o")))
     extra = {"runtime.cu": _headers(["boys_table.h", "eri_team_iface.h"]) + [_read(os.path.join(INCLUDE, "qchem_b200.h"))],

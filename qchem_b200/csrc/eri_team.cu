@@ -18,6 +18,12 @@
 #define QCG_CAT(a, b) QCG_CAT2(a, b)
 #include QCG_STR(gen/QCG_CAT(md_team_, QCG_CLASS).cuh)
 
+// the classes whose ket pair is (ss): X (X + 1) / 2
+#define QCG_SS_KET (QCG_CLASS == 0 || QCG_CLASS == 1 || QCG_CLASS == 3 || QCG_CLASS == 6 || QCG_CLASS == 10 || QCG_CLASS == 15)
+#if QCG_SS_KET
+#include "eri_ss.cuh"
+#endif
+
 namespace qcg {
 
 namespace {
@@ -116,11 +122,22 @@ struct Cls
     {
         gen::QCG_CAT(team_hrr_ket_, QCG_CLASS)<double>(p, y, CDx, CDy, CDz);
     }
-    static __device__ __forceinline__ void hrr_bra(const double* y, double* o, int os, double ABx, double ABy,
-                                                   double ABz)
+    template <class OT>
+    static __device__ __forceinline__ void hrr_bra(const double* y, OT* o, int os, double ABx, double ABy, double ABz)
     {
-        gen::QCG_CAT(team_hrr_bra_, QCG_CLASS)<double>(y, o, os, ABx, ABy, ABz);
+        gen::QCG_CAT(team_hrr_bra_, QCG_CLASS)<double, OT>(y, o, os, ABx, ABy, ABz);
     }
+#if QCG_SS_KET
+    static __device__ __forceinline__ void hermite_add(const TeamPair& ab, const TeamPair& cd, const BoysColumns& bt,
+                                                       double (&Y)[kNH])
+    {
+        gen::QCG_CAT(team_hermite_add_, QCG_CLASS)<double>(ab, cd, bt, Y);
+    }
+    static __device__ __forceinline__ void bra_pair(const TeamPair& ab, const double (&Y)[kNH], double (&acc)[kNE])
+    {
+        gen::QCG_CAT(team_bra_pair_, QCG_CLASS)<double>(ab, Y, acc);
+    }
+#endif
 };
 
 constexpr int kThreads = Cls::kNW * 32;
@@ -133,7 +150,7 @@ std::atomic<unsigned long long> g_smem_ready{0};
 
 TeamShape QCG_CAT(team_shape_, QCG_CLASS)(int nsm)
 {
-    auto k = eri_batch_team_kernel<Cls>;
+    auto k = eri_batch_team_kernel<Cls, double>;
     ensure_smem(k, kSmem, g_smem_ready);
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, kSmem) != cudaSuccess || per_sm < 1)
@@ -149,17 +166,71 @@ TeamShape QCG_CAT(team_shape_, QCG_CLASS)(int nsm)
     return sh;
 }
 
-void QCG_CAT(launch_eri_team_, QCG_CLASS)(const BasisDev& bs, const int4* q, const int* order, long long nq,
-                                          double* out, const double* boys, const TeamScratchDev& scr,
-                                          const TeamShape& sh, cudaStream_t st)
+namespace {
+template <class OT>
+void launch_batch(const BasisDev& bs, const int4* q, const int* order, long long nq, OT* out, const double* boys,
+                  const TeamScratchDev& scr, const TeamShape& sh, cudaStream_t st)
 {
     if (nq <= 0) return;
-    auto k = eri_batch_team_kernel<Cls>;
-    ensure_smem(k, kSmem, g_smem_ready);
+    auto k = eri_batch_team_kernel<Cls, OT>;
+    static std::atomic<unsigned long long> ready{0};
+    ensure_smem(k, kSmem, ready);
     // one wave of CTAs, each walking groups of 32 quartets; the scratch has room for sh.grid CTAs
     const long long ngroups = (nq + 31) / 32;
     const long long blocks = ngroups < sh.grid ? ngroups : sh.grid;
     k<<<(unsigned)blocks, kThreads, kSmem, st>>>(bs, q, order, nq, out, boys, scr);
+}
+#if QCG_SS_KET
+template <class OT, int SPLIT>
+void launch_ss_split(const BasisDev& bs, const int4* q, const int* order, long long nq, OT* out, const double* boys,
+                     int nsm, cudaStream_t st)
+{
+    auto k = eri_ss_kernel<Cls, OT, SPLIT>;
+    constexpr int warps = kSSThreads / 32, per = warps * (32 / SPLIT);
+    constexpr size_t smem =
+        (kBoysRows * kBoysColumns + warps * kSSKetSlots * kSSKetDoubles * (32 / SPLIT)) * sizeof(double);
+    static std::atomic<unsigned long long> ready{0};
+    ensure_smem(k, smem, ready);
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kSSThreads, smem) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    const long long blocks = std::min<long long>((nq + per - 1) / per, (long long)nsm * per_sm);
+    k<<<(unsigned)blocks, kSSThreads, smem, st>>>(bs, q, order, nq, out, boys);
+}
+// Lanes per quartet: one where one lane per quartet gives every SM a few warps, else as many of the up to nine
+// bra primitive pairs as lanes are free (a quartet of 81 primitive quartets is a serial chain of 81 otherwise).
+template <class OT>
+void launch_ss(const BasisDev& bs, const int4* q, const int* order, long long nq, OT* out, const double* boys,
+               int nsm, cudaStream_t st)
+{
+    if (nq <= 0) return;
+    const long long lanes = (long long)nsm * 4 * 32;
+    if (nq * 8 <= lanes) launch_ss_split<OT, 8>(bs, q, order, nq, out, boys, nsm, st);
+    else if (nq * 2 <= lanes) launch_ss_split<OT, 4>(bs, q, order, nq, out, boys, nsm, st);
+    else launch_ss_split<OT, 1>(bs, q, order, nq, out, boys, nsm, st);
+}
+#endif
+}   // namespace
+
+void QCG_CAT(launch_eri_team_, QCG_CLASS)(const BasisDev& bs, const int4* q, const int* order, long long nq,
+                                          double* out, const double* boys, const TeamScratchDev& scr,
+                                          const TeamShape& sh, cudaStream_t st)
+{
+#if QCG_SS_KET
+    launch_ss(bs, q, order, nq, out, boys, sh.nsm, st);
+#else
+    launch_batch(bs, q, order, nq, out, boys, scr, sh, st);
+#endif
+}
+void QCG_CAT(launch_eri_team32_, QCG_CLASS)(const BasisDev& bs, const int4* q, const int* order, long long nq,
+                                            float* out, const double* boys, const TeamScratchDev& scr,
+                                            const TeamShape& sh, cudaStream_t st)
+{
+#if QCG_SS_KET
+    launch_ss(bs, q, order, nq, out, boys, sh.nsm, st);
+#else
+    launch_batch(bs, q, order, nq, out, boys, scr, sh, st);
+#endif
 }
 
 // the team form of the direct J/K build of this class (jk_team_kernel); the scratch has room for sh.grid CTAs

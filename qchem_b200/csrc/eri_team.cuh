@@ -183,10 +183,11 @@ __device__ __forceinline__ bool team_contract(const double* __restrict__ rc, dou
     return true;
 }
 
-template <class Cls>
+// OT: the output type.  Float output (the FP32 batches) is the FP64 evaluation rounded once.
+template <class Cls, class OT>
 __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     eri_batch_team_kernel(BasisDev bs, const int4* __restrict__ quartets, const int* __restrict__ order, long long nq,
-                          double* __restrict__ out, const double* __restrict__ boys_table, TeamScratchDev scr)
+                          OT* __restrict__ out, const double* __restrict__ boys_table, TeamScratchDev scr)
 {
     constexpr int NW = Cls::kNW;
     constexpr int NF = Cls::kNF, NE = Cls::kNE;
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         if (valid)
         {
             const double ABx = A[0] - B[0], ABy = A[1] - B[1], ABz = A[2] - B[2];
-            double* const o = out + q * BLK;
+            OT* const o = out + q * BLK;
             for (int cd = warp; cd < NCD; cd += NW) Cls::hrr_bra(hB + cd * 32 + lane, o + cd, NCD, ABx, ABy, ABz);
         }
         __syncthreads();   // the scratch and the R cache are free for the next group

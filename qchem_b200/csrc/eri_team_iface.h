@@ -31,6 +31,9 @@ struct TeamShape
 
 using EriTeamLauncher = void (*)(const BasisDev&, const int4*, const int*, long long, double*, const double*,
                                  const TeamScratchDev&, const TeamShape&, cudaStream_t);
+// the FP32 batches: the same evaluation with float output
+using EriTeam32Launcher = void (*)(const BasisDev&, const int4*, const int*, long long, float*, const double*,
+                                   const TeamScratchDev&, const TeamShape&, cudaStream_t);
 using EriTeamShapeFn = TeamShape (*)(int nsm);
 
 using JKTeamLauncher = void (*)(const JKWorkDev&, const PairListDev&, const PairListDev&, const PrimPairsDev&,
@@ -38,6 +41,7 @@ using JKTeamLauncher = void (*)(const JKWorkDev&, const PairListDev&, const Pair
                                 const TeamScratchDev&, const TeamShape&, cudaStream_t);
 
 extern const EriTeamLauncher kEriTeamLaunchers[kNumQuartetClasses];
+extern const EriTeam32Launcher kEriTeam32Launchers[kNumQuartetClasses];
 extern const JKTeamLauncher kJKTeamLaunchers[kNumQuartetClasses];
 extern const EriTeamShapeFn kEriTeamShapes[kNumQuartetClasses];
 

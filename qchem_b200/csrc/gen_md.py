@@ -735,6 +735,21 @@ def gen_class_team(LA, LB, LC, LD, idx):
     w("    default: break;")
     w("    }")
     w("}")
+    def bra_sums():
+        for je, e in enumerate(E):
+            w("    {")
+            w("      RT sx = RT(0);")
+            for t in range(e[0] + 1):
+                w("      { RT sy = RT(0);")
+                for u in range(e[1] + 1):
+                    zs = f"ebz_{e[2]}_0_0 * Yf[{hslot[(t, u, 0)]}]"
+                    for vv in range(1, e[2] + 1):
+                        zs = f"qfma(ebz_{e[2]}_0_{vv}, Yf[{hslot[(t, u, vv)]}], {zs})"
+                    w(f"        sy = qfma(eby_{e[1]}_0_{u}, {zs}, sy);")
+                w(f"        sx = qfma(ebx_{e[0]}_0_{t}, sy, sx); }}")
+            w(f"      acc[{je}] += sx;")
+            w("    }")
+
     # bra step (the same for every f)
     w("// acc[e] += sum_t E^{ex 0}_t sum_u E^{ey 0}_u sum_v E^{ez 0}_v Y[tuv], e and tuv in the view's frame")
     w("template <class RT>")
@@ -746,20 +761,27 @@ def gen_class_team(LA, LB, LC, LD, idx):
         for i in range(1, LAB + 1):
             for t in range(i + 1):
                 w(f"    const RT {dn}_{i}_0_{t} = v.{ptr}[{e1_slot(i, t)} * 32];")
-    for je, e in enumerate(E):
-        w("    {")
-        w("      RT sx = RT(0);")
-        for t in range(e[0] + 1):
-            w("      { RT sy = RT(0);")
-            for u in range(e[1] + 1):
-                zs = f"ebz_{e[2]}_0_0 * Yf[{hslot[(t, u, 0)]}]"
-                for vv in range(1, e[2] + 1):
-                    zs = f"qfma(ebz_{e[2]}_0_{vv}, Yf[{hslot[(t, u, vv)]}], {zs})"
-                w(f"        sy = qfma(eby_{e[1]}_0_{u}, {zs}, sy);")
-            w(f"        sx = qfma(ebx_{e[0]}_0_{t}, sy, sx); }}")
-        w(f"      acc[{je}] += sx;")
-        w("    }")
+    bra_sums()
     w("}")
+    if LCD == 0:
+        # one ket component: the Hermite integrals straight into registers, the bra tables from the pair
+        w("// Y[h] += lambda R_h of one primitive quartet; acc[e] += the bra step with the tables of pair ab")
+        w("template <class RT, class Pair, class Table>")
+        w(f"__device__ __forceinline__ void team_hermite_add_{idx}(const Pair& ab, const Pair& cd, const Table& bt, RT (&Yf)[{NH}])")
+        w("{")
+        r_stream(L, w, lambda t, name: f"    Yf[{hslot[t]}] += {name};")
+        w("}")
+        w("template <class RT, class Pair>")
+        w(f"__device__ __forceinline__ void team_bra_pair_{idx}(const Pair& ab, const RT (&Yf)[{NH}], RT (&acc)[{len(E)}])")
+        w("{")
+        w("    const RT a12b = RT(pair_half_over_p(ab));")
+        w("    const RT bPAx = RT(ab.PAx), bPAy = RT(ab.PAy), bPAz = RT(ab.PAz);")
+        w("    (void)a12b; (void)bPAx; (void)bPAy; (void)bPAz;")
+        for dn, PA in (("ebx", "bPAx"), ("eby", "bPAy"), ("ebz", "bPAz")):
+            for s_ in gen_E(dn, LAB, 0, PA, "0", "a12b"):
+                w("    " + s_)
+        bra_sums()
+        w("}")
     # acc, in the frame of rotation r, to column fslot of [e0|f0] (row = slot of e)
     w("// acc (frame of rotation r) to rows e of [e0|f0]: hA points at this lane's entry of row 0, column f")
     w("template <class RT>")
@@ -804,12 +826,12 @@ def gen_class_team(LA, LB, LC, LD, idx):
     hrr_code(LC, LD, lambda k: f"p[{F.index(Fn[k])} * 32]",
              lambda ix, iy, v, nrm: f"    y[{ix * nd + iy} * 32] = {v} * RT({lit(nrm)});", ("CDx", "CDy", "CDz"), w, "t")
     w("}")
-    w("template <class RT>")
-    w(f"__device__ __forceinline__ void team_hrr_bra_{idx}(const RT* y, RT* o, const int os, const RT ABx,")
+    w("template <class RT, class OT>")
+    w(f"__device__ __forceinline__ void team_hrr_bra_{idx}(const RT* y, OT* o, const int os, const RT ABx,")
     w("    const RT ABy, const RT ABz)")
     w("{")
     hrr_code(LA, LB, lambda k: f"y[{E.index(En[k]) * ncd} * 32]",
-             lambda ix, iy, v, nrm: f"    o[{ix * nb + iy} * os] = {v} * RT({lit(nrm)});", ("ABx", "ABy", "ABz"), w, "t")
+             lambda ix, iy, v, nrm: f"    o[{ix * nb + iy} * os] = OT({v} * RT({lit(nrm)}));", ("ABx", "ABy", "ABz"), w, "t")
     w("}")
     # the J/K digestion's forms: a (c d) column as terms of [e0|f0] columns, and the bra recurrence from registers
     # into a sink.  (c, d) = sum over k <= d of binom(d, k) CD^(d - k) [c + k]; a term is a 16-bit field: the slot of

@@ -18,6 +18,8 @@ namespace qcg {
                          const double*, double*, double*, int, const double*, cudaStream_t, int);                    \
     void launch_eri_team_##k(const BasisDev&, const int4*, const int*, long long, double*, const double*,            \
                              const TeamScratchDev&, const TeamShape&, cudaStream_t);                                 \
+    void launch_eri_team32_##k(const BasisDev&, const int4*, const int*, long long, float*, const double*,          \
+                               const TeamScratchDev&, const TeamShape&, cudaStream_t);                               \
     TeamShape team_shape_##k(int);                                                                                  \
     void launch_jk_team_##k(const JKWorkDev&, const PairListDev&, const PairListDev&, const PrimPairsDev&,          \
                             const int*, const double*, double*, double*, int, const double*, const TeamScratchDev&, \
@@ -58,6 +60,12 @@ const EriTeamLauncher kEriTeamLaunchers[kNumQuartetClasses] = {
     launch_eri_team_10, launch_eri_team_11, launch_eri_team_12, launch_eri_team_13, launch_eri_team_14,
     launch_eri_team_15, launch_eri_team_16, launch_eri_team_17, launch_eri_team_18, launch_eri_team_19,
     launch_eri_team_20};
+const EriTeam32Launcher kEriTeam32Launchers[kNumQuartetClasses] = {
+    launch_eri_team32_0,  launch_eri_team32_1,  launch_eri_team32_2,  launch_eri_team32_3,  launch_eri_team32_4,
+    launch_eri_team32_5,  launch_eri_team32_6,  launch_eri_team32_7,  launch_eri_team32_8,  launch_eri_team32_9,
+    launch_eri_team32_10, launch_eri_team32_11, launch_eri_team32_12, launch_eri_team32_13, launch_eri_team32_14,
+    launch_eri_team32_15, launch_eri_team32_16, launch_eri_team32_17, launch_eri_team32_18, launch_eri_team32_19,
+    launch_eri_team32_20};
 const JKLauncher kJKLaunchers[kNumQuartetClasses] = {
     launch_jk_0,  launch_jk_1,  launch_jk_2,  launch_jk_3,  launch_jk_4,  launch_jk_5,  launch_jk_6,
     launch_jk_7,  launch_jk_8,  launch_jk_9,  launch_jk_10, launch_jk_11, launch_jk_12, launch_jk_13,

@@ -2620,22 +2620,49 @@ long long batch_chunk_bytes()
     return bytes;
 }
 
+// the scratch of a form that is not required of the call: false, with nothing held, where the handle's memory
+// limit or the device does not have it
+bool team_scratch_optional(qcg_handle* h, int k, TeamScratchDev& scr, TeamShape& sh)
+{
+    try
+    {
+        return team_scratch(h, k, scr, sh);
+    }
+    catch (const Error& e)
+    {
+        if (e.code != QCG_ERR_ALLOC) throw;
+        cudaGetLastError();
+        return false;
+    }
+}
+
+// FP64 batches: the team launcher for the classes in the mask (for an (ss) ket it runs eri_ss_kernel, which needs
+// no scratch).  FP32 batches: the same FP64 evaluation with float output -- an FP32 evaluation per quartet and
+// thread took 42.8 ms where this takes 6 (21 classes of 20 011 quartets), and is less exact -- and the FP32
+// thread-per-quartet kernels only where the scratch does not fit.
 template <class T>
 void eri_batch_launch(qcg_handle* h, int k, const int* dq, long long m, T* dout)
 {
+    constexpr bool f64 = std::is_same_v<T, double>;
     const int* order = batch_order(h, dq, m);
-    if constexpr (std::is_same_v<T, double>)
+    const unsigned mask = f64 ? (h->team_mask >= 0 ? (unsigned)h->team_mask : eri_team_mask()) : ~0u;
+    TeamScratchDev scr{};
+    TeamShape sh{};
+    sh.nsm = h->nsm;
+    const bool ss_ket = k == 0 || k == 1 || k == 3 || k == 6 || k == 10 || k == 15;
+    const bool team = ((mask >> k) & 1u) &&
+                      (ss_ket || (f64 ? team_scratch(h, k, scr, sh) : team_scratch_optional(h, k, scr, sh)));
+    const int4* q = (const int4*)dq;
+    if constexpr (f64)
     {
-        const unsigned mask = h->team_mask >= 0 ? (unsigned)h->team_mask : eri_team_mask();
-        TeamScratchDev scr{};
-        TeamShape sh{};
-        if (((mask >> k) & 1u) && team_scratch(h, k, scr, sh))
-            kEriTeamLaunchers[k](h->bs, (const int4*)dq, order, m, dout, h->d_boys, scr, sh, h->stream);
-        else
-            kEriBatchLaunchers[k](h->bs, (const int4*)dq, order, m, dout, h->d_boys, h->stream, h->nsm);
+        if (team) kEriTeamLaunchers[k](h->bs, q, order, m, dout, h->d_boys, scr, sh, h->stream);
+        else kEriBatchLaunchers[k](h->bs, q, order, m, dout, h->d_boys, h->stream, h->nsm);
     }
     else
-        kEriBatch32Launchers[k](h->bs, (const int4*)dq, order, m, dout, h->d_boys, h->stream, h->nsm);
+    {
+        if (team) kEriTeam32Launchers[k](h->bs, q, order, m, dout, h->d_boys, scr, sh, h->stream);
+        else kEriBatch32Launchers[k](h->bs, q, order, m, dout, h->d_boys, h->stream, h->nsm);
+    }
     CK(cudaGetLastError());
 }
 
