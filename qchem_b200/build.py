@@ -75,16 +75,27 @@ def _team_mask() -> int:
 
 
 # classes whose direct J/K build runs in the team form by default (QCG_JK_TEAM_MASK selects others at run time):
-# (dd|dd), (dd|dp), (dd|ds), (dd|pp), (dd|ps), (dp|dp).  Measured class by class on a B200 on the
-# uncontracted 32-water build (1824 functions), the team form took 0.47-0.93x the thread-per-quartet kernel's
-# time on these six ((dd|dd) 43 vs 92 ms, (dp|dp) 528 vs 826 ms) and 0.31-0.76x the warp-shared form's; on
-# (dp|pp) the warp-shared form is faster still (999 vs 1231 ms), and on the others the team form took
-# 1.07-4.7x the thread-per-quartet time.
+# (dd|dd), (dd|dp), (dd|ds), (dd|pp), (dd|ps), (dp|dp).  On a B200, on the uncontracted 16-water build (912
+# functions), per class and serialised, against the thread-per-quartet kernel: (dd|dd) 1.35 vs 6.1 ms, (dd|dp) 10.8
+# vs 46, (dd|ds) 7.2 vs 22, (dd|pp) 12.6 vs 34, (dd|ps) 13.1 vs 34, (dp|dp) 26 vs 86.
 JK_TEAM_CLASSES = (14, 16, 17, 18, 19, 20)
 
 
 def _jk_team_mask() -> int:
     return sum(1 << k for k in JK_TEAM_CLASSES)
+
+
+# ... and beside them, where the class is uncontracted in the basis (jk_group_kernel): (dp|pp) 54.8 ms against 110 in
+# the warp-shared form, (dp|ds) 35.9 against 77; on the classes with lighter quartets the warp-shared or
+# thread-per-quartet form is faster ((dp|ps) 39 vs 63 ms, (ps|ps) 46 vs 96).  Where it is contracted
+# (jk_team_kernel): every class whose ket pair is not (ss) -- eight waters in a split-valence basis of 296 functions
+# take 57 ms with this set, 62 with every class, 87 with the uncontracted set.  Both precede the warp-shared form.
+JK_TEAM_PLAIN_CLASSES = (12, 13)
+JK_TEAM_CONTRACTED_CLASSES = (2, 4, 5, 7, 8, 9, 11, 12, 13)
+
+
+def _mask(classes) -> int:
+    return sum(1 << k for k in classes)
 
 
 # classes whose direct J/K build runs in the warp-shared form by default (QCG_JK_WARP_MASK selects others):
@@ -128,6 +139,8 @@ def _jobs():
         s = os.path.join(CSRC, name)
         defs = HOST_OMP + [f"-DQCG_TEAM_DEFAULT_MASK={_team_mask():#x}u",
                            f"-DQCG_JK_TEAM_DEFAULT_MASK={_jk_team_mask():#x}u",
+                           f"-DQCG_JK_TEAM_PLAIN_MASK={_mask(JK_TEAM_PLAIN_CLASSES):#x}u",
+                           f"-DQCG_JK_TEAM_CONTRACTED_MASK={_mask(JK_TEAM_CONTRACTED_CLASSES):#x}u",
                            f"-DQCG_JK_WARP_DEFAULT_MASK={_jk_warp_mask():#x}u"] if name == "runtime.cu" else []
         key = _hash([_read(s)] + core + extra.get(name, []) + FLAGS + defs)
         jobs.append((s, defs, os.path.join(BUILD, f"{name[:-3]}_{key}.o")))

@@ -162,7 +162,9 @@ TeamShape QCG_CAT(team_shape_, QCG_CLASS)(int nsm)
     sh.slot_doubles = (long long)Cls::kStage * 32;
     // [e0|f0] and [e0|cd]: lane-minor blocks of the group's 32 quartets (the J/K form: [e0|f0] of its groups)
     sh.hrr_doubles = (long long)Cls::kNE * (Cls::kNF + kNCD) * 32;
-    sh.group_doubles = (long long)Cls::kGroups * Cls::kNE * Cls::kNF * 32 * nsm * Cls::kJKBlocks;
+    sh.jk_doubles = (long long)Cls::kNE * Cls::kNF * 32;
+    sh.group_grid = nsm * Cls::kJKBlocks;
+    sh.group_doubles = sh.jk_doubles * Cls::kGroups;
     return sh;
 }
 
@@ -244,13 +246,14 @@ void QCG_CAT(launch_jk_team_, QCG_CLASS)(const JKWorkDev& w, const PairListDev& 
     const long long ngroups = (span + 31) / 32;
     if (scr.kmax == 1)
     {
-        // one primitive quartet per quartet throughout: jk_group_kernel, one wave of CTAs
+        // one primitive quartet per quartet throughout: jk_group_kernel, one wave of CTAs.  A round has as many
+        // groups as the class's group count gives every CTA, so that a small class still spreads over the SMs.
         auto k = w.det_lo ? jk_group_kernel<Cls, true> : jk_group_kernel<Cls, false>;
         static std::atomic<unsigned long long> ready{0}, ready_det{0};
         ensure_smem(k, kGroupSmem, w.det_lo ? ready_det : ready);
-        const long long rounds = (ngroups + Cls::kGroups - 1) / Cls::kGroups;
-        const long long blocks = std::min<long long>(rounds, (long long)sh.nsm * Cls::kJKBlocks);
-        k<<<(unsigned)blocks, Cls::kJKWarps * 32, kGroupSmem, st>>>(w, bra, ket, P, f0, D, J, K, n, boys, scr.hrr);
+        const int per = (int)std::min<long long>(Cls::kGroups, std::max<long long>(1, ngroups / sh.group_grid));
+        const long long blocks = std::min<long long>((ngroups + per - 1) / per, sh.group_grid);
+        k<<<(unsigned)blocks, Cls::kJKWarps * 32, kGroupSmem, st>>>(w, bra, ket, P, f0, D, J, K, n, boys, scr.hrr, per);
         return;
     }
     auto k = w.det_lo ? jk_team_kernel<Cls, true> : jk_team_kernel<Cls, false>;

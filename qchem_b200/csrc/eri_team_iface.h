@@ -26,7 +26,9 @@ struct TeamShape
     int grid, threads, nsm;
     long long slot_doubles;    // one stage slot of the R cache
     long long hrr_doubles;     // recurrence blocks
-    long long group_doubles;   // all CTAs' blocks of the J/K build of an uncontracted class
+    // the J/K build: CTAs and [e0|f0] doubles per CTA of the uncontracted form, [e0|f0] doubles of the contracted one
+    int group_grid;
+    long long group_doubles, jk_doubles;
 };
 
 using EriTeamLauncher = void (*)(const BasisDev&, const int4*, const int*, long long, double*, const double*,

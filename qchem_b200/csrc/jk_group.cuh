@@ -171,7 +171,7 @@ template <class Cls, bool DET>
 __global__ void __launch_bounds__(Cls::kJKWarps * 32, Cls::kJKBlocks)
     jk_group_kernel(JKWorkDev w, PairListDev bra, PairListDev ket, PrimPairsDev P, const int* __restrict__ shell_f0,
                     const double* __restrict__ D, double* __restrict__ J, double* __restrict__ K, int n,
-                    const double* __restrict__ boys_table, double* __restrict__ scratch)
+                    const double* __restrict__ boys_table, double* __restrict__ scratch, const int ngrp)
 {
     constexpr int NGRP = Cls::kGroups, STAGE = Cls::kStage * 32;
     constexpr int NE = Cls::kNE, NF = Cls::kNF, NH = Cls::kNH, NC = Cls::kNCode;
@@ -183,18 +183,18 @@ __global__ void __launch_bounds__(Cls::kJKWarps * 32, Cls::kJKBlocks)
     const BoysColumns bt = team_boys<Cls>(qcg_team_smem + 2 * NGRP * STAGE, boys_table);
     if (threadIdx.x < 2) counter[threadIdx.x] = 0;
     __syncthreads();
-    double* const hA = scratch + (long long)blockIdx.x * NGRP * NE * NF * 32;
+    double* const hA = scratch + (long long)blockIdx.x * ngrp * NE * NF * 32;
     auto draw = [&](int c) {
         int t = 0;
         if (lane == 0) t = atomicAdd(&counter[c], 1);
         return __shfl_sync(0xffffffffu, t, 0);
     };
     const long long ngroups = (w.gend - w.gbeg + 31) >> 5;
-    const long long nround = (ngroups + NGRP - 1) / NGRP;
+    const long long nround = (ngroups + ngrp - 1) / ngrp;   // rounds of ngrp <= NGRP groups
 
     // the lanes' quartets and the stage of group slot s of round r, into set `set`
     auto make = [&](long long r, int s, int set) {
-        const long long gq = w.gbeg + (r * NGRP + s) * 32 + lane;
+        const long long gq = w.gbeg + (r * ngrp + s) * 32 + lane;
         bool valid = gq < w.gend;
         int i = 0, j = 0;
         if (valid)
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(Cls::kJKWarps * 32, Cls::kJKBlocks)
 
     int set = 0;
     if (blockIdx.x < nround)
-        for (int s = threadIdx.x >> 5; s < NGRP; s += Cls::kJKWarps) make(blockIdx.x, s, 0);
+        for (int s = threadIdx.x >> 5; s < ngrp; s += Cls::kJKWarps) make(blockIdx.x, s, 0);
     __syncthreads();
     for (long long r = blockIdx.x; r < nround; r += gridDim.x, set ^= 1)
     {
@@ -230,8 +230,8 @@ __global__ void __launch_bounds__(Cls::kJKWarps * 32, Cls::kJKBlocks)
         for (;;)
         {
             const int t = draw(0);
-            if (t >= NC * NGRP * 3) break;
-            const int jc = t / (NGRP * 3), u = t - jc * (NGRP * 3), s = u / 3, rot = u - 3 * s;
+            if (t >= NC * ngrp * 3) break;
+            const int jc = t / (ngrp * 3), u = t - jc * (ngrp * 3), s = u / 3, rot = u - 3 * s;
             if (!live[set][s] || (rot != 0 && Cls::fixed(jc))) continue;
             if (quartet[set][s][lane].x >= 0)
             {
@@ -254,13 +254,13 @@ __global__ void __launch_bounds__(Cls::kJKWarps * 32, Cls::kJKBlocks)
         for (;;)
         {
             int t = draw(1);
-            if (t < NGRP)
+            if (t < ngrp)
             {
                 if (more) make(r + gridDim.x, t, set ^ 1);
                 continue;
             }
-            t -= NGRP;
-            if (t >= NGRP * NCc) break;
+            t -= ngrp;
+            if (t >= ngrp * NCc) break;
             const int s = t / NCc, ic = t - s * NCc;
             if (!live[set][s]) continue;
             const int2 q = quartet[set][s][lane];

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <deque>
 #include <memory>
+#include <map>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -207,6 +208,64 @@ public:
         std::lock_guard<std::mutex> g(mu_);
         pinned_.emplace(cap, p);
     }
+    // Device scratch of the team kernels (a few MiB for a small molecule, up to GiB for contracted batches), at least
+    // `bytes`; *cap receives the capacity.  An idle buffer serves while it is not more than four times too large.
+    // Idle scratch is bounded by kScratchIdle per device; beyond it a returned buffer is freed.
+    static constexpr size_t kScratchIdle = (size_t)2 << 30;
+    void* scratch(int dev, size_t bytes, size_t* cap)
+    {
+        const size_t unit = (size_t)1 << 20;
+        *cap = (bytes + unit - 1) / unit * unit;
+        std::vector<void*> drop;
+        {
+            std::lock_guard<std::mutex> g(mu_);
+            auto& pd = per_[dev];
+            auto it = pd.scratch.lower_bound(*cap);
+            if (it != pd.scratch.end() && it->first / 4 <= *cap)
+            {
+                void* p = it->second;
+                *cap = it->first;
+                pd.scratch_idle -= it->first;
+                pd.scratch.erase(it);
+                return p;
+            }
+        }
+        void* p = nullptr;
+        cudaError_t e = cudaMalloc(&p, *cap);
+        if (e == cudaErrorMemoryAllocation)
+        {
+            cudaGetLastError();
+            {
+                std::lock_guard<std::mutex> g(mu_);
+                auto& pd = per_[dev];
+                for (auto& kv : pd.scratch) drop.push_back(kv.second);
+                pd.scratch.clear();
+                pd.scratch_idle = 0;
+            }
+            for (void* q : drop) cudaFree(q);
+            e = cudaMalloc(&p, *cap);
+        }
+        if (e != cudaSuccess)
+        {
+            cudaGetLastError();
+            throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+        }
+        return p;
+    }
+    void give_scratch(int dev, void* p, size_t cap)
+    {
+        {
+            std::lock_guard<std::mutex> g(mu_);
+            auto& pd = per_[dev];
+            if (pd.scratch_idle + cap <= kScratchIdle)
+            {
+                pd.scratch.emplace(cap, p);
+                pd.scratch_idle += cap;
+                return;
+            }
+        }
+        cudaFree(p);
+    }
     void give_slab(int dev, void* p)
     {
         std::lock_guard<std::mutex> g(mu_);
@@ -237,6 +296,7 @@ public:
         {
             cudaSetDevice(kv.first);
             for (void* p : kv.second.slabs) cudaFree(p);
+            for (auto& b : kv.second.scratch) cudaFree(b.second);
             for (cudaStream_t s : kv.second.streams) cudaStreamDestroy(s);
             for (cudaEvent_t e : kv.second.tevents) cudaEventDestroy(e);
             for (cudaEvent_t e : kv.second.sevents) cudaEventDestroy(e);
@@ -253,6 +313,8 @@ private:
     struct PerDevice
     {
         std::vector<void*> slabs;
+        std::multimap<size_t, void*> scratch;   // idle, by capacity
+        size_t scratch_idle = 0;
         std::vector<cudaStream_t> streams;
         std::vector<cudaEvent_t> tevents, sevents;
     };
@@ -359,9 +421,43 @@ struct qcg_handle
     int *d_order = nullptr, *d_hist = nullptr, *d_cursor = nullptr;
 
     // team-form ERI batches (eri_team.cu): per-CTA R cache and recurrence scratch (grow only), error word
-    double* d_team = nullptr;
-    long long team_cap = 0;   // doubles
+    // scratch of the team kernels: ERI batches, and J/K builds (whose address recorded graphs hold)
+    struct Scratch
+    {
+        void* p = nullptr;
+        size_t cap = 0;
+        long long counted = 0;   // bytes in mem_used: what was asked for, whatever the cache gave
+    };
+    Scratch team_scr, jk_scr;
+    // at least `doubles` in s, for work queued on the handle's stream from now on; a buffer that has to grow goes back
+    // to the cache once the work that may use it is done
+    double* scratch(Scratch& s, long long doubles)
+    {
+        const size_t bytes = (size_t)doubles * sizeof(double);
+        if (bytes <= s.cap) return (double*)s.p;
+        if (s.p)
+        {
+            if (&s == &jk_scr) drop_graphs();
+            CK(cudaStreamSynchronize(stream));
+            give_scratch(s, true);
+        }
+        if (mem_limit > 0 && mem_used + (long long)bytes > mem_limit)
+            throw Error{QCG_ERR_ALLOC, "device memory limit of " + std::to_string(mem_limit) + " bytes exceeded"};
+        s.p = ResourceCache::get().scratch(device, bytes, &s.cap);
+        s.counted = (long long)bytes;
+        mem_used += s.counted;
+        return (double*)s.p;
+    }
+    void give_scratch(Scratch& s, bool healthy)
+    {
+        if (!s.p) return;
+        mem_used -= s.counted;
+        if (healthy) ResourceCache::get().give_scratch(device, s.p, s.cap);
+        else cudaFree(s.p);
+        s = Scratch{};
+    }
     int* d_team_err = nullptr;
+    TeamShape team_shapes[kNumQuartetClasses]{};
     bool team_pending = false;   // a team kernel ran since the error word was last read
     unsigned char* d_pmask = nullptr;   // qcg_set_pair_subset (null: every quartet)
     int maxnp[kMaxL + 1] = {};   // largest contraction length per angular momentum (0: not yet computed)
@@ -564,6 +660,8 @@ struct qcg_handle
             if (healthy) rc.give_slab(device, a.p);
             else cudaFree(a.p);
         }
+        give_scratch(team_scr, healthy);
+        give_scratch(jk_scr, healthy);
         if (stage)
         {
             if (healthy) rc.give_stage(stage);
@@ -2070,6 +2168,10 @@ void warp_items(qcg_handle* h, int k)
 #ifndef QCG_JK_WARP_DEFAULT_MASK
 #define QCG_JK_WARP_DEFAULT_MASK 0u
 #endif
+#ifndef QCG_JK_TEAM_PLAIN_MASK
+#define QCG_JK_TEAM_PLAIN_MASK 0u
+#define QCG_JK_TEAM_CONTRACTED_MASK 0u
+#endif
 // The classes whose direct J/K build runs in the warp-shared form: the build's choice
 // (QCG_JK_WARP_DEFAULT_MASK), unless QCG_JK_WARP_MASK in the environment names others (read once; *forced
 // then true).
@@ -2082,11 +2184,76 @@ unsigned jk_warp_mask_default(bool* forced)
     return mask;
 }
 
-bool team_scratch(qcg_handle* h, int k, TeamScratchDev& scr, TeamShape& sh);
 unsigned jk_team_mask_default(bool* forced);
-// smallest per-rank quartet count of a class for the build's default team form (2^20: ~220 groups of 32
-// quartets per CTA on 148 SMs)
-constexpr long long kJKTeamMinQuartets = 1LL << 20;
+int team_kmax(qcg_handle* h, int k);
+const TeamShape& team_shape(qcg_handle* h, int k);
+int* team_error_word(qcg_handle* h);
+// most scratch of one class in the team form
+constexpr long long kTeamScratchMax = 4LL << 30;
+// smallest quartet count of a class for the warp-shared form by default
+constexpr long long kJKWarpMinQuartets = 1LL << 20;
+// most scratch that lets the team classes of one build run side by side (they share one class's worth beyond it)
+constexpr long long kJKTeamSideMax = 2LL << 30;
+
+// The classes of a J/K build that run in the team form, their launch shapes and scratch.  side: every class has its
+// own scratch and takes any side stream; else they share it and run one after another on the first one.
+struct JKTeamPlan
+{
+    bool on[kNumQuartetClasses] = {};
+    TeamScratchDev scr[kNumQuartetClasses]{};
+    TeamShape sh[kNumQuartetClasses]{};
+    bool side = false;
+};
+
+// want[k]: class k in the team form if its scratch can be had; required: the caller named the classes, so that a
+// failed allocation is an error rather than a reason for another form.
+void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool required, JKTeamPlan& plan)
+{
+    long long need[kNumQuartetClasses] = {}, all = 0, most = 0;
+    for (int k = 0; k < kNumQuartetClasses; ++k)
+    {
+        if (!want[k]) continue;
+        long long gb = 0, ge = 0;
+        shard_range(h, k, gb, ge);
+        const long long ngroups = (ge - gb + 31) / 32;
+        const int kmax = team_kmax(h, k);
+        TeamShape& sh = plan.sh[k];
+        sh = team_shape(h, k);
+        sh.grid = (int)std::min<long long>(sh.grid, ngroups);
+        sh.group_grid = (int)std::min<long long>(sh.group_grid, ngroups);
+        need[k] = kmax == 1 ? std::min<long long>(ngroups, sh.group_grid * (sh.group_doubles / sh.jk_doubles)) * sh.jk_doubles
+                            : sh.grid * (kmax * sh.slot_doubles + sh.jk_doubles);
+        if (need[k] * (long long)sizeof(double) > kTeamScratchMax) continue;
+        plan.on[k] = true;
+        plan.scr[k].kmax = kmax;
+        all += need[k];
+        most = std::max(most, need[k]);
+    }
+    if (most == 0) return;
+    plan.side = all * (long long)sizeof(double) <= kJKTeamSideMax;
+    const long long total = plan.side ? all : most;
+    double* p = nullptr;
+    try
+    {
+        p = h->scratch(h->jk_scr, total);
+    }
+    catch (const Error& e)
+    {
+        if (required || e.code != QCG_ERR_ALLOC) throw;
+        plan = JKTeamPlan{};
+        return;
+    }
+    int* const err = team_error_word(h);
+    for (int k = 0; k < kNumQuartetClasses; ++k)
+        if (plan.on[k])
+        {
+            TeamScratchDev& scr = plan.scr[k];
+            scr.rcache = p;
+            scr.hrr = scr.kmax == 1 ? p : p + (long long)plan.sh[k].grid * scr.kmax * plan.sh[k].slot_doubles;
+            scr.err = err;
+            if (plan.side) p += need[k];
+        }
+}
 
 // fp32_below: quartets whose density-weighted bound Q_ab Q_cd max|D| (max over the six D blocks the
 // quartet digests) is below it are evaluated in FP32 (FP64 accumulation); 0 = all FP64, HUGE_VAL = all
@@ -2127,27 +2294,25 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     ensure_side_streams(h);
     // the build: zero J'/K', class kernels over the side streams, symmetrisation (timing events only
     // when the build is not a graph)
-    // classes built in the team form (FP64 band only); their scratch is sized here, before any capture, and
-    // their launches share it, so they run one after another on the first side stream
-    // The build's default applies to a class only when its slice has at least kJKTeamMinQuartets quartets:
-    // the team form is a throughput design (a CTA per SM streaming groups of 32 quartets), and on a small
-    // build (a 57-function water) its classes took 3x the thread-per-quartet kernels' time.  A mask set by
-    // qcg_set_jk_team_classes or QCG_JK_TEAM_MASK applies whatever the size.
+    // Classes built in the team form (FP64 band only), planned before any capture.  The build's default depends on
+    // whether the class is contracted in this basis (build.py has the two sets), not on the size: the uncontracted
+    // set was faster from one water (197 -> 166 us) to sixteen (660 -> 528 ms), the contracted one likewise
+    // (1.7 -> 0.42 ms, and 204 -> 57 ms for eight).
     bool jk_forced = h->jk_team_mask >= 0;
-    unsigned jk_mask = jk_forced ? (unsigned)h->jk_team_mask : jk_team_mask_default(&jk_forced);
-    bool team_k[kNumQuartetClasses] = {};
-    TeamScratchDev team_scr[kNumQuartetClasses]{};
-    TeamShape team_sh[kNumQuartetClasses]{};
+    const unsigned jk_mask = jk_forced ? (unsigned)h->jk_team_mask : jk_team_mask_default(&jk_forced);
+    bool team_want[kNumQuartetClasses] = {};
     for (int k = 0; k < kNumQuartetClasses; ++k)
     {
         long long gb = 0, ge = 0;
         shard_range(h, k, gb, ge);
-        const long long span = ge - gb;
-        if (((jk_mask >> k) & 1u) && h->work[k].total > 0 && (jk_forced || span >= kJKTeamMinQuartets))
-            team_k[k] = team_scratch(h, k, team_scr[k], team_sh[k]);
+        if (ge <= gb || fp32_below >= HUGE_VAL) continue;
+        const unsigned mask = jk_forced                 ? jk_mask
+                              : team_kmax(h, k) == 1 ? jk_mask | (unsigned)(QCG_JK_TEAM_PLAIN_MASK)
+                                                     : jk_mask | (unsigned)(QCG_JK_TEAM_CONTRACTED_MASK);
+        team_want[k] = (mask >> k) & 1u;
     }
-    for (int k = 0; k < kNumQuartetClasses; ++k)   // the buffer may have grown after an earlier class's lookup
-        if (team_k[k]) team_scratch(h, k, team_scr[k], team_sh[k]);
+    JKTeamPlan team;
+    jk_team_plan(h, team_want, jk_forced, team);
     // classes in the warp-shared form (FP64 band, one rank, not deterministic; the team form comes first);
     // their work items are built here, before any capture.  The build's default applies to full builds of
     // classes with at least kJKTeamMinQuartets quartets: under density screening a warp evaluates every
@@ -2158,9 +2323,9 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
         warp_forced ? (unsigned)h->jk_warp_mask : jk_warp_mask_default(&warp_forced);
     bool warp_k[kNumQuartetClasses] = {};
     for (int k = 0; k < kNumQuartetClasses; ++k)
-        if (((warp_mask >> k) & 1u) && !team_k[k] && h->work[k].total > 0 && h->shard_world == 1 &&
+        if (((warp_mask >> k) & 1u) && !team.on[k] && h->work[k].total > 0 && h->shard_world == 1 &&
             !(flags & QCG_JK_DETERMINISTIC) &&
-            (warp_forced || (dmax == nullptr && dthr <= 0.0 && h->work[k].total >= kJKTeamMinQuartets)))
+            (warp_forced || (dmax == nullptr && dthr <= 0.0 && h->work[k].total >= kJKWarpMinQuartets)))
         {
             warp_items(h, k);
             warp_k[k] = h->nwitems[k] > 0;
@@ -2200,9 +2365,12 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
             {
                 wk.lo = fp32_below;
                 wk.hi = HUGE_VAL;
-                if (team_k[k])
+                if (team.on[k])
+                {
                     kJKTeamLaunchers[k](wk, h->pl_dev[X], h->pl_dev[Y], h->pp_dev, h->d_f0, dD, h->d_Jp, h->d_Kp, n,
-                                        h->d_boys, team_scr[k], team_sh[k], h->side[0]);
+                                        h->d_boys, team.scr[k], team.sh[k], h->side[team.side ? slot : 0]);
+                    if (team.side) slot = (slot + 1) % qcg_handle::kSide;
+                }
                 else if (warp_k[k])
                 {
                     kJKWarpLaunchers[k](wk, h->pl_dev[X], h->pl_dev[Y], h->pp_dev, h->d_f0, dD, h->d_Jp, h->d_Kp, n,
@@ -2534,13 +2702,9 @@ unsigned eri_team_mask()
     return mask;
 }
 
-// the team form's scratch for class k: one wave of CTAs, each with stage slots for the class's longest
-// primitive loop in this basis (the product of the largest contraction lengths of the four angular
-// momenta) and its recurrence blocks.  False when that exceeds kTeamScratchMax bytes; the batch then runs in
-// the thread-per-quartet form.
-constexpr long long kTeamScratchMax = 4LL << 30;
-
-bool team_scratch(qcg_handle* h, int k, TeamScratchDev& scr, TeamShape& sh)
+// the longest primitive loop of class k in this basis: the product of the largest contraction lengths of its four
+// angular momenta
+int team_kmax(qcg_handle* h, int k)
 {
     int X = 0;
     while ((X + 1) * (X + 2) / 2 <= k) ++X;
@@ -2554,45 +2718,71 @@ bool team_scratch(qcg_handle* h, int k, TeamScratchDev& scr, TeamShape& sh)
                 if (h->L[i] == l) mx = std::max(mx, h->nprim[i]);
             h->maxnp[l] = mx;
         }
-    long long kmax = 1;
+    int kmax = 1;
     for (int l : Ls) kmax *= h->maxnp[l];
-    sh = kEriTeamShapes[k](h->nsm);
-    long long need = (long long)sh.grid * (kmax * sh.slot_doubles + sh.hrr_doubles);
-    if (kmax == 1) need = std::max(need, (long long)sh.grid * sh.slot_doubles + sh.group_doubles);
-    if (need * (long long)sizeof(double) > kTeamScratchMax) return false;
-    if (need > h->team_cap)
-    {
-        if (h->d_team) h->release(h->d_team);
-        h->d_team = nullptr;
-        h->team_cap = 0;
-        h->d_team = h->alloc<double>((size_t)need);
-        h->team_cap = need;
-    }
+    return kmax;
+}
+
+// the team launch shape of class k (an occupancy query, made once per handle)
+const TeamShape& team_shape(qcg_handle* h, int k)
+{
+    if (!h->team_shapes[k].nsm) h->team_shapes[k] = kEriTeamShapes[k](h->nsm);
+    return h->team_shapes[k];
+}
+
+// the error word of the team kernels, read by the next check_team_error
+int* team_error_word(qcg_handle* h)
+{
     if (!h->d_team_err)
     {
         h->d_team_err = h->alloc<int>(1);
         CK(cudaMemsetAsync(h->d_team_err, 0, sizeof(int), h->stream));
     }
-    scr.rcache = h->d_team;
-    scr.kmax = (int)kmax;
-    scr.hrr = h->d_team + (long long)sh.grid * kmax * sh.slot_doubles;
-    scr.err = h->d_team_err;
     h->team_pending = true;
+    return h->d_team_err;
+}
+
+// the team form's scratch for a batch of nq quartets of class k: at most one wave of CTAs, each with stage slots for the class's
+// longest primitive loop in this basis and its recurrence blocks.  False when that exceeds kTeamScratchMax bytes;
+// the batch then runs in the thread-per-quartet form.
+bool team_scratch(qcg_handle* h, int k, long long nq, TeamScratchDev& scr, TeamShape& sh)
+{
+    const long long kmax = team_kmax(h, k);
+    sh = team_shape(h, k);
+    sh.grid = (int)std::min<long long>(sh.grid, (nq + 31) / 32);
+    const long long need = (long long)sh.grid * (kmax * sh.slot_doubles + sh.hrr_doubles);
+    if (need * (long long)sizeof(double) > kTeamScratchMax) return false;
+    scr.rcache = h->scratch(h->team_scr, need);
+    scr.kmax = (int)kmax;
+    scr.hrr = scr.rcache + (long long)sh.grid * kmax * sh.slot_doubles;
+    scr.err = team_error_word(h);
     return true;
 }
 
 // the team kernels' error word (a bulk-copy wait that gave up, or a group longer than the stage slots):
 // read after a synchronising call, then cleared
-void check_team_error(qcg_handle* h)
+void raise_team_error(qcg_handle* h, int e)
 {
-    if (!h->d_team_err || !h->team_pending) return;
     h->team_pending = false;
-    int e = 0;
-    CK(cudaMemcpy(&e, h->d_team_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (!e) return;
     CK(cudaMemset(h->d_team_err, 0, sizeof(int)));
     throw Error{QCG_ERR_CUDA, e & 1 ? "team kernel: a bulk-copy wait gave up; the results are not valid"
                                     : "team kernel: a primitive loop longer than the stage slots"};
+}
+void check_team_error(qcg_handle* h)
+{
+    if (!h->d_team_err || !h->team_pending) return;
+    int e = 0;
+    CK(cudaMemcpy(&e, h->d_team_err, sizeof(int), cudaMemcpyDeviceToHost));
+    raise_team_error(h, e);
+}
+// the same without a synchronising copy of its own: queue_team_error before the caller's synchronisation of the
+// handle's stream, into pinned memory, raise_team_error with the value after it
+void queue_team_error(qcg_handle* h, int* pinned)
+{
+    *pinned = 0;
+    if (h->d_team_err && h->team_pending)
+        CK(cudaMemcpyAsync(pinned, h->d_team_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
 }
 
 #ifndef QCG_JK_TEAM_DEFAULT_MASK
@@ -2622,16 +2812,15 @@ long long batch_chunk_bytes()
 
 // the scratch of a form that is not required of the call: false, with nothing held, where the handle's memory
 // limit or the device does not have it
-bool team_scratch_optional(qcg_handle* h, int k, TeamScratchDev& scr, TeamShape& sh)
+bool team_scratch_optional(qcg_handle* h, int k, long long nq, TeamScratchDev& scr, TeamShape& sh)
 {
     try
     {
-        return team_scratch(h, k, scr, sh);
+        return team_scratch(h, k, nq, scr, sh);
     }
     catch (const Error& e)
     {
         if (e.code != QCG_ERR_ALLOC) throw;
-        cudaGetLastError();
         return false;
     }
 }
@@ -2651,7 +2840,7 @@ void eri_batch_launch(qcg_handle* h, int k, const int* dq, long long m, T* dout)
     sh.nsm = h->nsm;
     const bool ss_ket = k == 0 || k == 1 || k == 3 || k == 6 || k == 10 || k == 15;
     const bool team = ((mask >> k) & 1u) &&
-                      (ss_ket || (f64 ? team_scratch(h, k, scr, sh) : team_scratch_optional(h, k, scr, sh)));
+                      (ss_ket || (f64 ? team_scratch(h, k, m, scr, sh) : team_scratch_optional(h, k, m, scr, sh)));
     const int4* q = (const int4*)dq;
     if constexpr (f64)
     {
@@ -3435,7 +3624,8 @@ int qcg_rhf(qcg_handle* h, int natom, const double* Z, const double* R, int nele
         std::vector<double>& D = sc.D;
         std::vector<double> J(nn), K(nn);
         // the density goes up and J, K come back every iteration: through pinned (cached) host arrays
-        PinnedArray Dpin(nn), Jpin(nn), Kpin(nn);
+        PinnedArray Dpin(nn), Jpin(nn), Kpin(nn + 1);
+        int* const team_err = (int*)(Kpin.p + nn);
         std::vector<double> Dc(sph ? nn : 0), Js(sph ? (size_t)nw * nw : 0), Ks(sph ? (size_t)nw * nw : 0);
         std::vector<double> Dprev, Jprev, Kprev;
         double fock_ms = 0;
@@ -3506,8 +3696,9 @@ int qcg_rhf(qcg_handle* h, int natom, const double* Z, const double* R, int nele
             const auto c1 = clk::now();
             CK(cudaMemcpyAsync(Jpin.p, h->d_J, nn * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
             CK(cudaMemcpyAsync(Kpin.p, h->d_K, nn * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+            queue_team_error(h, team_err);
             CK(cudaStreamSynchronize(h->stream));
-            check_team_error(h);
+            raise_team_error(h, *team_err);
             std::copy(Jpin.p, Jpin.p + nn, J.begin());
             std::copy(Kpin.p, Kpin.p + nn, K.begin());
             const auto c2 = clk::now();
