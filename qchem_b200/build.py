@@ -128,12 +128,12 @@ def _jobs():
     for k in range(NCLASS):
         defs = [f"-DQCG_CLASS={k}"]
         parts = [_read(team_src), _read(os.path.join(GEN, f"md_team_{k}.cuh"))]
-        key = _hash(parts + core + _headers(["eri_kernels.cuh", "eri_team.cuh", "eri_ss.cuh", "jk_group.cuh", "eri_team_iface.h", "team_sync.cuh", "smem_attr.h"])
+        key = _hash(parts + core + _headers(["eri_kernels.cuh", "eri_team.cuh", "eri_ss.cuh", "jk_group.cuh", "eri_team_iface.h", "team_sync.cuh", "smem_attr.h", "batch_plan.h"])
                     + FLAGS + defs)
         jobs.append((team_src, defs, os.path.join(BUILD, f"eri_team_{k}_{key}.o")))
-    extra = {"runtime.cu": _headers(["boys_table.h", "eri_team_iface.h"]) + [_read(os.path.join(INCLUDE, "qchem_b200.h"))],
-             "registry.cu": _headers(["eri_team_iface.h"]),
-             "fock_kernels.cu": _headers(["team_sync.cuh"]),
+    extra = {"runtime.cu": _headers(["boys_table.h", "eri_team_iface.h", "batch_plan.h"]) + [_read(os.path.join(INCLUDE, "qchem_b200.h"))],
+             "registry.cu": _headers(["eri_team_iface.h", "batch_plan.h"]),
+             "fock_kernels.cu": _headers(["team_sync.cuh", "batch_plan.h"]),
              "mlp.cu": [_read(os.path.join(INCLUDE, "qchem_b200.h"))] + _headers(["smem_attr.h", "team_sync.cuh"])}
     for name in ("registry.cu", "fock_kernels.cu", "runtime.cu", "mlp.cu"):
         s = os.path.join(CSRC, name)

@@ -68,7 +68,7 @@ constexpr size_t team_smem(int stage)
 // CTAs per SM to compile for: about twelve warps, as far as their shared memory fits
 constexpr int team_min_blocks(int ng, int stage)
 {
-    const int fit = (int)((227 * 1024) / (team_smem(stage) + 1024)), want = 12 / (3 * ng);
+    const int fit = (int)((227 * 1024) / (team_smem(stage) + sizeof(BatchPlanDev) + 2048)), want = 12 / (3 * ng);
     const int m = fit < want ? fit : want;
     return m < 1 ? 1 : m;
 }
@@ -177,10 +177,8 @@ void launch_batch(const BasisDev& bs, const int4* q, const int* order, long long
     auto k = eri_batch_team_kernel<Cls, OT>;
     static std::atomic<unsigned long long> ready{0};
     ensure_smem(k, kSmem, ready);
-    // one wave of CTAs, each walking groups of 32 quartets; the scratch has room for sh.grid CTAs
-    const long long ngroups = (nq + 31) / 32;
-    const long long blocks = ngroups < sh.grid ? ngroups : sh.grid;
-    k<<<(unsigned)blocks, kThreads, kSmem, st>>>(bs, q, order, nq, out, boys, scr);
+    // one wave of CTAs, each walking groups of the plan; the scratch has room for sh.grid CTAs
+    k<<<(unsigned)sh.grid, kThreads, kSmem, st>>>(bs, q, order, out, boys, scr);
 }
 #if QCG_SS_KET
 template <class OT, int SPLIT>

@@ -1,7 +1,8 @@
 // eri_team.cuh -- warp-specialised ERI-batch kernel for the high-L classes (team form).
 //
-// A CTA takes 32 contracted quartets at a time (a "group": 32 consecutive entries of the batch's visiting
-// order, which groups equal contraction patterns), one per lane, and works through them in three phases.
+// A CTA takes 32 contracted quartets of one contraction pattern at a time (a "group": batch_plan.h), one per lane
+// -- or, where a batch is too small to hide a long primitive loop, fewer quartets with the bra primitive pairs of
+// each split over several lanes, whose [e0|f0] are added -- and works through them in three phases.
 //
 //  1. Stage tables.  For every primitive quartet x of the group (bra primitive pair outer, ket inner) and
 //     every lane, a "stage" holds R^0_{tuv} scaled by the prefactor lambda and the single-centre Hermite
@@ -186,7 +187,7 @@ __device__ __forceinline__ bool team_contract(const double* __restrict__ rc, dou
 // OT: the output type.  Float output (the FP32 batches) is the FP64 evaluation rounded once.
 template <class Cls, class OT>
 __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
-    eri_batch_team_kernel(BasisDev bs, const int4* __restrict__ quartets, const int* __restrict__ order, long long nq,
+    eri_batch_team_kernel(BasisDev bs, const int4* __restrict__ quartets, const int* __restrict__ order,
                           OT* __restrict__ out, const double* __restrict__ boys_table, TeamScratchDev scr)
 {
     constexpr int NW = Cls::kNW;
@@ -209,13 +210,23 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     double* const hA = scr.hrr + (long long)blockIdx.x * (NE * NF + NE * NCD) * 32;
     double* const hB = hA + NE * NF * 32;
     unsigned long long G = 0;   // steps streamed so far: step G uses stage G % 3, phase (G / 3) & 1
-    const long long ngroups = (nq + 31) >> 5;
-    for (long long g = blockIdx.x; g < ngroups; g += gridDim.x)
+    __shared__ BatchPlanDev plan;
+    __shared__ int lane_q[32];   // each lane's quartet, for the phases after the contraction; -1: none
+    for (int k = threadIdx.x; k < (int)(sizeof(BatchPlanDev) / sizeof(int)); k += blockDim.x)
+        reinterpret_cast<int*>(&plan)[k] = reinterpret_cast<const int*>(scr.plan)[k];
+    __syncthreads();
+    const int ngroups = plan.group[256];
+    int b = 0;   // the group's bucket: groups come in increasing order
+    for (int g = blockIdx.x; g < ngroups; g += gridDim.x)
     {
-        // every warp reads the same 32 quartets: lane l of every warp holds quartet l of the group
-        const long long gi = g * 32 + lane;
-        const bool valid = gi < nq;
-        const long long q = valid ? (order ? (long long)order[gi] : gi) : 0;
+        while (plan.group[b + 1] <= g) ++b;
+        // every warp reads the same quartets: lane l of every warp holds bra primitive pairs sub, sub + S, ... of its
+        // quartet, S = 1 << lg
+        const int lg = plan.lanes[b], sub = lane & ((1 << lg) - 1);
+        const int gi = plan.first[b] + (g - plan.group[b]) * (32 >> lg) + (lane >> lg);
+        const bool valid = gi < plan.first[b + 1];
+        const long long q = valid ? (long long)order[gi] : 0;
+        if (warp == 0) lane_q[lane] = valid && sub == 0 ? (int)q : -1;
         const int4 s = quartets[q];
         int ni = 0, nj = 0, nk = 0, nl = 0;
         if (valid)
@@ -225,7 +236,8 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
             nk = bs.nprim[s.z];
             nl = bs.nprim[s.w];
         }
-        const int Kcd = nk * nl, K = ni * nj * Kcd;
+        const int Kab = sub < ni * nj ? (ni * nj - sub - 1 >> lg) + 1 : 0;   // this lane's bra primitive pairs
+        const int Kcd = nk * nl, K = Kab * Kcd;
         const int Kg = __reduce_max_sync(0xffffffffu, K);   // the group's longest primitive loop (CTA-uniform)
         if (Kg > scr.kmax)
         {
@@ -234,26 +246,43 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         }
         // 1. stage tables of every primitive quartet, written once to the R cache
         team_stages<Cls>(
-            rc, ni * nj, Kcd, Kg, bt, [&](int ij) { return shell_prim_pair(bs, s.x, ij / nj, s.y, ij % nj); },
+            rc, Kab, Kcd, Kg, bt,
+            [&](int m) {
+                const int ij = (m << lg) + sub;
+                return shell_prim_pair(bs, s.x, ij / nj, s.y, ij % nj);
+            },
             [&](int kl) { return shell_prim_pair(bs, s.z, kl / nl, s.w, kl % nl); });
         // 2. contraction, the stages streamed back through shared memory three deep
         if (!team_contract<Cls>(rc, hA, K, Kcd, Kg, G, full, scr.err)) return;
-        // 3. recurrences: ket per e row into [e0|cd], bra per (c d) column into the output block
-        const double* A = bs.cen + 3 * s.x;
-        const double* B = bs.cen + 3 * s.y;
-        const double* C = bs.cen + 3 * s.z;
-        const double* D = bs.cen + 3 * s.w;
-        if (valid)
+        // the lanes that share a quartet add their [e0|f0]
+        if (const int share = plan.lanes[b]; share > 0)
         {
+            for (int k = warp; k < NE * NF; k += NW)
+            {
+                double v = hA[k * 32 + lane];
+                for (int o = 1; o < 1 << share; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                hA[k * 32 + lane] = v;
+            }
+            __syncthreads();
+        }
+        // 3. recurrences: ket per e row into [e0|cd], bra per (c d) column into the output block
+        const int hq = lane_q[lane];
+        const int4 hs = quartets[hq < 0 ? 0 : hq];
+        if (hq >= 0)
+        {
+            const double* const C = bs.cen + 3 * hs.z;
+            const double* const D = bs.cen + 3 * hs.w;
             const double CDx = C[0] - D[0], CDy = C[1] - D[1], CDz = C[2] - D[2];
             for (int e = warp; e < NE; e += NW)
                 Cls::hrr_ket(hA + e * NF * 32 + lane, hB + e * NCD * 32 + lane, CDx, CDy, CDz);
         }
         __syncthreads();
-        if (valid)
+        if (hq >= 0)
         {
+            const double* const A = bs.cen + 3 * hs.x;
+            const double* const B = bs.cen + 3 * hs.y;
             const double ABx = A[0] - B[0], ABy = A[1] - B[1], ABz = A[2] - B[2];
-            OT* const o = out + q * BLK;
+            OT* const o = out + hq * BLK;
             for (int cd = warp; cd < NCD; cd += NW) Cls::hrr_bra(hB + cd * 32 + lane, o + cd, NCD, ABx, ABy, ABz);
         }
         __syncthreads();   // the scratch and the R cache are free for the next group

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "batch_plan.h"
 #include "qcg_internal.h"
 
 namespace qcg {
@@ -18,6 +19,7 @@ struct TeamScratchDev
     int kmax;
     double* hrr;
     int* err;
+    const BatchPlanDev* plan;   // ERI batches: the groups
 };
 
 // The launch shape of class k on nsm SMs and the scratch it needs per CTA, in doubles.

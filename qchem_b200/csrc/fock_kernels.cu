@@ -2,6 +2,7 @@
 // and the one-electron integrals (overlap, kinetic, nuclear attraction) of the RHF Hamiltonian.
 #include <algorithm>
 
+#include "batch_plan.h"
 #include "md_core.cuh"
 #include "qcg_internal.h"
 #include "team_sync.cuh"
@@ -73,7 +74,60 @@ __global__ void symmetrize_kernel(const double* __restrict__ Jp, const double* _
 // Grouping of an ERI batch by contraction pattern (counting sort over 256 buckets): the batch kernels
 // then visit quartets with equal primitive-loop shapes in the same warp.
 // ------------------------------------------------------------------------------------------------
-// contraction-pattern key of every quartet (primitive counts up to 4 per shell; larger ones share a bucket)
+// contraction-pattern key of a quartet (primitive counts up to 4 per shell; larger ones share a bucket)
+__device__ __forceinline__ int pattern_key(const BasisDev& bs, const int4 s)
+{
+    const int a = min(bs.nprim[s.x], 4) - 1, b = min(bs.nprim[s.y], 4) - 1, c = min(bs.nprim[s.z], 4) - 1,
+              d = min(bs.nprim[s.w], 4) - 1;
+    return ((a * 4 + b) * 4 + c) * 4 + d;
+}
+
+// The visiting order of the buckets and the groups the team kernel cuts them into, by a block of 256 threads from
+// the bucket counts n[256] in shared memory; returns the first position of bucket threadIdx.x.
+// A group is 32 lanes of one pattern; S lanes share a quartet, taking its bra primitive pairs in turn.  S is 1 as
+// long as a quartet's primitive loop is no longer than a CTA's average share of all loops; a longer one (up to
+// 81 primitive quartets, a serial chain that alone outlasted the rest of a small batch) is split until it is.
+// Buckets go by decreasing loop length, so that the long loops start first and the short ones fill the last wave.
+// 32 quartets of each of 21 classes: 2.50 -> 0.95 ms; 3001 each 2.86 -> 1.93; 20 011 each 5.0 -> 4.7.
+__device__ int pattern_plan(const int* n, int ctas, BatchPlanDev* __restrict__ plan)
+{
+    __shared__ int w[256], rn[256], rg[256];
+    __shared__ unsigned long long all;
+    const int t = threadIdx.x;
+    const int kab = ((t >> 6) + 1) * (((t >> 4) & 3) + 1), kcd = (((t >> 2) & 3) + 1) * ((t & 3) + 1);
+    if (t == 0) all = 0;
+    __syncthreads();
+    if (n[t]) atomicAdd(&all, (unsigned long long)n[t] * (kab * kcd));
+    __syncthreads();
+    const int share = (int)min((unsigned long long)(1 << 20), all / (32ull * ctas));
+    const int most = max(share, kBatchChain);
+    int l = 0;
+    while (l < 4 && (1 << l) < kab && ((kab + (1 << l) - 1) >> l) * kcd > most) ++l;
+    w[t] = ((kab + (1 << l) - 1) >> l) * kcd;
+    __syncthreads();
+    int rank = 0;
+    for (int u = 0; u < 256; ++u)
+        if (w[u] > w[t] || (w[u] == w[t] && u < t)) ++rank;
+    rn[rank] = n[t];
+    rg[rank] = (int)((((long long)n[t] << l) + 31) >> 5);
+    __syncthreads();
+    int before = 0, groups = 0;
+    for (int r = 0; r < rank; ++r)
+    {
+        before += rn[r];
+        groups += rg[r];
+    }
+    plan->first[rank] = before;
+    plan->group[rank] = groups;
+    plan->lanes[rank] = l;
+    if (rank == 255)
+    {
+        plan->first[256] = before + rn[255];
+        plan->group[256] = groups + rg[255];
+    }
+    return before;
+}
+
 __global__ void pattern_key_kernel(BasisDev bs, const int4* __restrict__ quartets, long long nq,
                                    unsigned char* __restrict__ key, int* __restrict__ hist)
 {
@@ -82,10 +136,7 @@ __global__ void pattern_key_kernel(BasisDev bs, const int4* __restrict__ quartet
     __syncthreads();
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nq; q += (long long)gridDim.x * blockDim.x)
     {
-        const int4 s = quartets[q];
-        const int a = min(bs.nprim[s.x], 4) - 1, b = min(bs.nprim[s.y], 4) - 1, c = min(bs.nprim[s.z], 4) - 1,
-                  d = min(bs.nprim[s.w], 4) - 1;
-        const int k = ((a * 4 + b) * 4 + c) * 4 + d;
+        const int k = pattern_key(bs, quartets[q]);
         key[q] = (unsigned char)k;
         atomicAdd(&h[k], 1);
     }
@@ -94,20 +145,13 @@ __global__ void pattern_key_kernel(BasisDev bs, const int4* __restrict__ quartet
         if (h[i]) atomicAdd(&hist[i], h[i]);
 }
 
-// First position of every bucket (one block of 256 threads).  Buckets go by decreasing primitive-quartet count:
-// the batch kernels hand out groups of neighbouring quartets round robin, so the long primitive loops start
-// first and the short ones fill the last wave.
-__global__ void pattern_scan_kernel(const int* __restrict__ hist, int* __restrict__ cursor)
+__global__ void pattern_scan_kernel(const int* __restrict__ hist, int* __restrict__ cursor, int ctas,
+                                    BatchPlanDev* __restrict__ plan)
 {
-    __shared__ int n[256], w[256];
-    const int t = threadIdx.x;
-    n[t] = hist[t];
-    w[t] = ((t >> 6) + 1) * (((t >> 4) & 3) + 1) * (((t >> 2) & 3) + 1) * ((t & 3) + 1);
+    __shared__ int n[256];
+    n[threadIdx.x] = hist[threadIdx.x];
     __syncthreads();
-    int before = 0;
-    for (int u = 0; u < 256; ++u)
-        if (w[u] > w[t] || (w[u] == w[t] && u < t)) before += n[u];
-    cursor[t] = before;
+    cursor[threadIdx.x] = pattern_plan(n, ctas, plan);
 }
 
 __global__ void pattern_scatter_kernel(const unsigned char* __restrict__ key, long long nq, int* __restrict__ cursor,
@@ -117,13 +161,40 @@ __global__ void pattern_scatter_kernel(const unsigned char* __restrict__ key, lo
         order[atomicAdd(&cursor[key[q]], 1)] = (int)q;
 }
 
-void launch_pattern_sort(const BasisDev& bs, const int4* quartets, long long nq, unsigned char* key, int* hist,
-                         int* cursor, int* order, cudaStream_t st, int nsm)
+// The three steps above by one block, for batches that one block sorts sooner than four launches start.
+constexpr long long kSortSmall = 4096;
+__global__ void __launch_bounds__(256)
+    pattern_sort_small_kernel(BasisDev bs, const int4* __restrict__ quartets, int nq, int* __restrict__ order, int ctas,
+                              BatchPlanDev* __restrict__ plan)
 {
+    __shared__ int n[256], cursor[256];
+    __shared__ unsigned char key[kSortSmall];
+    n[threadIdx.x] = 0;
+    __syncthreads();
+    for (int q = threadIdx.x; q < nq; q += 256)
+    {
+        const int k = pattern_key(bs, quartets[q]);
+        key[q] = (unsigned char)k;
+        atomicAdd(&n[k], 1);
+    }
+    __syncthreads();
+    cursor[threadIdx.x] = pattern_plan(n, ctas, plan);
+    __syncthreads();
+    for (int q = threadIdx.x; q < nq; q += 256) order[atomicAdd(&cursor[key[q]], 1)] = q;
+}
+
+void launch_pattern_sort(const BasisDev& bs, const int4* quartets, long long nq, unsigned char* key, int* hist,
+                         int* cursor, int* order, int ctas, BatchPlanDev* plan, cudaStream_t st, int nsm)
+{
+    if (nq <= kSortSmall)
+    {
+        pattern_sort_small_kernel<<<1, 256, 0, st>>>(bs, quartets, (int)nq, order, ctas, plan);
+        return;
+    }
     cudaMemsetAsync(hist, 0, 256 * sizeof(int), st);
     const long long blocks = std::min<long long>((nq + 255) / 256, (long long)nsm * 8);
     pattern_key_kernel<<<(unsigned)blocks, 256, 0, st>>>(bs, quartets, nq, key, hist);
-    pattern_scan_kernel<<<1, 256, 0, st>>>(hist, cursor);
+    pattern_scan_kernel<<<1, 256, 0, st>>>(hist, cursor, ctas, plan);
     pattern_scatter_kernel<<<(unsigned)blocks, 256, 0, st>>>(key, nq, cursor, order);
 }
 

@@ -419,6 +419,7 @@ struct qcg_handle
     long long sort_cap = 0;
     unsigned char* d_key = nullptr;
     int *d_order = nullptr, *d_hist = nullptr, *d_cursor = nullptr;
+    BatchPlanDev* d_plan = nullptr;
 
     // team-form ERI batches (eri_team.cu): per-CTA R cache and recurrence scratch (grow only), error word
     // scratch of the team kernels: ERI batches, and J/K builds (whose address recorded graphs hold)
@@ -2470,19 +2471,24 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
 }
 
 // grouped visiting order of a batch (returns the device permutation)
-const int* batch_order(qcg_handle* h, const int* d_quartets, long long nq)
+const int* batch_order(qcg_handle* h, const int* d_quartets, long long nq, int ctas)
 {
     require(nq <= 0x7fffffffLL, "at most 2^31-1 quartets per batch");
     if (nq > h->sort_cap)
     {
         if (h->d_key) { h->release(h->d_key); h->release(h->d_order); }
-        if (!h->d_hist) { h->d_hist = h->alloc<int>(256); h->d_cursor = h->alloc<int>(256); }
+        if (!h->d_hist)
+        {
+            h->d_hist = h->alloc<int>(256);
+            h->d_cursor = h->alloc<int>(256);
+            h->d_plan = h->alloc<BatchPlanDev>(1);
+        }
         h->d_key = h->alloc<unsigned char>(nq);
         h->d_order = h->alloc<int>(nq);
         h->sort_cap = nq;
     }
-    launch_pattern_sort(h->bs, (const int4*)d_quartets, nq, h->d_key, h->d_hist, h->d_cursor, h->d_order, h->stream,
-                        h->nsm);
+    launch_pattern_sort(h->bs, (const int4*)d_quartets, nq, h->d_key, h->d_hist, h->d_cursor, h->d_order, ctas,
+                        h->d_plan, h->stream, h->nsm);
     CK(cudaGetLastError());
     return h->d_order;
 }
@@ -2749,7 +2755,7 @@ bool team_scratch(qcg_handle* h, int k, long long nq, TeamScratchDev& scr, TeamS
 {
     const long long kmax = team_kmax(h, k);
     sh = team_shape(h, k);
-    sh.grid = (int)std::min<long long>(sh.grid, (nq + 31) / 32);
+    sh.grid = (int)std::min<long long>(sh.grid, nq);   // a group has at least one quartet
     const long long need = (long long)sh.grid * (kmax * sh.slot_doubles + sh.hrr_doubles);
     if (need * (long long)sizeof(double) > kTeamScratchMax) return false;
     scr.rcache = h->scratch(h->team_scr, need);
@@ -2833,7 +2839,6 @@ template <class T>
 void eri_batch_launch(qcg_handle* h, int k, const int* dq, long long m, T* dout)
 {
     constexpr bool f64 = std::is_same_v<T, double>;
-    const int* order = batch_order(h, dq, m);
     const unsigned mask = f64 ? (h->team_mask >= 0 ? (unsigned)h->team_mask : eri_team_mask()) : ~0u;
     TeamScratchDev scr{};
     TeamShape sh{};
@@ -2841,6 +2846,8 @@ void eri_batch_launch(qcg_handle* h, int k, const int* dq, long long m, T* dout)
     const bool ss_ket = k == 0 || k == 1 || k == 3 || k == 6 || k == 10 || k == 15;
     const bool team = ((mask >> k) & 1u) &&
                       (ss_ket || (f64 ? team_scratch(h, k, m, scr, sh) : team_scratch_optional(h, k, m, scr, sh)));
+    const int* order = batch_order(h, dq, m, team && !ss_ket ? sh.grid : h->nsm);
+    scr.plan = h->d_plan;
     const int4* q = (const int4*)dq;
     if constexpr (f64)
     {
