@@ -55,20 +55,24 @@ constexpr int team_pieces(int ncode, int nh, int ne)
     const int npass = (ncode + g - 1) / g;
     return (ncode + npass - 1) / npass;
 }
-// Doubles of the stage space: three stages, and at least 18 primitive pairs (contractions of three).
-constexpr int team_stage_space(int stage)
+// Doubles of the stage space: three stages, and at least 18 primitive pairs (contractions of three) and the columns
+// of the bra recurrence that go out together.
+constexpr int team_stage_space(int ng, int stage)
 {
-    const int pairs = 18 * kTeamPairDoubles;
-    return (3 * stage > pairs ? 3 * stage : pairs) * 32;
+    const int ncd = ncart(kPairLA[kY]) * ncart(kPairLB[kY]), nab = ncart(kPairLA[kX]) * ncart(kPairLB[kX]);
+    const int columns = nab * (ncd < 3 * ng ? ncd : 3 * ng) * 33;
+    int n = 18 * kTeamPairDoubles * 32;
+    if (n < 3 * stage * 32) n = 3 * stage * 32;
+    return n < columns ? columns : n;
 }
-constexpr size_t team_smem(int stage)
+constexpr size_t team_smem(int ng, int stage)
 {
-    return (size_t)(team_stage_space(stage) + kBoysRows * kBoysColumns) * sizeof(double);
+    return (size_t)(team_stage_space(ng, stage) + kBoysRows * kBoysColumns) * sizeof(double);
 }
 // CTAs per SM to compile for: about twelve warps, as far as their shared memory fits
 constexpr int team_min_blocks(int ng, int stage)
 {
-    const int fit = (int)((227 * 1024) / (team_smem(stage) + sizeof(BatchPlanDev) + 2048)), want = 12 / (3 * ng);
+    const int fit = (int)((227 * 1024) / (team_smem(ng, stage) + sizeof(BatchPlanDev) + 2048)), want = 12 / (3 * ng);
     const int m = fit < want ? fit : want;
     return m < 1 ? 1 : m;
 }
@@ -100,7 +104,7 @@ struct Cls
     using View = gen::QCG_CAT(TeamView, QCG_CLASS)<double>;
     static __device__ __forceinline__ constexpr int fslot(int jc) { return gen::QCG_CAT(team_fslot_, QCG_CLASS)(jc); }
     static __device__ __forceinline__ constexpr bool fixed(int jc) { return gen::QCG_CAT(team_ffixed_, QCG_CLASS)(jc); }
-    static constexpr int kStageSpace = team_stage_space(kStage), kPairSlots = kStageSpace / (32 * kTeamPairDoubles);
+    static constexpr int kStageSpace = team_stage_space(kNG, kStage), kPairSlots = kStageSpace / (32 * kTeamPairDoubles);
     static __device__ __forceinline__ void produce(double* st, const TeamPair& ab, const TeamPair& cd,
                                                    const BoysColumns& bt, bool bra_e)
     {
@@ -142,7 +146,7 @@ struct Cls
 
 constexpr int kThreads = Cls::kNW * 32;
 constexpr int kNCD = ncart(Cls::LC) * ncart(Cls::LD);
-constexpr size_t kSmem = team_smem(Cls::kStage);   // the stages and the Boys columns
+constexpr size_t kSmem = team_smem(Cls::kNG, Cls::kStage);   // the stages and the Boys columns
 constexpr size_t kGroupSmem =
     (2 * (size_t)Cls::kGroups * Cls::kStage * 32 + kBoysRows * kBoysColumns) * sizeof(double);
 std::atomic<unsigned long long> g_smem_ready{0};

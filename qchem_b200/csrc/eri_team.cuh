@@ -277,15 +277,35 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
                 Cls::hrr_ket(hA + e * NF * 32 + lane, hB + e * NCD * 32 + lane, CDx, CDy, CDz);
         }
         __syncthreads();
-        if (hq >= 0)
+        // the bra recurrence of W neighbouring columns at a time into the stage space, one column per warp and lane,
+        // then out quartet by quartet: a quartet's runs of W values go out by neighbouring lanes.  (Each lane
+        // storing its own column wrote 8 bytes at 32 places, on 32 pages, per instruction.)
+        constexpr int NAB = ncart(Cls::LA) * ncart(Cls::LB), W = NCD < NW ? NCD : NW;
+        static_assert(NAB * W * 33 <= Cls::kStageSpace, "the columns fit the stage space");
+        for (int c0 = 0; c0 < NCD; c0 += W)
         {
-            const double* const A = bs.cen + 3 * hs.x;
-            const double* const B = bs.cen + 3 * hs.y;
-            const double ABx = A[0] - B[0], ABy = A[1] - B[1], ABz = A[2] - B[2];
-            OT* const o = out + hq * BLK;
-            for (int cd = warp; cd < NCD; cd += NW) Cls::hrr_bra(hB + cd * 32 + lane, o + cd, NCD, ABx, ABy, ABz);
+            const int width = c0 + W < NCD ? W : NCD - c0;
+            if (hq >= 0 && warp < width)
+            {
+                const double* const A = bs.cen + 3 * hs.x;
+                const double* const B = bs.cen + 3 * hs.y;
+                const double ABx = A[0] - B[0], ABy = A[1] - B[1], ABz = A[2] - B[2];
+                Cls::hrr_bra(hB + (c0 + warp) * 32 + lane, qcg_team_smem + warp * 33 + lane, W * 33, ABx, ABy, ABz);
+            }
+            __syncthreads();
+            for (int l = warp; l < 32; l += NW)
+            {
+                const int lq = lane_q[l];
+                if (lq < 0) continue;
+                OT* const o = out + lq * BLK + c0;
+                for (int k = lane; k < NAB * width; k += 32)
+                {
+                    const int ab = k / width, c = k - ab * width;
+                    o[ab * NCD + c] = (OT)qcg_team_smem[(ab * W + c) * 33 + l];
+                }
+            }
+            __syncthreads();
         }
-        __syncthreads();   // the scratch and the R cache are free for the next group
     }
 }
 
