@@ -2,6 +2,8 @@
 // fused ERI + J/K digestion.  Included by eri_class.cu, which is compiled once per quartet class and
 // supplies Cls::quartet (the generated straight-line primitive-quartet evaluation of that class).
 #pragma once
+#include <type_traits>
+
 #include "md_core.cuh"
 #include "qcg_internal.h"
 
@@ -381,6 +383,7 @@ struct JKSink
         for (int k = 0; k < NB; ++k) { acc(K, (size_t)(fb + k) * n + row_la, kbc[k]); kbc[k] = 0.0; }
         row_la = -1;
     }
+    __device__ __forceinline__ void quartet_begin() {}
     // the end of one quartet: in the deterministic mode J'[a b] leaves the registers after every quartet, so
     // that each quartet's contribution is rounded alone and the integer sums do not depend on how many
     // quartets a lane runs (the launch shape); the FP64 mode keeps summing over the lane's run
@@ -404,6 +407,149 @@ struct JKSink
                 const double x = jab[ia * NB + ib];
                 if (x != 0.0) acc(J, (size_t)(fa + ia) * n + fb + ib, 2.0 * x);
             }
+    }
+};
+
+// The digestion of the light classes (kWholeQuartet): J'(c d) and the four K' blocks of a quartet stay in registers
+// until its last integral, so that K'(a d), K'(b d) leave once per quartet and not once per c component ((pp|pp): 45
+// updates of J' and K' instead of 81), and no update stands between the loads of D, which the compiler then shares
+// among the components.  D(a b) is loaded once per bra pair.
+// WARP: for jk_warp_kernel, where the lanes of a half warp share a, c and d: J'(c d), K'(a d) and K'(a c) are added
+// over the half by shuffles and written once.
+template <int LA, int LB, int LC, int LD>
+constexpr bool kWholeQuartet =
+    (ncart(LA) + ncart(LB)) * (ncart(LC) + ncart(LD)) <= 28 && ncart(LA) * ncart(LB) <= 9;
+
+template <int P>
+__device__ __forceinline__ double half_warp_transpose_sum(double (&v)[P], int lane);
+constexpr int pow2_at_least(int v) { return v <= 1 ? 1 : 2 * pow2_at_least((v + 1) / 2); }
+
+template <class RT, int LA, int LB, int LC, int LD, bool DET, bool WARP>
+struct QuartetSink
+{
+    static constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NAB = NA * NB;
+    const double* __restrict__ D;
+    double* __restrict__ J;
+    double* __restrict__ K;
+    int n, fa, fb, fc, fd, lane = 0;
+    double s;   // symmetry weight; 0 for an absent quartet of a warp
+    long long det_lo = 0;
+    double dab[NAB], jab[NAB], jcd[NC * ND], kac[NA * NC], kad[NA * ND], kbc[NB * NC], kbd[NB * ND];
+    double dls, das[NA], dal[NA], dbs[NB], dbl[NB];
+
+    __device__ __forceinline__ void acc(double* M, size_t k, double v)
+    {
+        if constexpr (DET) fixed_add(M, k, det_lo, v);
+        else if (!WARP || v != 0.0) atomicAdd(M + k, v);
+    }
+    __device__ __forceinline__ void set_bra(int fa_, int fb_)
+    {
+        fa = fa_;
+        fb = fb_;
+#pragma unroll
+        for (int k = 0; k < NAB; ++k)
+        {
+            jab[k] = 0.0;
+            dab[k] = __ldg(D + (size_t)(fa + k / NB) * n + fb + k % NB);
+        }
+    }
+    __device__ __forceinline__ void quartet_begin()
+    {
+#pragma unroll
+        for (int k = 0; k < NC * ND; ++k) jcd[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < NA * NC; ++k) kac[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < NA * ND; ++k) kad[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < NB * NC; ++k) kbc[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < NB * ND; ++k) kbd[k] = 0.0;
+    }
+    __device__ __forceinline__ void ket_begin(int ic, int id)
+    {
+        const int la = fc + ic, si = fd + id;
+        dls = __ldg(D + (size_t)la * n + si);
+#pragma unroll
+        for (int k = 0; k < NA; ++k)
+        {
+            das[k] = __ldg(D + (size_t)(fa + k) * n + si);
+            dal[k] = __ldg(D + (size_t)(fa + k) * n + la);
+        }
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+        {
+            dbs[k] = __ldg(D + (size_t)(fb + k) * n + si);
+            dbl[k] = __ldg(D + (size_t)(fb + k) * n + la);
+        }
+    }
+    __device__ __forceinline__ void operator()(int ia, int ib, int ic, int id, RT v)
+    {
+        const double w = s * (double)v;   // FP64 accumulation in either arithmetic type
+        jab[ia * NB + ib] += w * dls;
+        jcd[ic * ND + id] += w * dab[ia * NB + ib];
+        kac[ia * NC + ic] += w * dbs[ib];
+        kbc[ib * NC + ic] += w * das[ia];
+        kad[ia * ND + id] += w * dbl[ib];
+        kbd[ib * ND + id] += w * dal[ia];
+    }
+    __device__ __forceinline__ void ket_end(int, int) {}
+    __device__ __forceinline__ void quartet_end()
+    {
+#pragma unroll
+        for (int k = 0; k < NB * NC; ++k) acc(K, (size_t)(fb + k / NC) * n + fc + k % NC, kbc[k]);
+#pragma unroll
+        for (int k = 0; k < NB * ND; ++k) acc(K, (size_t)(fb + k / ND) * n + fd + k % ND, kbd[k]);
+        if constexpr (WARP) flush_shared();
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < NC * ND; ++k) acc(J, (size_t)(fc + k / ND) * n + fd + k % ND, 2.0 * jcd[k]);
+#pragma unroll
+            for (int k = 0; k < NA * NC; ++k) acc(K, (size_t)(fa + k / NC) * n + fc + k % NC, kac[k]);
+#pragma unroll
+            for (int k = 0; k < NA * ND; ++k) acc(K, (size_t)(fa + k / ND) * n + fd + k % ND, kad[k]);
+        }
+        // each quartet's J'(a b) rounded alone (see JKSink::quartet_end)
+        if constexpr (DET)
+        {
+            flush_bra();
+#pragma unroll
+            for (int k = 0; k < NAB; ++k) jab[k] = 0.0;
+        }
+    }
+    // the targets shared by the half warp, up to sixteen at a time
+    __device__ __forceinline__ void flush_shared()
+    {
+        constexpr int NJ = NC * ND, N1 = NJ + NA * ND, V = N1 + NA * NC;
+#pragma unroll
+        for (int v0 = 0; v0 < V; v0 += 16) flush_some<(V < 16 ? pow2_at_least(V) : 16), NJ, N1, V>(v0);
+    }
+    template <int P, int NJ, int N1, int V>
+    __device__ __forceinline__ void flush_some(const int v0)
+    {
+        double v[P];
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+        {
+            const int x = v0 + k;
+            v[k] = x < NJ ? 2.0 * jcd[x < NJ ? x : 0]
+                   : x < N1 ? kad[x >= NJ && x < N1 ? x - NJ : 0]
+                   : x < V ? kac[x >= N1 && x < V ? x - N1 : 0] : 0.0;
+        }
+        const double sum = half_warp_transpose_sum<P>(v, lane);
+        constexpr int PER = 16 / P;   // lanes of the half that hold one value
+        const int x = v0 + (lane & 15) / PER;
+        if ((lane & (PER - 1)) != 0 || x >= V || sum == 0.0) return;
+        if (x < NJ) atomicAdd(J + (size_t)(fc + x / ND) * n + fd + x % ND, sum);
+        else if (x < N1) atomicAdd(K + (size_t)(fa + (x - NJ) / ND) * n + fd + (x - NJ) % ND, sum);
+        else atomicAdd(K + (size_t)(fa + (x - N1) / NC) * n + fc + (x - N1) % NC, sum);
+    }
+    __device__ __forceinline__ void flush_bra()
+    {
+#pragma unroll
+        for (int k = 0; k < NAB; ++k)
+            if (jab[k] != 0.0) acc(J, (size_t)(fa + k / NB) * n + fb + k % NB, 2.0 * jab[k]);
     }
 };
 
@@ -464,7 +610,10 @@ __global__ void __launch_bounds__(THREADS) jk_kernel(JKWorkDev w, PairListDev br
         }
         int i = lo;
         long long next = w.offs[i + 1];
-        JKSink<RT, Cls::LA, Cls::LB, Cls::LC, Cls::LD, DET> sink;
+        std::conditional_t<kWholeQuartet<Cls::LA, Cls::LB, Cls::LC, Cls::LD>,
+                           QuartetSink<RT, Cls::LA, Cls::LB, Cls::LC, Cls::LD, DET, false>,
+                           JKSink<RT, Cls::LA, Cls::LB, Cls::LC, Cls::LD, DET>>
+            sink;
         sink.D = D; sink.J = J; sink.K = K; sink.n = n;
         if constexpr (DET) sink.det_lo = w.det_lo;
         // several molecules: the bra pair's molecule selects the packed blocks and their dimension
@@ -505,6 +654,7 @@ __global__ void __launch_bounds__(THREADS) jk_kernel(JKWorkDev w, PairListDev br
             sink.fd = shell_f0[sd];
             sink.s = (sa == sb ? 0.5 : 1.0) * (sc == sd ? 0.5 : 1.0) * ((w.same_class && i == j) ? 0.5 : 1.0);
             const int oi = bra.ppo[i], ni = bra.npp[i], oj = ket.ppo[j], nj = ket.npp[j];
+            sink.quartet_begin();
             for (int x = 0; x < ni; ++x)
             {
                 const PrimPairData ab = load_pp(P, oi + x);
@@ -561,8 +711,6 @@ __device__ __forceinline__ double half_warp_transpose_sum(double (&v)[P], int la
     return x;
 }
 
-constexpr int pow2_at_least(int v) { return v <= 1 ? 1 : 2 * pow2_at_least((v + 1) / 2); }
-
 template <int LA, int LB, int LC, int LD>
 struct WarpJKSink
 {
@@ -584,6 +732,8 @@ struct WarpJKSink
 #pragma unroll
         for (int k = 0; k < NAB; ++k) jab[k] = 0.0;
     }
+    __device__ __forceinline__ void quartet_begin() {}
+    __device__ __forceinline__ void quartet_end() {}
     __device__ __forceinline__ void ket_begin(int ic, int id)
     {
         const int la = fc + ic, si = fd + id;
@@ -699,7 +849,10 @@ __global__ void __launch_bounds__(THREADS) jk_warp_kernel(JKWorkDev w, PairListD
         const int prefix = real ? (int)(w.offs[i + 1] - w.offs[i]) : 0;
         const int jb = w.kbase ? w.kbase[i] : 0;   // the same within a half: one molecule per set
         const int sa = bra.sa[i], sb = bra.sb[i];
-        WarpJKSink<Cls::LA, Cls::LB, Cls::LC, Cls::LD> sink;
+        std::conditional_t<kWholeQuartet<Cls::LA, Cls::LB, Cls::LC, Cls::LD>,
+                           QuartetSink<double, Cls::LA, Cls::LB, Cls::LC, Cls::LD, false, true>,
+                           WarpJKSink<Cls::LA, Cls::LB, Cls::LC, Cls::LD>>
+            sink;
         sink.D = D;
         sink.J = J;
         sink.K = K;
@@ -733,6 +886,7 @@ __global__ void __launch_bounds__(THREADS) jk_warp_kernel(JKWorkDev w, PairListD
                 (sa == sb ? 0.5 : 1.0) * (sc == sd ? 0.5 : 1.0) * ((w.same_class && i == j) ? 0.5 : 1.0);
             const int oj = ket.ppo[j], nj = ket.npp[j];
             const int njmax = __reduce_max_sync(0xffffffffu, nj);
+            sink.quartet_begin();
             for (int x = 0; x < nimax; ++x)
             {
                 const PrimPairData ab = load_pp(P, oi + (x < ni ? x : ni - 1));
@@ -743,6 +897,7 @@ __global__ void __launch_bounds__(THREADS) jk_warp_kernel(JKWorkDev w, PairListD
                     Cls::template quartet<double>(ab, cd, boys_table, rs, THREADS, sink);
                 }
             }
+            sink.quartet_end();
         }
         sink.flush_bra();
     }

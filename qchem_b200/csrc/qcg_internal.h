@@ -125,9 +125,6 @@ using EriBatch32Launcher = void (*)(const BasisDev&, const int4*, const int*, lo
 extern const EriBatchLauncher kEriBatchLaunchers[kNumQuartetClasses];
 extern const EriBatch32Launcher kEriBatch32Launchers[kNumQuartetClasses];
 
-// counting sort of a quartet batch by contraction pattern -> order (a permutation of 0..nq-1)
-void launch_pattern_sort(const BasisDev& bs, const int4* quartets, long long nq, unsigned char* key, int* hist,
-                         int* cursor, int* order, cudaStream_t st, int nsm);
 extern const JKLauncher kJKLaunchers[kNumQuartetClasses];     // FP64 evaluation
 extern const JKLauncher kJK32Launchers[kNumQuartetClasses];   // FP32 evaluation, FP64 accumulation
 extern const SchwarzLauncher kSchwarzLaunchers[kNumPairClasses];
