@@ -2256,9 +2256,14 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
         }
 }
 
+// Classes from this many quartets on are evaluated in FP64 whatever the FP32 bound: their FP64 launch over every
+// quartet is faster than an FP64 and an FP32 launch that each pass over the list and skip the other's quartets
+// (four waters, 228 functions, bound 1e-7: 5.4 ms in two bands, 3.9 ms in one).
+constexpr long long kFP32BandMaxQuartets = 1LL << 15;
+
 // fp32_below: quartets whose density-weighted bound Q_ab Q_cd max|D| (max over the six D blocks the
-// quartet digests) is below it are evaluated in FP32 (FP64 accumulation); 0 = all FP64, HUGE_VAL = all
-// FP32.  The weighting is what makes FP32 safe: the FP32 error of a quartet's contribution to J and K is
+// quartet digests) is below it may be evaluated in FP32 (FP64 accumulation), and are in the classes below
+// kFP32BandMaxQuartets; 0 = all FP64, HUGE_VAL = all FP32.  The weighting is what makes FP32 safe: the FP32 error of a quartet's contribution to J and K is
 // about 3e-7 of its bound.  dmax (the density maxima of dD) is computed here when the caller has none.
 void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flags, qcg_stats* stats,
                const double* dmax = nullptr, double dthr = 0.0, double fp32_below = 0.0)
@@ -2270,11 +2275,17 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     // density screening and the density-weighted FP32 band index a shell x shell table: single molecule
     require(h->nmol == 1 || (!dmax && (fp32_below <= 0 || fp32_below >= HUGE_VAL)),
             "density-weighted screening and mixed precision need a single-molecule handle");
-    if (fp32_below > 0 && fp32_below < HUGE_VAL && !dmax)
+    // split[k]: class k has an FP64 and an FP32 band
+    bool split[kNumQuartetClasses] = {}, any_split = false;
+    if (fp32_below > 0 && fp32_below < HUGE_VAL)
+        for (int k = 0; k < kNumQuartetClasses; ++k)
+            any_split |= split[k] = h->work[k].total > 0 && h->work[k].total < kFP32BandMaxQuartets;
+    const double* band_dmax = dmax;
+    if (any_split && !dmax)
     {
         if (!h->d_dmaxD) h->d_dmaxD = h->alloc<double>((size_t)h->nshell * h->nshell);
         launch_block_max(dD, h->d_f0, h->bs.L, h->nshell, n, h->d_dmaxD, h->stream, h->nsm);
-        dmax = h->d_dmaxD;
+        band_dmax = h->d_dmaxD;
     }
     if (!h->ev0)
     {
@@ -2326,7 +2337,7 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     for (int k = 0; k < kNumQuartetClasses; ++k)
         if (((warp_mask >> k) & 1u) && !team.on[k] && h->work[k].total > 0 && h->shard_world == 1 &&
             !(flags & QCG_JK_DETERMINISTIC) &&
-            (warp_forced || (dmax == nullptr && dthr <= 0.0 && h->work[k].total >= kJKWarpMinQuartets)))
+            (warp_forced || (dmax == nullptr && dthr <= 0.0 && !split[k] && h->work[k].total >= kJKWarpMinQuartets)))
         {
             warp_items(h, k);
             warp_k[k] = h->nwitems[k] > 0;
@@ -2357,14 +2368,14 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
             // this rank's contiguous slice of the class's quartets (equal shares of its primitive quartets)
             shard_range(h, k, wk.gbeg, wk.gend);
             if (wk.gend <= wk.gbeg) continue;
-            wk.dmax = dmax;
+            wk.dmax = split[k] ? band_dmax : dmax;
             wk.nshell = h->nshell;
             wk.dthr = dthr;
             wk.pmask = h->d_pmask;
             wk.det_lo = det ? (long long)nn : 0;
             if (fp32_below < HUGE_VAL)
             {
-                wk.lo = fp32_below;
+                wk.lo = split[k] ? fp32_below : 0.0;
                 wk.hi = HUGE_VAL;
                 if (team.on[k])
                 {
@@ -2386,7 +2397,7 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
                     slot = (slot + 1) % qcg_handle::kSide;
                 }
             }
-            if (fp32_below > 0)
+            if (split[k] || fp32_below >= HUGE_VAL)
             {
                 wk.lo = 0.0;
                 wk.hi = fp32_below;
