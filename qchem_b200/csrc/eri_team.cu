@@ -243,7 +243,7 @@ void QCG_CAT(launch_jk_team_, QCG_CLASS)(const JKWorkDev& w, const PairListDev& 
                                          double* K, int n, const double* boys, const TeamScratchDev& scr,
                                          const TeamShape& sh, cudaStream_t st)
 {
-    const long long span = w.gend - w.gbeg;
+    const long long span = scr.list.n ? scr.list.total : w.gend - w.gbeg;
     if (span <= 0) return;
     const long long ngroups = (span + 31) / 32;
     if (scr.kmax == 1)

@@ -317,9 +317,10 @@ namespace qcg {
 
 // ------------------------------------------------------------------------------------------------
 // The team form of the direct J/K build (contracted classes; uncontracted ones: jk_group.cuh).  The same stages
-// and contraction on 32 quartets of a class's screened work list at a time (lane l: quartet gbeg + 32 g + l, its
-// bra pair found by binary search, its kets from the Q-sorted list), the stages built from the primitive-pair
-// table; then the digestion of [e0|f0] into J' and K' (team_digest), the (c d) columns split over the warps.
+// and contraction on 32 quartets at a time, in the class's own order for this form (JKTeamListDev: quartets of equal
+// primitive-loop length together, longest first, in a small build cut into runs of bra primitive pairs, each
+// digested by itself, which the linearity of J and K allows) or in that of its screened work list; lane l takes
+// item gbeg + 32 g + l, its entry found by binary search.  The stages are built from the primitive-pair table; then the digestion of [e0|f0] into J' and K' (team_digest), the (c d) columns split over the warps.
 // This replaces qchem's MakeDirect/MakeExchange + ERI4::MatMul (Molecule/IrrepBasisSet.C:138-183,
 // Internal/Imp/ERI4.C:10-17) without storing the integrals.
 // ------------------------------------------------------------------------------------------------
@@ -346,31 +347,48 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     double* const rc = scr.rcache + (long long)blockIdx.x * scr.kmax * STAGE;
     double* const hA = scr.hrr + (long long)blockIdx.x * NE * NF * 32;
     unsigned long long G = 0;
-    const long long ngroups = (w.gend - w.gbeg + 31) >> 5;
+    const JKTeamListDev& list = scr.list;
+    const long long* const offs = list.n ? list.offs : w.offs;
+    const long long gend = list.n ? list.total : w.gend, gbeg = list.n ? 0 : w.gbeg;
+    const long long ngroups = (gend - gbeg + 31) >> 5;
     for (long long g = blockIdx.x; g < ngroups; g += gridDim.x)
     {
-        const long long gq = w.gbeg + g * 32 + lane;
-        bool valid = gq < w.gend;
-        int i = 0, j = 0, sa = 0, sb = 0, sc = 0, sd = 0;
+        const long long gq = gbeg + g * 32 + lane;
+        bool valid = gq < gend;
+        int i = 0, j = 0, p0 = 0, Kab = 0, Kcd = 0;
         if (valid)
         {
-            int lo = 0, hi = bra.n;   // bra pair i: offs[i] <= gq < offs[i+1]
+            int lo = 0, hi = list.n ? list.n : bra.n;   // entry or bra pair: offs[lo] <= gq < offs[lo + 1]
             while (hi - lo > 1)
             {
                 const int mid = (lo + hi) >> 1;
-                if (w.offs[mid] <= gq) lo = mid;
+                if (offs[mid] <= gq) lo = mid;
                 else hi = mid;
             }
-            i = lo;
-            j = (w.kbase ? w.kbase[i] : 0) + (int)(gq - w.offs[i]);
-            sa = bra.sa[i];
-            sb = bra.sb[i];
-            sc = ket.sa[j];
-            sd = ket.sb[j];
-            if (w.mol_active && bra.mol && !w.mol_active[bra.mol[i]]) valid = false;
-            else if (jk_skip(w, bra, ket, i, j, sa, sb, sc, sd)) valid = false;
+            const int pos = (int)(gq - offs[lo]);
+            if (list.n)
+            {
+                const int4 e = list.entry[lo];
+                i = e.x;
+                p0 = e.y;
+                Kab = e.z;
+                j = list.kets[e.w + pos];
+            }
+            else
+            {
+                i = lo;
+                Kab = bra.npp[i];
+                j = (w.kbase ? w.kbase[i] : 0) + pos;
+            }
+            Kcd = ket.npp[j];
+            if ((w.mol_active && bra.mol && !w.mol_active[bra.mol[i]]) ||
+                jk_skip(w, bra, ket, i, j, bra.sa[i], bra.sb[i], ket.sa[j], ket.sb[j]))
+            {
+                valid = false;
+                Kab = Kcd = 0;
+            }
         }
-        const int Kab = valid ? bra.npp[i] : 0, Kcd = valid ? ket.npp[j] : 0, Kq = Kab * Kcd;
+        const int Kq = Kab * Kcd;
         const int Kg = __reduce_max_sync(0xffffffffu, Kq);   // CTA-uniform: every warp sees the same lanes
         if (Kg == 0) continue;                               // every quartet of the group skipped
         if (Kg > scr.kmax)
@@ -380,7 +398,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         }
         // 1. stage tables, from the primitive-pair table
         team_stages<Cls>(
-            rc, Kab, Kcd, Kg, bt, [&](int ij) { return load_pp(P, bra.ppo[i] + ij); },
+            rc, Kab, Kcd, Kg, bt, [&](int ij) { return load_pp(P, bra.ppo[i] + p0 + ij); },
             [&](int kl) { return load_pp(P, ket.ppo[j] + kl); });
         // 2. contraction (as in eri_batch_team_kernel)
         if (!team_contract<Cls>(rc, hA, Kq, Kcd, Kg, G, full, scr.err)) return;

@@ -7,6 +7,18 @@
 
 namespace qcg {
 
+// The contracted J/K build's own order of a class's screened quartets (jk_team_list, runtime.cu): entry e is a run of
+// bra primitive pairs [y, y + z) of bra pair x against the kets kets[w ..] of one primitive-pair count, items
+// offs[e] .. offs[e + 1); n = 0: the class's work list as it is.
+struct JKTeamListDev
+{
+    int n;
+    const long long* offs;
+    const int4* entry;
+    const int* kets;
+    long long total;
+};
+
 // Device memory a team launch works in, beside its inputs and outputs (the handle owns it):
 //   rcache -- per CTA, kmax stage slots: the primitive quartets' R tables and Hermite tables, written once
 //             per group of quartets and streamed back into shared memory once per pass;
@@ -20,6 +32,7 @@ struct TeamScratchDev
     double* hrr;
     int* err;
     const BatchPlanDev* plan;   // ERI batches: the groups
+    JKTeamListDev list;         // contracted J/K builds: the order of the quartets
 };
 
 // The launch shape of class k on nsm SMs and the scratch it needs per CTA, in doubles.

@@ -404,6 +404,8 @@ struct qcg_handle
     int4* d_witems[kNumQuartetClasses] = {};
     long long nwitems[kNumQuartetClasses] = {};
     bool witems_ready[kNumQuartetClasses] = {};
+    JKTeamListDev team_list[kNumQuartetClasses] = {};
+    bool team_list_ready[kNumQuartetClasses] = {};
     long long jk_warp_mask = -1;   // qcg_set_jk_warp_classes; -1: the process default
     double fp32_below = 0;   // qcg_set_fp32_bound: quartets with a smaller bound are evaluated in FP32
     int shard_rank = 0, shard_world = 1;   // qcg_set_shard: this handle's slice of every J/K build
@@ -2206,6 +2208,88 @@ struct JKTeamPlan
     bool side = false;
 };
 
+// The order in which the contracted team form takes class k's quartets (JKTeamListDev).  In the work list a bra pair's
+// kets come by their bounds, contraction lengths mixed, and a group of 32 runs its longest primitive loop for all
+// lanes.  Here the kets of a pair class are also listed by primitive-pair count (bounds descending within one), so
+// that a bra pair's screened kets are a run of each count's list; the runs are taken longest loop first.  A loop
+// longer than a CTA's average share of all loops (at least kTeamChain) is cut into runs of bra primitive pairs.
+// Built once per screening, before any capture.
+constexpr int kTeamChain = 9;
+const JKTeamListDev& jk_team_list(qcg_handle* h, int k, int ctas)
+{
+    JKTeamListDev& list = h->team_list[k];
+    if (h->team_list_ready[k]) return list;
+    h->team_list_ready[k] = true;
+    int X = 0;
+    while ((X + 1) * (X + 2) / 2 <= k) ++X;
+    const int Y = k - X * (X + 1) / 2;
+    const std::vector<int>&nx = h->pl_npp[X], &ny = h->pl_npp[Y], &mol = h->pl_mol[Y];
+    const std::vector<long long>& offs = h->wh_offs[k];
+    std::vector<int> counts(ny);
+    std::sort(counts.begin(), counts.end(), std::greater<int>());
+    counts.erase(std::unique(counts.begin(), counts.end()), counts.end());
+    const int nv = (int)counts.size(), n = (int)ny.size();
+    // kets by molecule, then count; before[v][j]: kets of count v among the first j; start[m][v]
+    std::vector<int> kets;
+    kets.reserve(n);
+    std::vector<std::vector<int>> before(nv, std::vector<int>(n + 1, 0));
+    std::vector<std::vector<int>> start(h->nmol, std::vector<int>(nv, 0));
+    for (int v = 0; v < nv; ++v)
+        for (int j = 0; j < n; ++j) before[v][j + 1] = before[v][j] + (ny[j] == counts[v]);
+    for (int j0 = 0; j0 < n;)
+    {
+        int j1 = j0;
+        while (j1 < n && mol[j1] == mol[j0]) ++j1;
+        for (int v = 0; v < nv; ++v)
+        {
+            start[mol[j0]][v] = (int)kets.size();
+            for (int j = j0; j < j1; ++j)
+                if (ny[j] == counts[v]) kets.push_back(j);
+        }
+        j0 = j1;
+    }
+    const long long share = h->wh_cum[k].empty() ? 0 : h->wh_cum[k].back() / (32LL * ctas);
+    const long long most = std::max<long long>(share, kTeamChain);
+    struct Run
+    {
+        long long loop, cnt;
+        int4 e;
+    };
+    std::vector<Run> runs;
+    for (size_t i = 0; i + 1 < offs.size(); ++i)
+    {
+        const long long cnt = offs[i + 1] - offs[i];
+        if (cnt <= 0) continue;
+        const int jb = h->wh_kbase[k][i], m = mol[jb];
+        for (int v = 0; v < nv; ++v)
+        {
+            const int c = before[v][jb + cnt] - before[v][jb];
+            if (!c) continue;
+            const int piece = (long long)nx[i] * counts[v] <= most ? nx[i] : std::max(1, (int)(most / counts[v]));
+            for (int p = 0; p < nx[i]; p += piece)
+            {
+                const int np = std::min(piece, nx[i] - p);
+                runs.push_back({(long long)np * counts[v], c, make_int4((int)i, p, np, start[m][v])});
+            }
+        }
+    }
+    std::stable_sort(runs.begin(), runs.end(), [](const Run& a, const Run& b) { return a.loop > b.loop; });
+    std::vector<long long> at(runs.size() + 1, 0);
+    std::vector<int4> entry(runs.size());
+    for (size_t r = 0; r < runs.size(); ++r)
+    {
+        entry[r] = runs[r].e;
+        at[r + 1] = at[r] + runs[r].cnt;
+    }
+    if (runs.empty()) return list;
+    list.offs = h->upload(at);
+    list.entry = h->upload(entry);
+    list.kets = h->upload(kets);
+    list.total = at.back();
+    list.n = (int)runs.size();
+    return list;
+}
+
 // want[k]: class k in the team form if its scratch can be had; required: the caller named the classes, so that a
 // failed allocation is an error rather than a reason for another form.
 void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool required, JKTeamPlan& plan)
@@ -2216,10 +2300,11 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
         if (!want[k]) continue;
         long long gb = 0, ge = 0;
         shard_range(h, k, gb, ge);
-        const long long ngroups = (ge - gb + 31) / 32;
         const int kmax = team_kmax(h, k);
         TeamShape& sh = plan.sh[k];
         sh = team_shape(h, k);
+        if (kmax > 1 && h->shard_world == 1) plan.scr[k].list = jk_team_list(h, k, sh.grid);
+        const long long ngroups = ((plan.scr[k].list.n ? plan.scr[k].list.total : ge - gb) + 31) / 32;
         sh.grid = (int)std::min<long long>(sh.grid, ngroups);
         sh.group_grid = (int)std::min<long long>(sh.group_grid, ngroups);
         need[k] = kmax == 1 ? std::min<long long>(ngroups, sh.group_grid * (sh.group_doubles / sh.jk_doubles)) * sh.jk_doubles
@@ -2373,6 +2458,13 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
             wk.dthr = dthr;
             wk.pmask = h->d_pmask;
             wk.det_lo = det ? (long long)nn : 0;
+            const bool alone = false;
+            auto stream = [&]() {
+                if (alone) return h->side[0];
+                const cudaStream_t st = h->side[slot];
+                slot = (slot + 1) % qcg_handle::kSide;
+                return st;
+            };
             if (fp32_below < HUGE_VAL)
             {
                 wk.lo = split[k] ? fp32_below : 0.0;
@@ -2380,21 +2472,17 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
                 if (team.on[k])
                 {
                     kJKTeamLaunchers[k](wk, h->pl_dev[X], h->pl_dev[Y], h->pp_dev, h->d_f0, dD, h->d_Jp, h->d_Kp, n,
-                                        h->d_boys, team.scr[k], team.sh[k], h->side[team.side ? slot : 0]);
-                    if (team.side) slot = (slot + 1) % qcg_handle::kSide;
+                                        h->d_boys, team.scr[k], team.sh[k], team.side ? stream() : h->side[0]);
                 }
                 else if (warp_k[k])
                 {
                     kJKWarpLaunchers[k](wk, h->pl_dev[X], h->pl_dev[Y], h->pp_dev, h->d_f0, dD, h->d_Jp, h->d_Kp, n,
-                                        h->d_boys, h->d_wgbra[k], h->d_witems[k], h->nwitems[k], h->side[slot],
-                                        h->nsm);
-                    slot = (slot + 1) % qcg_handle::kSide;
+                                        h->d_boys, h->d_wgbra[k], h->d_witems[k], h->nwitems[k], stream(), h->nsm);
                 }
                 else
                 {
                     kJKLaunchers[k](wk, h->pl_dev[X], h->pl_dev[Y], h->pp_dev, h->d_f0, dD, h->d_Jp, h->d_Kp, n,
-                                    h->d_boys, h->side[slot], h->nsm);
-                    slot = (slot + 1) % qcg_handle::kSide;
+                                    h->d_boys, stream(), h->nsm);
                 }
             }
             if (split[k] || fp32_below >= HUGE_VAL)
@@ -2402,8 +2490,7 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
                 wk.lo = 0.0;
                 wk.hi = fp32_below;
                 kJK32Launchers[k](wk, h->pl_dev[X], h->pl_dev[Y], h->pp_dev, h->d_f0, dD, h->d_Jp, h->d_Kp, n,
-                                  h->d_boys, h->side[slot], h->nsm);
-                slot = (slot + 1) % qcg_handle::kSide;
+                                  h->d_boys, stream(), h->nsm);
             }
         }
         CK(cudaGetLastError());
@@ -3084,6 +3171,11 @@ int qcg_schwarz(qcg_handle* h, double thresh, double* Q)
                     h->d_witems[k] = nullptr;
                     h->nwitems[k] = 0;
                     h->witems_ready[k] = false;
+                    for (const void* p : {(const void*)h->team_list[k].offs, (const void*)h->team_list[k].entry,
+                                          (const void*)h->team_list[k].kets})
+                        if (p) h->release((void*)p);
+                    h->team_list[k] = JKTeamListDev{};
+                    h->team_list_ready[k] = false;
                 }
                 h->screened = false;
             }
