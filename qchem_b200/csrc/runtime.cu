@@ -2195,6 +2195,11 @@ int* team_error_word(qcg_handle* h);
 constexpr long long kTeamScratchMax = 4LL << 30;
 // smallest quartet count of a class for the warp-shared form by default
 constexpr long long kJKWarpMinQuartets = 1LL << 20;
+// Classes from this many quartets on take the first side stream, one after another: each fills the GPU for
+// milliseconds, and side by side their CTAs take each other's registers and shared memory (912 functions: 474 ms
+// spread over the streams, 396 ms so; 456 functions: 40.5, 37.7).  Smaller ones fill each other's gaps (228
+// functions: 4.1 ms spread, 6.0 with the classes of 2^20 quartets alone).
+constexpr long long kJKAloneQuartets = 1LL << 24;
 // most scratch that lets the team classes of one build run side by side (they share one class's worth beyond it)
 constexpr long long kJKTeamSideMax = 2LL << 30;
 
@@ -2458,7 +2463,7 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
             wk.dthr = dthr;
             wk.pmask = h->d_pmask;
             wk.det_lo = det ? (long long)nn : 0;
-            const bool alone = false;
+            const bool alone = wk.gend - wk.gbeg >= kJKAloneQuartets;
             auto stream = [&]() {
                 if (alone) return h->side[0];
                 const cudaStream_t st = h->side[slot];
