@@ -55,26 +55,35 @@ constexpr int team_pieces(int ncode, int nh, int ne)
     const int npass = (ncode + g - 1) / g;
     return (ncode + npass - 1) / npass;
 }
-// Doubles of the stage space: three stages, and at least 18 primitive pairs (contractions of three) and the columns
+// CTAs per SM to compile for: about twelve warps, as far as three stages each fit the shared memory, of which a
+// CTA may then use kSmemPerSM / m bytes less what it holds beside the stages
+constexpr int kSmemPerSM = 227 * 1024;
+constexpr int kSmemBeside = 2048 + (int)sizeof(BatchPlanDev) + (int)(kBoysRows * kBoysColumns * sizeof(double));
+constexpr int team_min_blocks(int ng, int stage)
+{
+    const int fit = kSmemPerSM / (3 * stage * 32 * 8 + kSmemBeside), want = 12 / (3 * ng);
+    const int m = fit < want ? fit : want;
+    return m < 1 ? 1 : m;
+}
+// stages per slot of the ring (team_contract): what three slots leave room for, eight at most
+constexpr int team_unroll(int ng, int stage)
+{
+    const int u = (kSmemPerSM / team_min_blocks(ng, stage) - kSmemBeside) / (3 * stage * 32 * 8);
+    return u < 1 ? 1 : (u > 8 ? 8 : u);
+}
+// Doubles of the stage space: three slots, and at least 18 primitive pairs (contractions of three) and the columns
 // of the bra recurrence that go out together.
 constexpr int team_stage_space(int ng, int stage)
 {
     const int ncd = ncart(kPairLA[kY]) * ncart(kPairLB[kY]), nab = ncart(kPairLA[kX]) * ncart(kPairLB[kX]);
-    const int columns = nab * (ncd < 3 * ng ? ncd : 3 * ng) * 33;
+    const int columns = nab * (ncd < 3 * ng ? ncd : 3 * ng) * 33, slots = 3 * team_unroll(ng, stage) * stage * 32;
     int n = 18 * kTeamPairDoubles * 32;
-    if (n < 3 * stage * 32) n = 3 * stage * 32;
+    if (n < slots) n = slots;
     return n < columns ? columns : n;
 }
 constexpr size_t team_smem(int ng, int stage)
 {
     return (size_t)(team_stage_space(ng, stage) + kBoysRows * kBoysColumns) * sizeof(double);
-}
-// CTAs per SM to compile for: about twelve warps, as far as their shared memory fits
-constexpr int team_min_blocks(int ng, int stage)
-{
-    const int fit = (int)((227 * 1024) / (team_smem(ng, stage) + sizeof(BatchPlanDev) + 2048)), want = 12 / (3 * ng);
-    const int m = fit < want ? fit : want;
-    return m < 1 ? 1 : m;
 }
 
 struct Cls
@@ -85,7 +94,7 @@ struct Cls
     static constexpr int kNCode = gen::QCG_CAT(kTeamNCode, QCG_CLASS);
     static constexpr int kKetStage = gen::QCG_CAT(kTeamKetStage, QCG_CLASS);
     static constexpr int kNG = team_pieces(kNCode, kNH, kNE), kNW = 3 * kNG;
-    static constexpr int kMinBlocks = team_min_blocks(kNG, kStage);
+    static constexpr int kMinBlocks = team_min_blocks(kNG, kStage), kUnroll = team_unroll(kNG, kStage);
     // jk_group_kernel: groups of 32 quartets per round (two sets of stages within the shared memory), its warps --
     // eight where Y_f, acc_f or the digestion of a (dd| bra need more registers than twelve leave -- and CTAs per SM
     static constexpr int kGroups = [] {

@@ -20,8 +20,8 @@
 //     registers Y_f -- the ket step summed over the ket primitives of the current bra primitive pair -- and
 //     acc_f = [e0|f] for every e, adding the bra step of Y_f to acc_f after the bra pair's last ket primitive
 //     (team_ket_piece_<k>, team_bra_view_<k>).  The stages stream from the R cache into shared memory, three
-//     deep, by bulk copies (cp.async.bulk, the Tensor Memory Accelerator's untiled form) that one warp issues
-//     on an mbarrier, without a gap between passes; one barrier per primitive quartet.  With more pieces than
+//     deep, by bulk copies (cp.async.bulk, the Tensor Memory Accelerator's untiled form) on mbarriers, without a
+//     gap between passes.  With more pieces than
 //     a pass holds, each pass reads the stages again (from L2 or HBM) instead of recomputing them.
 //  3. Recurrences.  acc_f goes to the CTA's scratch as [e0|f0] (lane-minor, so every access of a warp is
 //     one coalesced line); the ket recurrence per e row gives [e0|cd] there, and the bra recurrence per
@@ -101,38 +101,49 @@ __device__ __forceinline__ void team_stages(double* __restrict__ rc, const int K
     __syncthreads();
 }
 
+// The ring of three slots in shared memory that the stages pass through, kUnroll stages to a slot: full[s] completes
+// when slot s holds its stages, done[s] counts the warps that have finished with them.  slot, phase: the next step's
+// slot and the parity its full[] completes with.
+struct TeamRing
+{
+    uint64_t* full;
+    int* done;
+    int slot = 0;
+    uint32_t phase = 0;
+};
+
 // Phase 2 of both kernels: [e0|f0] of the group (lane-minor, rows and columns in slot order) from the Kg stages
-// in rc; K and Kcd are this lane's primitive-quartet and ket-pair counts (0 for an absent quartet), G the
-// number of steps streamed so far.  False, CTA-uniform, when a bulk copy did not arrive.
+// in rc; K and Kcd are this lane's primitive-quartet and ket-pair counts (0 for an absent quartet).  Warps are not
+// held together: each waits for a step's stages by itself, and the warp that leaves a slot last starts the copy of
+// the step three later into it (a fixed warp that refilled slots as it came to them took 3.0 ms where this takes 2.6
+// on (dd|pp)).  A step costs some hundred cycles of waits and barrier traffic beside its arithmetic (480 cycles
+// for a (pp|pp) stage), so it takes as many stages as the shared memory gives three slots for.
+// False, in every warp that sees it, when a bulk copy did not arrive.
 template <class Cls>
 __device__ __forceinline__ bool team_contract(const double* __restrict__ rc, double* __restrict__ hA, const int K,
-                                              const int Kcd, const int Kg, unsigned long long& G, uint64_t* full,
-                                              int* err)
+                                              const int Kcd, const int Kg, TeamRing& ring, int* err)
 {
-    constexpr int NG = Cls::kNG, NF = Cls::kNF, NE = Cls::kNE, NH = Cls::kNH, NC = Cls::kNCode;
+    constexpr int NG = Cls::kNG, NE = Cls::kNE, NH = Cls::kNH, NC = Cls::kNCode, NW = Cls::kNW, U = Cls::kUnroll;
     constexpr int NPASS = (NC + NG - 1) / NG;
     constexpr int STAGE = Cls::kStage * 32;        // doubles per stage (entry-major, lane-minor)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int piece = warp / 3, rot = warp - 3 * piece;
-    const bool leader = threadIdx.x == 0;
-    const int nsteps = NPASS * Kg;
-    // step t = pass * Kg + x reads stage x; warp 0 issues its copy, without the bra tables when no lane needs them
-    int ix = 0, ikl = 0;   // the next issued step's stage and its ket primitive in this lane
-    auto issue = [&](int t) {
-        const bool bra = __any_sync(0xffffffffu, ix < K && ikl == Kcd - 1);
-        if (leader)
-        {
-            const unsigned long long gs = G + t;
-            team::bulk_load(qcg_team_smem + (gs % 3) * STAGE, rc + (long long)ix * STAGE,
-                            (bra ? Cls::kStage : Cls::kKetStage) * 32 * (uint32_t)sizeof(double), &full[gs % 3]);
-        }
-        ikl = ikl == Kcd - 1 ? 0 : ikl + 1;
-        if (++ix == Kg) ix = ikl = 0;
+    const int per = (Kg + U - 1) / U, nsteps = NPASS * per;   // steps of a pass, and in all
+    // the copy of a pass's step c into slot, by one warp; a single stage goes without the bra tables where no lane's
+    // bra step needs them
+    auto issue = [&](int c, int slot) {
+        const int x0 = c * U, n = Kg - x0 < U ? Kg - x0 : U;
+        uint32_t bytes = (uint32_t)n * STAGE * sizeof(double);
+        if (U == 1 && !__any_sync(0xffffffffu, x0 < K && (x0 + 1) % Kcd == 0))
+            bytes = Cls::kKetStage * 32 * (uint32_t)sizeof(double);
+        if (lane == 0)
+            team::bulk_load(qcg_team_smem + slot * U * STAGE, rc + (long long)x0 * STAGE, bytes, &ring.full[slot]);
     };
-    if (warp == 0)
+    int ahead = 0;   // the step three later, within its pass
+    for (int t = 0, slot = ring.slot; t < 3; ++t, slot = slot == 2 ? 0 : slot + 1)
     {
-        issue(0);
-        if (nsteps > 1) issue(1);
+        if (warp == 0 && t < nsteps) issue(ahead, slot);
+        if (++ahead == per) ahead = 0;
     }
     int t = 0;
     for (int pass = 0; pass < NPASS; ++pass)
@@ -145,41 +156,50 @@ __device__ __forceinline__ bool team_contract(const double* __restrict__ rc, dou
 #pragma unroll
         for (int e = 0; e < NE; ++e) acc[e] = 0.0;
         int kl = 0;
-        for (int x = 0; x < Kg; ++x, ++t)
+        for (int c = 0; c < per; ++c, ++t)
         {
-            const unsigned long long gs = G + t;
-            bool late = false;
-            if (leader) late = !team::mbar_wait(&full[gs % 3], (uint32_t)((gs / 3) & 1));
-            // stage x is in shared memory; every warp has left the step before
-            if (__syncthreads_or(late))
+            const int slot = ring.slot;
+            if (!team::mbar_wait(&ring.full[slot], ring.phase))
             {
-                // a copy did not arrive: let the ones in flight land and record it
-                if (leader)
+                // a copy did not arrive: record it, let the ones in flight land and leave
+                if (lane == 0)
                 {
-                    team::drain(full, G, t, nsteps);
                     atomicOr(err, 1);
+                    team::drain(ring.full, slot, ring.phase, nsteps - t < 3 ? nsteps - t : 3);
                 }
+                __syncwarp();
                 return false;
             }
-            if (warp == 0 && t + 2 < nsteps) issue(t + 2);   // into the stage the step before used
-            if (on && x < K)
-            {
-                const typename Cls::View v(qcg_team_smem + (gs % 3) * STAGE + lane, rot);
-                Cls::ket(jc, v, Y);
-                if (kl == Kcd - 1)
+            const int n = Kg - c * U < U ? Kg - c * U : U;
+            for (int u = 0; u < n; ++u)
+                if (on && c * U + u < K)
                 {
-                    Cls::bra(v, Y, acc);
+                    const typename Cls::View v(qcg_team_smem + (slot * U + u) * STAGE + lane, rot);
+                    Cls::ket(jc, v, Y);
+                    if (kl == Kcd - 1)
+                    {
+                        Cls::bra(v, Y, acc);
 #pragma unroll
-                    for (int h = 0; h < NH; ++h) Y[h] = 0.0;
-                    kl = 0;
+                        for (int h = 0; h < NH; ++h) Y[h] = 0.0;
+                        kl = 0;
+                    }
+                    else
+                        ++kl;
                 }
-                else
-                    ++kl;
+            __syncwarp();
+            int last = 0;
+            if (lane == 0) last = team::count_done(&ring.done[slot]) == NW - 1;
+            if (__shfl_sync(0xffffffffu, last, 0))
+            {
+                if (lane == 0) ring.done[slot] = 0;
+                if (t + 3 < nsteps) issue(ahead, slot);
             }
+            if (++ahead == per) ahead = 0;
+            ring.slot = slot == 2 ? 0 : slot + 1;
+            if (slot == 2) ring.phase ^= 1;
         }
         if (on) Cls::store(acc, hA + (Cls::fslot(jc) + rot) * 32 + lane, rot);
     }
-    G += nsteps;
     __syncthreads();   // the stages are no longer read; [e0|f0] is written
     return true;
 }
@@ -197,11 +217,16 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     constexpr long long BLK = (long long)ncart(Cls::LA) * ncart(Cls::LB) * NCD;
     static_assert(NE <= ncart(Cls::LA) * ncart(Cls::LB) && NF <= NCD, "[e0|f0] fits the output block");
     __shared__ uint64_t full[3];
+    __shared__ int done[3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool leader = threadIdx.x == 0;
     if (leader)
     {
-        for (int s = 0; s < 3; ++s) team::mbar_init(&full[s]);
+        for (int s = 0; s < 3; ++s)
+        {
+            team::mbar_init(&full[s]);
+            done[s] = 0;
+        }
         team::mbar_init_fence();
     }
     const BoysColumns bt = team_boys<Cls>(qcg_team_smem + Cls::kStageSpace, boys_table);
@@ -209,7 +234,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     double* const rc = scr.rcache + (long long)blockIdx.x * scr.kmax * STAGE;   // this CTA's stage slots
     double* const hA = scr.hrr + (long long)blockIdx.x * (NE * NF + NE * NCD) * 32;
     double* const hB = hA + NE * NF * 32;
-    unsigned long long G = 0;   // steps streamed so far: step G uses stage G % 3, phase (G / 3) & 1
+    TeamRing ring{full, done};
     __shared__ BatchPlanDev plan;
     __shared__ int lane_q[32];   // each lane's quartet, for the phases after the contraction; -1: none
     for (int k = threadIdx.x; k < (int)(sizeof(BatchPlanDev) / sizeof(int)); k += blockDim.x)
@@ -253,7 +278,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
             },
             [&](int kl) { return shell_prim_pair(bs, s.z, kl / nl, s.w, kl % nl); });
         // 2. contraction, the stages streamed back through shared memory three deep
-        if (!team_contract<Cls>(rc, hA, K, Kcd, Kg, G, full, scr.err)) return;
+        if (!team_contract<Cls>(rc, hA, K, Kcd, Kg, ring, scr.err)) return;
         // the lanes that share a quartet add their [e0|f0]
         if (const int share = plan.lanes[b]; share > 0)
         {
@@ -335,18 +360,23 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     constexpr int STAGE = Cls::kStage * 32;
     constexpr int NCD = ncart(Cls::LC) * ncart(Cls::LD);
     __shared__ uint64_t full[3];
+    __shared__ int done[3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool leader = threadIdx.x == 0;
     if (leader)
     {
-        for (int s = 0; s < 3; ++s) team::mbar_init(&full[s]);
+        for (int s = 0; s < 3; ++s)
+        {
+            team::mbar_init(&full[s]);
+            done[s] = 0;
+        }
         team::mbar_init_fence();
     }
     const BoysColumns bt = team_boys<Cls>(qcg_team_smem + Cls::kStageSpace, boys_table);
     __syncthreads();
     double* const rc = scr.rcache + (long long)blockIdx.x * scr.kmax * STAGE;
     double* const hA = scr.hrr + (long long)blockIdx.x * NE * NF * 32;
-    unsigned long long G = 0;
+    TeamRing ring{full, done};
     const JKTeamListDev& list = scr.list;
     const long long* const offs = list.n ? list.offs : w.offs;
     const long long gend = list.n ? list.total : w.gend, gbeg = list.n ? 0 : w.gbeg;
@@ -401,7 +431,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
             rc, Kab, Kcd, Kg, bt, [&](int ij) { return load_pp(P, bra.ppo[i] + p0 + ij); },
             [&](int kl) { return load_pp(P, ket.ppo[j] + kl); });
         // 2. contraction (as in eri_batch_team_kernel)
-        if (!team_contract<Cls>(rc, hA, Kq, Kcd, Kg, G, full, scr.err)) return;
+        if (!team_contract<Cls>(rc, hA, Kq, Kcd, Kg, ring, scr.err)) return;
         // 3. recurrences and digestion, the (c d) columns in runs of neighbours over the warps
         constexpr int PER = (NCD + NW - 1) / NW;
         const int cd0 = warp * PER, cd1 = cd0 + PER < NCD ? cd0 + PER : NCD;

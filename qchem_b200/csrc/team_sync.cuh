@@ -56,16 +56,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
     return false;
 }
 
-// After the wait for step `step` of a stream of `nsteps` stages (stage of step x: base + x, three deep, the
-// copy of step x issued while step x - 2 is consumed) gave up: wait, bounded, for the copies still in
-// flight -- steps `step` and `step` + 1 -- so that none lands in this CTA's shared memory after it exited.
-__device__ __forceinline__ void drain(uint64_t* full, unsigned long long base, int step, int nsteps)
+// After the wait for slot `slot` of the ring of three gave up: wait, bounded, for the copies still in flight -- that
+// slot's and the ones after it, n in all -- so that none lands in this CTA's shared memory after it exited.
+__device__ __forceinline__ void drain(uint64_t* full, int slot, uint32_t phase, int n)
 {
-    for (int x = step; x < nsteps && x <= step + 1; ++x)
+    for (int x = 0; x < n; ++x)
     {
-        const unsigned long long gs = base + x;
-        mbar_wait(&full[gs % 3], (uint32_t)((gs / 3) & 1));
+        mbar_wait(&full[slot], phase);
+        if (++slot == 3)
+        {
+            slot = 0;
+            phase ^= 1;
+        }
     }
+}
+
+// one more warp is done with a slot (its reads come before, the slot's next copy after); the count before
+__device__ __forceinline__ int count_done(int* done)
+{
+    int old;
+    asm volatile("atom.acq_rel.cta.shared::cta.add.s32 %0, [%1], 1;" : "=r"(old) : "r"(smem_addr(done)) : "memory");
+    return old;
 }
 
 // the barrier's memory may be reused for other data afterwards
