@@ -210,16 +210,17 @@ void launch_ss_split(const BasisDev& bs, const int4* q, const int* order, long l
     const long long blocks = std::min<long long>((nq + per - 1) / per, (long long)nsm * per_sm);
     k<<<(unsigned)blocks, kSSThreads, smem, st>>>(bs, q, order, nq, out, boys);
 }
-// Lanes per quartet: one where one lane per quartet gives every SM a few warps, else as many of the up to nine
-// bra primitive pairs as lanes are free (a quartet of 81 primitive quartets is a serial chain of 81 otherwise).
+// Lanes per quartet: one where one lane per quartet keeps every SM's sixteen warps busy, else as many of the up to nine
+// bra primitive pairs as there are lanes (a quartet of 81 primitive quartets is a serial chain of 81 otherwise).
 template <class OT>
 void launch_ss(const BasisDev& bs, const int4* q, const int* order, long long nq, OT* out, const double* boys,
                int nsm, cudaStream_t st)
 {
     if (nq <= 0) return;
-    const long long lanes = (long long)nsm * 4 * 32;
+    const long long lanes = (long long)nsm * 16 * 32;
     if (nq * 8 <= lanes) launch_ss_split<OT, 8>(bs, q, order, nq, out, boys, nsm, st);
-    else if (nq * 2 <= lanes) launch_ss_split<OT, 4>(bs, q, order, nq, out, boys, nsm, st);
+    else if (nq * 3 <= lanes) launch_ss_split<OT, 4>(bs, q, order, nq, out, boys, nsm, st);
+    else if (nq <= lanes) launch_ss_split<OT, 2>(bs, q, order, nq, out, boys, nsm, st);
     else launch_ss_split<OT, 1>(bs, q, order, nq, out, boys, nsm, st);
 }
 #endif
