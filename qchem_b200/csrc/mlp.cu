@@ -55,6 +55,7 @@ constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A
 // two stages need 64 KB; the allocation is 96 KB so that every address a descriptor of these tiles can
 // form, read either way round (LBO and SBO), stays inside it
 constexpr size_t SMEM = 96 * 1024;
+static_assert(SMEM >= (size_t)BM * (BN + 1) * sizeof(float), "the epilogue's tile fits");
 // instruction descriptor: FP32 accumulator (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), both
 // K-major (bits 15, 16 = 0), N >> 3 at bit 17, M >> 4 at bit 24
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
@@ -102,32 +103,63 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16])
 // Rows [r0, r0 + R) x k [k0, k0 + BK) of an operand whose element (r, k) is X[r*ld + k] (KMAJ) or
 // X[k*ld + r], zero outside [0, nrows) x [0, K), rounded to BF16 into the canonical layout at dst: the
 // 16-byte chunk (r, c) (k = 8c..8c+7) at byte c*R*16 + r*16.  Consecutive threads take consecutive rows, so
-// that the shared-memory stores do not conflict and the loads of a non-K-major operand coalesce.
-template <bool KMAJ, int R>
-__device__ __forceinline__ void stage(const float* __restrict__ X, int ld, int nrows, int K, int r0, int k0,
-                                      uint8_t* dst)
+// that the shared-memory stores do not conflict and the loads of a non-K-major operand coalesce.  A K-major row that
+// starts on 16 bytes is read four floats at a time.
+// The products of the network are small (768 x 256 x 256: 12 tiles, 4 steps), so what counts is the trips to memory: every
+// load of a step, of both operands, is issued before the first is used, and the next step's while this one's MMAs
+// run.  (A loop of one chunk after the other made sixteen trips per step and such a product 55 us.)
+constexpr int NCHUNK = BK / 8;   // chunks per thread: thread t takes row t of every chunk column
+static_assert(BM == THREADS && BN == THREADS, "a row per thread");
+
+template <bool KMAJ>
+__device__ __forceinline__ void load_rows(float (&v)[NCHUNK][8], const float* __restrict__ X, int ld, int nrows, int K,
+                                          int r0, int k0)
 {
-    for (int e = threadIdx.x; e < R * (BK / 8); e += THREADS)
+    constexpr int N = NCHUNK;
+    const int gr = r0 + threadIdx.x;
+    const bool wide = KMAJ && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0 && k0 + BK <= K;
+    if (wide)
     {
-        const int r = e % R, c = e / R;
-        const int gr = r0 + r, gk = k0 + 8 * c;
-        float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-        {
-            v[j] = 0.f;
-            if (gr < nrows && gk + j < K)
-                v[j] = KMAJ ? __ldg(X + (size_t)gr * ld + gk + j) : __ldg(X + (size_t)(gk + j) * ld + gr);
-        }
+        for (int c = 0; c < N; ++c)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+            {
+                float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (gr < nrows) f = __ldg(reinterpret_cast<const float4*>(X + (size_t)gr * ld + k0 + 8 * c + 4 * h));
+                v[c][4 * h] = f.x; v[c][4 * h + 1] = f.y; v[c][4 * h + 2] = f.z; v[c][4 * h + 3] = f.w;
+            }
+    }
+    else
+    {
+#pragma unroll
+        for (int c = 0; c < N; ++c)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                const int gk = k0 + 8 * c + j;
+                v[c][j] = 0.f;
+                if (gr < nrows && gk < K) v[c][j] = KMAJ ? __ldg(X + (size_t)gr * ld + gk) : __ldg(X + (size_t)gk * ld + gr);
+            }
+    }
+}
+
+__device__ __forceinline__ void store_rows(const float (&v)[NCHUNK][8], uint8_t* dst)
+{
+    constexpr int N = NCHUNK, R = THREADS;
+    const int r = threadIdx.x;
+#pragma unroll
+    for (int c = 0; c < N; ++c)
+    {
         uint4 u;
         __nv_bfloat162 h;
-        h = __floats2bfloat162_rn(v[0], v[1]);
+        h = __floats2bfloat162_rn(v[c][0], v[c][1]);
         u.x = *reinterpret_cast<uint32_t*>(&h);
-        h = __floats2bfloat162_rn(v[2], v[3]);
+        h = __floats2bfloat162_rn(v[c][2], v[c][3]);
         u.y = *reinterpret_cast<uint32_t*>(&h);
-        h = __floats2bfloat162_rn(v[4], v[5]);
+        h = __floats2bfloat162_rn(v[c][4], v[c][5]);
         u.z = *reinterpret_cast<uint32_t*>(&h);
-        h = __floats2bfloat162_rn(v[6], v[7]);
+        h = __floats2bfloat162_rn(v[c][6], v[c][7]);
         u.w = *reinterpret_cast<uint32_t*>(&h);
         *reinterpret_cast<uint4*>(dst + (size_t)c * R * 16 + (size_t)r * 16) = u;
     }
@@ -167,6 +199,9 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(int M, int N, int K, cons
     const uint32_t tmem = tmem_base;
     bool ok = true;
     int issued = 0;   // steps whose MMAs were committed
+    float va[NCHUNK][8], vb[NCHUNK][8];   // the next step's operands
+    load_rows<!TA>(va, A, lda, M, K, m0, kc0 * BK);
+    load_rows<TB>(vb, B, ldb, N, K, n0, kc0 * BK);
     for (int i = 0; i < nk; ++i)
     {
         const int s = i % NSTAGE;
@@ -183,9 +218,8 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(int M, int N, int K, cons
                 break;
             }
         }
-        const int k0 = (kc0 + i) * BK;
-        stage<!TA, BM>(A, lda, M, K, m0, k0, sa);
-        stage<TB, BN>(B, ldb, N, K, n0, k0, sb);
+        store_rows(va, sa);
+        store_rows(vb, sb);
         // the generic-proxy stores become visible to the tensor cores (async proxy)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
@@ -200,6 +234,11 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(int M, int N, int K, cons
             commit(&bar[s]);
         }
         issued = i + 1;
+        if (i + 1 < nk)
+        {
+            load_rows<!TA>(va, A, lda, M, K, m0, (kc0 + i + 1) * BK);
+            load_rows<TB>(vb, B, ldb, N, K, n0, (kc0 + i + 1) * BK);
+        }
     }
     if (ok)
     {
@@ -214,25 +253,39 @@ __global__ void __launch_bounds__(THREADS) gemm_kernel(int M, int N, int K, cons
     fence_after();
     if (ok)
     {
-        const int row = m0 + 32 * warp + lane;
-        const bool add_bias = bias && blockIdx.z == 0;
+        // accumulator rows (one per thread) to shared memory -- the MMAs that read the stages are done -- and from there
+        // row by row, neighbouring lanes at neighbouring columns (a thread writing its own row touched 32 rows per
+        // instruction)
+        constexpr int LD = BN + 1;
+        float* const tile = reinterpret_cast<float*>(tc_smem);
         for (int c = 0; c < BN; c += 16)
         {
             uint32_t r[16];
             tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c, r);
-            if (row < M)
-            {
-                float* crow = C + (size_t)row * ldc;
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                {
-                    const int n = n0 + c + j;
-                    if (n >= N) continue;
-                    const float v = __uint_as_float(r[j]) + (add_bias ? bias[n] : 0.f);
-                    if (mode == 2) atomicAdd(crow + n, v);
-                    else if (mode == 1) crow[n] += v;
-                    else crow[n] = v;
-                }
+            for (int j = 0; j < 16; ++j) tile[(32 * warp + lane) * LD + c + j] = __uint_as_float(r[j]);
+        }
+        __syncwarp();
+        const bool add_bias = bias && blockIdx.z == 0;
+        float b[BN / 32];
+#pragma unroll
+        for (int j = 0; j < BN / 32; ++j)
+        {
+            const int n = n0 + 32 * j + lane;
+            b[j] = add_bias && n < N ? bias[n] : 0.f;
+        }
+        for (int i = 0; i < 32 && m0 + 32 * warp + i < M; ++i)
+        {
+            float* const crow = C + (size_t)(m0 + 32 * warp + i) * ldc;
+#pragma unroll
+            for (int j = 0; j < BN / 32; ++j)
+            {
+                const int n = n0 + 32 * j + lane;
+                if (n >= N) continue;
+                const float v = tile[(32 * warp + i) * LD + 32 * j + lane] + b[j];
+                if (mode == 2) atomicAdd(crow + n, v);
+                else if (mode == 1) crow[n] += v;
+                else crow[n] = v;
             }
         }
     }
@@ -267,8 +320,9 @@ void gemm(int M, int N, int K, const float* A, int lda, const float* B, int ldb,
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const int tm = (M + tc::BM - 1) / tc::BM, tn = (N + tc::BN - 1) / tc::BN;
     const int nchunks = std::max(1, (K + tc::BK - 1) / tc::BK);
-    // split K until about two CTAs per SM are busy, keeping at least 4 steps per split
-    int splits = std::min(std::max(1, nchunks / 4), std::max(1, 2 * nsm / (tm * tn)));
+    // a long K (the weight gradients, 8 steps or more) is split until about two CTAs per SM are busy, keeping at
+    // least 2 steps per split
+    int splits = nchunks < 8 ? 1 : std::min(nchunks / 2, std::max(1, 2 * nsm / (tm * tn)));
     const int per = (nchunks + splits - 1) / splits;
     splits = (nchunks + per - 1) / per;   // no empty split
     int mode = accumulate ? 1 : 0;
@@ -313,14 +367,30 @@ __global__ void silu_back_kernel(const float* __restrict__ z, float* __restrict_
     }
 }
 
+// sum of s over the block's threads (a multiple of 32, at most 1024), in thread 0
+__device__ __forceinline__ float block_sum(float s)
+{
+    __shared__ float part[32];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32)
+    {
+        s = threadIdx.x < blockDim.x / 32 ? part[threadIdx.x] : 0.f;
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
+    return s;
+}
+
 // masked mean-squared error: dy = 2 mask (y - t) / sum(mask); loss partial sums into acc[0], mask sum in acc[1]
+// (one atomic per block: one per warp, all on the same address, took most of the kernels' 17 us)
 __global__ void mask_sum_kernel(const float* __restrict__ mask, long long n, float* acc)
 {
     float s = 0.f;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         s += mask[i];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(acc + 1, s);
+    s = block_sum(s);
+    if (threadIdx.x == 0) atomicAdd(acc + 1, s);
 }
 
 __global__ void mse_grad_kernel(const float* __restrict__ y, const float* __restrict__ t, const float* __restrict__ mask,
@@ -334,18 +404,28 @@ __global__ void mse_grad_kernel(const float* __restrict__ y, const float* __rest
         s += r * r;
         dy[i] = 2.f * r * inv;
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(acc, s * inv);
+    s = block_sum(s);
+    if (threadIdx.x == 0) atomicAdd(acc, s * inv);
 }
 
-// db[o] = sum_rows d[row][o]
-__global__ void colsum_kernel(const float* __restrict__ d, int rows, int cols, float* __restrict__ db)
+// db[o] = sum_rows d[row][o]: a block takes 32 columns, its 32 rows of threads every 32nd row each (one thread per
+// column over all rows was a chain of `rows` loads: 46 us at 768 rows)
+__global__ void __launch_bounds__(1024) colsum_kernel(const float* __restrict__ d, int rows, int cols, float* __restrict__ db)
 {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= cols) return;
+    __shared__ float part[32][33];
+    const int o = blockIdx.x * 32 + threadIdx.x;
     float s = 0.f;
-    for (int r = 0; r < rows; ++r) s += d[(size_t)r * cols + o];
-    db[o] = s;
+    if (o < cols)
+    {
+#pragma unroll 8
+        for (int r = threadIdx.y; r < rows; r += 32) s += d[(size_t)r * cols + o];
+    }
+    part[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    s = part[threadIdx.x][threadIdx.y];
+    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    const int c = blockIdx.x * 32 + threadIdx.y;
+    if (threadIdx.x == 0 && c < cols) db[c] = s;
 }
 
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -589,7 +669,7 @@ int qcg_mlp_loss_grad(qcg_mlp* m, int rows, const float* d_x, const float* d_t, 
             // dW = dZ^T X  ([out x rows] [rows x in]),  db = column sums of dZ,  dX = dZ W
             gemm<true, false>(out, in, rows, dcur, out, m->X[l], in, m->d_g + m->woff[l], in, nullptr, false,
                               m->stream);
-            colsum_kernel<<<(out + 255) / 256, 256, 0, m->stream>>>(dcur, rows, out, m->d_g + m->boff[l]);
+            colsum_kernel<<<(out + 31) / 32, dim3(32, 32), 0, m->stream>>>(dcur, rows, out, m->d_g + m->boff[l]);
             if (l > 0)
             {
                 gemm<false, false>(rows, in, out, dcur, out, m->d_p + m->woff[l], in, dnext, in, nullptr, false,
