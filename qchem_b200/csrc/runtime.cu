@@ -478,7 +478,7 @@ struct qcg_handle
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     // side streams for the class kernels of one build (fork after the accumulators are zeroed, join before
     // the symmetrisation), so that classes with few quartets run side by side
-    static constexpr int kSide = 6;
+    static constexpr int kSide = 16;
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork = nullptr, join[kSide] = {};
     // J/K builds replayed as CUDA graphs, keyed by their arguments and the screening generation
@@ -2437,12 +2437,16 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     const bool det = (flags & QCG_JK_DETERMINISTIC) != 0;
     require(!det || fp32_below <= 0, "the deterministic J/K build evaluates every quartet in FP64 (no FP32 band)");
     const size_t nacc = det ? 2 * nn : nn;
+    // side streams of this build: a molecule's few quartets are a dozen lone blocks per class, so every class gets a
+    // stream (one water: 158 us on six streams, 139 on sixteen; contracted 235, 177); from a few hundred thousand
+    // quartets on more classes side by side cost more than they fill (two waters: 571 and 614 us)
+    const int nside = h->work_quartets <= (1LL << 19) ? qcg_handle::kSide : 6;
     auto enqueue = [&](bool timed) {
         CK(cudaMemsetAsync(h->d_Jp, 0, nacc * sizeof(double), h->stream));
         CK(cudaMemsetAsync(h->d_Kp, 0, nacc * sizeof(double), h->stream));
         if (timed) CK(cudaEventRecord(h->ev1, h->stream));
         CK(cudaEventRecord(h->fork, h->stream));
-        for (int s = 0; s < qcg_handle::kSide; ++s) CK(cudaStreamWaitEvent(h->side[s], h->fork, 0));
+        for (int s = 0; s < nside; ++s) CK(cudaStreamWaitEvent(h->side[s], h->fork, 0));
         // heaviest classes first so that the short ones fill the tail; classes spread over the side streams
         int slot = 0;
         for (int k = kNumQuartetClasses - 1; k >= 0; --k)
@@ -2467,7 +2471,7 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
             auto stream = [&]() {
                 if (alone) return h->side[0];
                 const cudaStream_t st = h->side[slot];
-                slot = (slot + 1) % qcg_handle::kSide;
+                slot = (slot + 1) % nside;
                 return st;
             };
             if (fp32_below < HUGE_VAL)
@@ -2499,7 +2503,7 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
             }
         }
         CK(cudaGetLastError());
-        for (int s = 0; s < qcg_handle::kSide; ++s)
+        for (int s = 0; s < nside; ++s)
         {
             CK(cudaEventRecord(h->join[s], h->side[s]));
             CK(cudaStreamWaitEvent(h->stream, h->join[s], 0));
