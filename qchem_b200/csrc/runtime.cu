@@ -2417,9 +2417,11 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     jk_team_plan(h, team_want, jk_forced, team);
     // classes in the warp-shared form (FP64 band, one rank, not deterministic; the team form comes first);
     // their work items are built here, before any capture.  The build's default applies to full builds of
-    // classes with at least kJKTeamMinQuartets quartets: under density screening a warp evaluates every
-    // quartet that one of its lanes needs, where the thread-per-quartet form skips each one alone.  A mask
-    // set by qcg_set_jk_warp_classes or QCG_JK_WARP_MASK applies to every build.
+    // uncontracted classes with at least kJKWarpMinQuartets quartets: under density screening a warp evaluates every
+    // quartet that one of its lanes needs, where the thread-per-quartet form skips each one alone, and of a
+    // contracted basis its few items of 256 kets run serial primitive loops (eight waters, 296 functions: (dp|ss)
+    // 13.2 ms against 1.8 thread-per-quartet, (pp|ss) 10.2 against 2.4).  A mask set by qcg_set_jk_warp_classes or
+    // QCG_JK_WARP_MASK applies to every build.
     bool warp_forced = h->jk_warp_mask >= 0;
     const unsigned warp_mask =
         warp_forced ? (unsigned)h->jk_warp_mask : jk_warp_mask_default(&warp_forced);
@@ -2427,7 +2429,8 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     for (int k = 0; k < kNumQuartetClasses; ++k)
         if (((warp_mask >> k) & 1u) && !team.on[k] && h->work[k].total > 0 && h->shard_world == 1 &&
             !(flags & QCG_JK_DETERMINISTIC) &&
-            (warp_forced || (dmax == nullptr && dthr <= 0.0 && !split[k] && h->work[k].total >= kJKWarpMinQuartets)))
+            (warp_forced || (dmax == nullptr && dthr <= 0.0 && !split[k] && team_kmax(h, k) == 1 &&
+                             h->work[k].total >= kJKWarpMinQuartets)))
         {
             warp_items(h, k);
             warp_k[k] = h->nwitems[k] > 0;
