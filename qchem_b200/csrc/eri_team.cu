@@ -95,14 +95,14 @@ struct Cls
     static constexpr int kKetStage = gen::QCG_CAT(kTeamKetStage, QCG_CLASS);
     static constexpr int kNG = team_pieces(kNCode, kNH, kNE), kNW = 3 * kNG;
     static constexpr int kMinBlocks = team_min_blocks(kNG, kStage), kUnroll = team_unroll(kNG, kStage);
-    // jk_group_kernel: groups of 32 quartets per round (two sets of stages within the shared memory), its warps --
-    // eight where Y_f, acc_f or the digestion of a (dd| bra need more registers than twelve leave -- and CTAs per SM
+    // jk_group_kernel: eight warps (the digestion needs more registers than twelve leave), and up to eight groups of 32
+    // quartets, one per warp, as far as their stages fit the shared memory
     static constexpr int kGroups = [] {
-        const int g = (int)((227 * 1024 - 8192 - (int)(kBoysRows * kBoysColumns * sizeof(double))) /
-                            (2 * kStage * 32 * sizeof(double)));
-        return g < 1 ? 1 : (g > 4 ? 4 : g);
+        const int g = (int)((227 * 1024 - 4096 - (int)(kBoysRows * kBoysColumns * sizeof(double))) /
+                            (kStage * 32 * sizeof(double)));
+        return g < 1 ? 1 : (g > 8 ? 8 : g);
     }();
-    static constexpr int kJKWarps = LA + LB == 4 ? 8 : 12, kJKBlocks = 1;
+    static constexpr int kJKWarps = 8, kJKBlocks = 1;
     static __device__ __forceinline__ unsigned long long column(int cd) { return gen::QCG_CAT(kTeamColumn, QCG_CLASS)[cd]; }
     static __device__ __forceinline__ double column_norm(int cd) { return gen::QCG_CAT(kTeamColumnNorm, QCG_CLASS)[cd]; }
     template <class Sink>
@@ -157,7 +157,7 @@ constexpr int kThreads = Cls::kNW * 32;
 constexpr int kNCD = ncart(Cls::LC) * ncart(Cls::LD);
 constexpr size_t kSmem = team_smem(Cls::kNG, Cls::kStage);   // the stages and the Boys columns
 constexpr size_t kGroupSmem =
-    (2 * (size_t)Cls::kGroups * Cls::kStage * 32 + kBoysRows * kBoysColumns) * sizeof(double);
+    ((size_t)Cls::kGroups * Cls::kStage * 32 + kBoysRows * kBoysColumns) * sizeof(double);
 std::atomic<unsigned long long> g_smem_ready{0};
 }   // namespace
 
