@@ -156,9 +156,10 @@ int qcg_eri_batch_device(qcg_handle* h, int la, int lb, int lc, int ld, long lon
  * (src/BasisSet/Molecule/Evaluators/PG_Cart_MnD/Evaluator.C:1905-1908, primitive integral GaussianRF.C:415-444),
  * the integrals of density-fitted Coulomb.  Fitting shells are ordinary shells of the handle.  Host buffers. */
 int qcg_eri3_batch(qcg_handle* h, int la, int lb, int lc, long long nt, const int* triples, double* out);
-/* FP32 forms of the two batch calls: the same integrals evaluated in FP32 arithmetic (pair data, Boys
- * argument, prefactor and Boys below T = 12 in FP64, rounded once) with float output.  No reference
- * counterpart (the reference is FP64 only). */
+/* FP32 forms of the two batch calls: the same integrals with float output, accurate to FP32 or better.  The team
+ * kernels evaluate them in FP64 and round once (on this GPU faster than the FP32 evaluation); where their scratch
+ * does not fit the handle's memory limit, the FP32 kernels run (pair data, Boys argument, prefactor and Boys below
+ * T = 12 in FP64, rounded once).  No reference counterpart (the reference is FP64 only). */
 int qcg_eri_batch_f32(qcg_handle* h, int la, int lb, int lc, int ld, long long nq, const int* quartets, float* out);
 int qcg_eri_batch_device_f32(qcg_handle* h, int la, int lb, int lc, int ld, long long nq, const int* d_quartets,
                              float* d_out);
@@ -173,7 +174,8 @@ int qcg_fock_jk(qcg_handle* h, const double* D, double* J, double* K, int flags,
 int qcg_fock_jk_device(qcg_handle* h, const double* d_D, double* d_J, double* d_K, int flags, qcg_stats* stats);
 /* Mixed precision for later qcg_fock_jk / qcg_fock_jk_device calls: quartets whose density-weighted
  * Schwarz bound Q_ab Q_cd max|D| (max over the six D blocks the quartet touches) is below `bound` are
- * evaluated in FP32 (accumulated in FP64), the rest in FP64.  0 (the default) keeps every quartet FP64.
+ * evaluated in FP32 (accumulated in FP64), the rest in FP64, in classes of fewer than 2^15 quartets; larger classes
+ * are faster in FP64 throughout and are evaluated so.  0 (the default) keeps every quartet FP64.
  * No reference counterpart. */
 int qcg_set_fp32_bound(qcg_handle* h, double bound);
 /* 1: J/K builds repeated with the same arguments (device pointers, screening, precision) are captured as
@@ -187,20 +189,19 @@ int qcg_set_graphs(qcg_handle* h, int enable);
  * choice, or the mask in the environment variable QCG_ERI_TEAM_MASK.  Both forms give the same integrals
  * to rounding.  No reference counterpart. */
 int qcg_set_eri_team_classes(qcg_handle* h, long long mask);
-/* The same choice for the direct J/K build (bit k: class k of the work lists): the team kernel, whose CTAs
- * digest each group's integral blocks into J and K, or the thread-per-quartet kernel; -1 (default): the
- * library's choice -- the team form for the (dd|xx) classes except (dd|ss), and (dp|dp), of a build with at least
- * 2^20 quartets in the class -- or QCG_JK_TEAM_MASK in the environment (a mask set here or there applies at
- * any size).  Same J and K to rounding (bit for bit under QCG_JK_DETERMINISTIC only within one form).  No
- * reference counterpart. */
+/* The same choice for the direct J/K build (bit k: class k of the work lists): the team kernels, whose CTAs
+ * digest each group's integral blocks into J and K, or the other forms; -1 (default): the library's choice -- the
+ * (dd|xx) classes except (dd|ss), and (dp|dp), (dp|pp) and (dp|ds), where the class is uncontracted in the basis, every
+ * class without an (ss) ket where it is contracted -- or QCG_JK_TEAM_MASK in the environment.  Same J and K to
+ * rounding (bit for bit under QCG_JK_DETERMINISTIC only within one form).  No reference counterpart. */
 int qcg_set_jk_team_classes(qcg_handle* h, long long mask);
 /* The warp-shared form of the direct J/K build for the classes in mask (bit k: class k; the team form takes
  * precedence where both are set): each half of a warp takes up to 16 bra pairs sharing their first shell
  * against one ket pair at a time, so that the J'(cd), K'(ac) and K'(ad) contributions of its lanes are added
  * by warp shuffles and written once per half warp instead of once per lane.  FP64 builds of one rank (not
  * with qcg_set_shard or QCG_JK_DETERMINISTIC).  -1 (default): the library's choice -- the (ps|ss), (ps|ps),
- * (pp|ss), (pp|ps), (ds|xx), (dp|ss), (dp|ps), (dp|pp) and (dp|ds) classes of full builds with at least 2^20
- * quartets in the class -- or QCG_JK_WARP_MASK in the environment (a mask set here or there applies to every
+ * (pp|ss), (pp|ps), (ds|xx), (dp|ss) and (dp|ps) classes of full builds with at least 2^20 quartets in the class,
+ * where it is uncontracted in the basis -- or QCG_JK_WARP_MASK in the environment (a mask set here or there applies to every
  * build).  Same J
  * and K to rounding.  No reference counterpart. */
 int qcg_set_jk_warp_classes(qcg_handle* h, long long mask);

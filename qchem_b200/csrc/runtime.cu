@@ -214,8 +214,10 @@ public:
     static constexpr size_t kScratchIdle = (size_t)2 << 30;
     void* scratch(int dev, size_t bytes, size_t* cap)
     {
-        const size_t unit = (size_t)1 << 20;
-        *cap = (bytes + unit - 1) / unit * unit;
+        // capacities are powers of two from 1 MiB, so that the classes of one batch after another grow the scratch a few
+        // times at most and later handles find the same sizes idle
+        *cap = (size_t)1 << 20;
+        while (*cap < bytes) *cap <<= 1;
         std::vector<void*> drop;
         {
             std::lock_guard<std::mutex> g(mu_);
@@ -244,6 +246,12 @@ public:
             }
             for (void* q : drop) cudaFree(q);
             e = cudaMalloc(&p, *cap);
+            if (e == cudaErrorMemoryAllocation)
+            {
+                cudaGetLastError();
+                *cap = bytes;
+                e = cudaMalloc(&p, *cap);
+            }
         }
         if (e != cudaSuccess)
         {
