@@ -36,7 +36,10 @@ constexpr int cls_X()
 constexpr int kX = cls_X();
 constexpr int kY = QCG_CLASS - kX * (kX + 1) / 2;
 
-// Pieces of ket code per pass (kNG; each runs on three warps, one per rotation).  A thread keeps Y_f and acc_f
+// Pieces of ket code per pass (kNG; each runs on three warps, one per rotation).  With a piece per component, 31 for
+// (dd|dd), four warps on four pieces outran eight on eight, because the code in flight has to fit the instruction
+// cache: 8 passes, 19.2 ms for 250 000 quartets.  With a piece per orbit twelve warps run four pieces: 3 passes,
+// 12.1 ms, and no_instruction fell from 24% of the stall samples to 2%.  A thread keeps Y_f and acc_f
 // in registers, and the SM's 65 536 registers are split among four schedulers, so ceil(3 g / 4) warps per
 // scheduler leave each thread 512 / ceil(3 g / 4) registers (255 at most): g is the largest for which Y_f, acc_f
 // and kTemps further registers fit, and the pieces are then spread evenly over the passes.

@@ -72,7 +72,8 @@ __device__ __forceinline__ TeamPair team_pair_load(int t, int lane)
 
 // Phase 1 of both kernels: the stage tables of the group's primitive quartets into rc.  bra(i) and ket(i) give
 // this lane's primitive pairs; each is formed once, by the warps in turn, and read back from shared memory by the
-// stages that use it (a contraction too long for that space forms them stage by stage).
+// stages that use it (a contraction too long for that space forms them stage by stage).  A pair is two divisions and
+// an exponential; formed by every stage they took half of a (ps|ps) stage's 2150 cycles.
 template <class Cls, class Bra, class Ket>
 __device__ __forceinline__ void team_stages(double* __restrict__ rc, const int Kab, const int Kcd, const int Kg,
                                             const BoysColumns& bt, Bra bra, Ket ket)
@@ -304,7 +305,8 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         __syncthreads();
         // the bra recurrence of W neighbouring columns at a time into the stage space, one column per warp and lane,
         // then out quartet by quartet: a quartet's runs of W values go out by neighbouring lanes.  (Each lane
-        // storing its own column wrote 8 bytes at 32 places, on 32 pages, per instruction.)
+        // storing its own column wrote 8 bytes at 32 places, on 32 pages, per instruction: 4.3k of 22k cycles per
+        // primitive quartet of (dd|dd), 1.5k so.)
         constexpr int NAB = ncart(Cls::LA) * ncart(Cls::LB), W = NCD < NW ? NCD : NW;
         static_assert(NAB * W * 33 <= Cls::kStageSpace, "the columns fit the stage space");
         for (int c0 = 0; c0 < NCD; c0 += W)

@@ -2226,7 +2226,8 @@ struct JKTeamPlan
 // lanes.  Here the kets of a pair class are also listed by primitive-pair count (bounds descending within one), so
 // that a bra pair's screened kets are a run of each count's list; the runs are taken longest loop first.  A loop
 // longer than a CTA's average share of all loops (at least kTeamChain) is cut into runs of bra primitive pairs.
-// Built once per screening, before any capture.
+// Built once per screening, before any capture.  Split-valence basis: one water 416 -> 254 us, four 5.2 -> 3.3 ms,
+// eight 51.8 -> 41.3 ms.
 constexpr int kTeamChain = 9;
 const JKTeamListDev& jk_team_list(qcg_handle* h, int k, int ctas)
 {
