@@ -84,7 +84,7 @@ template <class Cls, bool DET>
 __device__ __forceinline__ void team_digest(const JKWorkDev& w, const PairListDev& bra, const PairListDev& ket,
                                             const PrimPairsDev& P, const int* __restrict__ shell_f0,
                                             const double* __restrict__ D, double* __restrict__ J,
-                                            double* __restrict__ K, int n, const double* __restrict__ h, bool valid,
+                                            double* __restrict__ K, int n, const double* h, bool valid,
                                             int i, int j, int cd0, int cd1, int lane)
 {
     constexpr int NE = Cls::kNE, NF = Cls::kNF;
@@ -252,7 +252,7 @@ template <class Cls, bool DET>
 __device__ __forceinline__ void team_digest_rows(const JKWorkDev& w, const PairListDev& bra, const PairListDev& ket,
                                                  const PrimPairsDev& P, const int* __restrict__ shell_f0,
                                                  const double* __restrict__ D, double* __restrict__ J,
-                                                 double* __restrict__ K, int n, const double* __restrict__ h, bool valid,
+                                                 double* __restrict__ K, int n, const double* h, bool valid,
                                                  int i, int j, int ic0, int ic1, int lane)
 {
     constexpr int NE = Cls::kNE, NF = Cls::kNF;

@@ -440,8 +440,10 @@ struct qcg_handle
         long long counted = 0;   // bytes in mem_used: what was asked for, whatever the cache gave
     };
     Scratch team_scr, jk_scr;
-    // at least `doubles` in s, for work queued on the handle's stream from now on; a buffer that has to grow goes back
-    // to the cache once the work that may use it is done
+    // at least `doubles` in s, for work queued on the handle's stream from now on.  A buffer that has to grow stays with
+    // the handle until it goes: work in flight, or a graph that the caller captured, may hold its address.  (Under a
+    // memory limit it goes back to the cache at once, after the work that may use it.)
+    std::vector<Scratch> retired;
     double* scratch(Scratch& s, long long doubles)
     {
         const size_t bytes = (size_t)doubles * sizeof(double);
@@ -449,8 +451,16 @@ struct qcg_handle
         if (s.p)
         {
             if (&s == &jk_scr) drop_graphs();
-            CK(cudaStreamSynchronize(stream));
-            give_scratch(s, true);
+            if (mem_limit > 0)
+            {
+                CK(cudaStreamSynchronize(stream));
+                give_scratch(s, true);
+            }
+            else
+            {
+                retired.push_back(s);
+                s = Scratch{};
+            }
         }
         if (mem_limit > 0 && mem_used + (long long)bytes > mem_limit)
             throw Error{QCG_ERR_ALLOC, "device memory limit of " + std::to_string(mem_limit) + " bytes exceeded"};
@@ -673,6 +683,7 @@ struct qcg_handle
         }
         give_scratch(team_scr, healthy);
         give_scratch(jk_scr, healthy);
+        for (Scratch& r : retired) give_scratch(r, healthy);
         if (stage)
         {
             if (healthy) rc.give_stage(stage);
@@ -2317,7 +2328,17 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
         const int kmax = team_kmax(h, k);
         TeamShape& sh = plan.sh[k];
         sh = team_shape(h, k);
-        if (kmax > 1 && h->shard_world == 1) plan.scr[k].list = jk_team_list(h, k, sh.grid);
+        try
+        {
+            if (kmax > 1 && h->shard_world == 1) plan.scr[k].list = jk_team_list(h, k, sh.grid);
+        }
+        catch (const Error& e)
+        {
+            if (required || e.code != QCG_ERR_ALLOC) throw;
+            h->team_list[k] = JKTeamListDev{};
+            h->team_list_ready[k] = false;
+            continue;
+        }
         const long long ngroups = ((plan.scr[k].list.n ? plan.scr[k].list.total : ge - gb) + 31) / 32;
         sh.grid = (int)std::min<long long>(sh.grid, ngroups);
         sh.group_grid = (int)std::min<long long>(sh.group_grid, ngroups);
