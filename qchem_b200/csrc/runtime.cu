@@ -484,8 +484,8 @@ struct qcg_handle
     int maxnp[kMaxL + 1] = {};   // largest contraction length per angular momentum (0: not yet computed)
 
     // host-buffer ERI batches: two quartet/output buffer pairs (grow only) and a copy-out stream
-    void* hb_q[2] = {nullptr, nullptr};
-    void* hb_out[2] = {nullptr, nullptr};
+    char* hb_q[2] = {nullptr, nullptr};
+    char* hb_out[2] = {nullptr, nullptr};
     size_t hb_qcap[2] = {0, 0}, hb_ocap[2] = {0, 0};
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t hb_done[2] = {nullptr, nullptr}, hb_free[2] = {nullptr, nullptr};
@@ -590,6 +590,15 @@ struct qcg_handle
                 allocs.erase(allocs.begin() + i);
                 return;
             }
+    }
+    // p, released, as a buffer of `count` elements; null if that cannot be had, so that no address of released memory
+    // is left behind (the caller's capacity must be zero meanwhile)
+    template <class T>
+    void regrow(T*& p, size_t count)
+    {
+        if (p) release(p);
+        p = nullptr;
+        p = alloc<T>(count);
     }
     // Uploads between begin_uploads() and flush_uploads() are merged: a piece whose device address and
     // staging offset both continue the previous piece (consecutive slab allocations do) extends one pending
@@ -1831,14 +1840,14 @@ void ensure_side_streams(qcg_handle* h)
 
 void ensure_jk_buffers(qcg_handle* h)
 {
-    if (h->d_Jp) return;
+    if (h->d_flag) return;   // the last one: after a call that could not have them all the next one goes on
     const size_t nn = (size_t)h->packed;
-    h->d_D = h->alloc<double>(nn);
+    if (!h->d_D) h->d_D = h->alloc<double>(nn);
     // room for the deterministic mode's low words (QCG_JK_DETERMINISTIC): J' and K' are 2 nn words each
-    h->d_Jp = h->alloc<double>(2 * nn);
-    h->d_Kp = h->alloc<double>(2 * nn);
-    h->d_J = h->alloc<double>(nn);
-    h->d_K = h->alloc<double>(nn);
+    if (!h->d_Jp) h->d_Jp = h->alloc<double>(2 * nn);
+    if (!h->d_Kp) h->d_Kp = h->alloc<double>(2 * nn);
+    if (!h->d_J) h->d_J = h->alloc<double>(nn);
+    if (!h->d_K) h->d_K = h->alloc<double>(nn);
     h->d_flag = h->alloc<int>(1);
 }
 
@@ -2616,15 +2625,12 @@ const int* batch_order(qcg_handle* h, const int* d_quartets, long long nq, int c
     require(nq <= 0x7fffffffLL, "at most 2^31-1 quartets per batch");
     if (nq > h->sort_cap)
     {
-        if (h->d_key) { h->release(h->d_key); h->release(h->d_order); }
-        if (!h->d_hist)
-        {
-            h->d_hist = h->alloc<int>(256);
-            h->d_cursor = h->alloc<int>(256);
-            h->d_plan = h->alloc<BatchPlanDev>(1);
-        }
-        h->d_key = h->alloc<unsigned char>(nq);
-        h->d_order = h->alloc<int>(nq);
+        h->sort_cap = 0;
+        if (!h->d_hist) h->d_hist = h->alloc<int>(256);
+        if (!h->d_cursor) h->d_cursor = h->alloc<int>(256);
+        if (!h->d_plan) h->d_plan = h->alloc<BatchPlanDev>(1);
+        h->regrow(h->d_key, nq);
+        h->regrow(h->d_order, nq);
         h->sort_cap = nq;
     }
     launch_pattern_sort(h->bs, (const int4*)d_quartets, nq, h->d_key, h->d_hist, h->d_cursor, h->d_order, ctas,
@@ -3090,14 +3096,14 @@ void eri_batch_run(qcg_handle* h, int la, int lb, int lc, int ld, long long nq, 
         {
             if (h->hb_qcap[b] < qbytes)
             {
-                if (h->hb_q[b]) h->release(h->hb_q[b]);
-                h->hb_q[b] = h->alloc<char>(qbytes);
+                h->hb_qcap[b] = 0;
+                h->regrow(h->hb_q[b], qbytes);
                 h->hb_qcap[b] = qbytes;
             }
             if (h->hb_ocap[b] < obytes)
             {
-                if (h->hb_out[b]) h->release(h->hb_out[b]);
-                h->hb_out[b] = h->alloc<char>(obytes);
+                h->hb_ocap[b] = 0;
+                h->regrow(h->hb_out[b], obytes);
                 h->hb_ocap[b] = obytes;
             }
             CK(cudaEventRecord(h->hb_free[b], h->copy_stream));   // both buffers start free

@@ -1,0 +1,54 @@
+"""Handles that cannot have all the device memory they ask for: a call that fails leaves the handle usable, a form that
+is chosen for speed makes room for what a call cannot do without, and the cap on a handle's memory is kept."""
+import numpy as np
+import pytest
+
+from qchem_b200 import api, basis as B, workloads as W
+
+pytestmark = pytest.mark.gpu
+
+FOCK_ABS = 1e-10
+ERI_ABS = 1e-12
+
+
+def _pool(n, most, seed):
+    rng = np.random.default_rng(seed)
+    return [B.Shell(L, tuple(rng.uniform(0.0, 6.0, size=3)), list(np.exp(rng.uniform(np.log(0.05), np.log(50.0), size=k))),
+                    list(rng.uniform(0.1, 1.0, size=k)))
+            for L in range(3) for k in rng.integers(1, most + 1, size=n)]
+
+
+def _density(n, seed=3):
+    Q, _ = np.linalg.qr(np.random.default_rng(seed).normal(size=(n, 5)))
+    return 2.0 * Q @ Q.T
+
+
+def _refused(call):
+    with pytest.raises(api.QcgError) as e:
+        call()
+    assert e.value.code == api.QCG_ERR_ALLOC
+
+
+def test_buffers_that_could_not_grow(oracle_mod):
+    """A batch, and a J/K build, that find no room leave no address of released memory: what the handle allocates next
+    and a smaller batch after it do not meet."""
+    sh = B.even_tempered(W.water())
+    eng, ob = api.Engine(sh), oracle_mod.OracleBasis(sh)
+    cls = (1, 0, 0, 0)
+    s, p = ([i for i, x in enumerate(sh) if x.L == L] for L in (0, 1))
+    q = np.array([[p[i % len(p)], s[i % 3], s[i % 5], s[i % 2]] for i in range(300)], dtype=np.int32)
+    ref = ob.eri_batch(q).reshape(300, -1)
+    assert np.abs(eng.eri_batch(cls, q[:60]) - ref[:60]).max() <= ERI_ABS
+    eng.set_memory_limit(1)
+    _refused(lambda: eng.eri_batch(cls, q))
+    eng.set_memory_limit(0)
+    eng.schwarz(1e-10)
+    eng.set_memory_limit(1)
+    D = _density(eng.nbf)
+    _refused(lambda: eng.fock_jk(D))
+    eng.set_memory_limit(0)
+    Jr, Kr = ob.jk_direct(D)[:2]
+    for n in (60, 20, 300):
+        J, K, _ = eng.fock_jk(D)
+        assert np.abs(J - Jr).max() <= FOCK_ABS and np.abs(K - Kr).max() <= FOCK_ABS
+        assert np.abs(eng.eri_batch(cls, q[:n]) - ref[:n]).max() <= ERI_ABS
