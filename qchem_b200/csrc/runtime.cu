@@ -132,7 +132,11 @@ public:
         }
         void* p = nullptr;
         const cudaError_t e = cudaMalloc(&p, kSlab);
-        if (e != cudaSuccess) throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+        if (e != cudaSuccess)
+        {
+            cudaGetLastError();   // reported here; the call may go on in another form
+            throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+        }
         return p;
     }
     char* stage()
@@ -412,8 +416,19 @@ struct qcg_handle
     int4* d_witems[kNumQuartetClasses] = {};
     long long nwitems[kNumQuartetClasses] = {};
     bool witems_ready[kNumQuartetClasses] = {};
+    // the contracted team form's order of each class (jk_team_list), built on first use after each screening; one that
+    // could not be had is not tried again until the next screening or another memory limit
+    enum class ListState { none, ready, refused };
     JKTeamListDev team_list[kNumQuartetClasses] = {};
-    bool team_list_ready[kNumQuartetClasses] = {};
+    ListState team_list_state[kNumQuartetClasses] = {};
+    void drop_team_list(int k)
+    {
+        for (const void* p : {(const void*)team_list[k].offs, (const void*)team_list[k].entry,
+                              (const void*)team_list[k].kets})
+            if (p) release((void*)p);
+        team_list[k] = JKTeamListDev{};
+        team_list_state[k] = ListState::none;
+    }
     long long jk_warp_mask = -1;   // qcg_set_jk_warp_classes; -1: the process default
     double fp32_below = 0;   // qcg_set_fp32_bound: quartets with a smaller bound are evaluated in FP32
     int shard_rank = 0, shard_world = 1;   // qcg_set_shard: this handle's slice of every J/K build
@@ -533,7 +548,11 @@ struct qcg_handle
     {
         void* p = nullptr;
         cudaError_t e = cudaMalloc(&p, bytes);
-        if (e != cudaSuccess) throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+        if (e != cudaSuccess)
+        {
+            cudaGetLastError();   // reported here; the call may go on in another form
+            throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
+        }
         return p;
     }
     // mem_used counts the bytes handed out (the limit applies to those, not to slab capacity)
@@ -2252,8 +2271,7 @@ constexpr int kTeamChain = 9;
 const JKTeamListDev& jk_team_list(qcg_handle* h, int k, int ctas)
 {
     JKTeamListDev& list = h->team_list[k];
-    if (h->team_list_ready[k]) return list;
-    h->team_list_ready[k] = true;
+    if (h->team_list_state[k] == qcg_handle::ListState::ready) return list;
     int X = 0;
     while ((X + 1) * (X + 2) / 2 <= k) ++X;
     const int Y = k - X * (X + 1) / 2;
@@ -2315,12 +2333,23 @@ const JKTeamListDev& jk_team_list(qcg_handle* h, int k, int ctas)
         entry[r] = runs[r].e;
         at[r + 1] = at[r] + runs[r].cnt;
     }
-    if (runs.empty()) return list;
-    list.offs = h->upload(at);
-    list.entry = h->upload(entry);
-    list.kets = h->upload(kets);
-    list.total = at.back();
-    list.n = (int)runs.size();
+    if (!runs.empty())
+    {
+        try
+        {
+            list.offs = h->upload(at);
+            list.entry = h->upload(entry);
+            list.kets = h->upload(kets);
+        }
+        catch (...)
+        {
+            h->drop_team_list(k);
+            throw;
+        }
+        list.total = at.back();
+        list.n = (int)runs.size();
+    }
+    h->team_list_state[k] = qcg_handle::ListState::ready;
     return list;
 }
 
@@ -2329,6 +2358,14 @@ const JKTeamListDev& jk_team_list(qcg_handle* h, int k, int ctas)
 void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool required, JKTeamPlan& plan)
 {
     long long need[kNumQuartetClasses] = {}, all = 0, most = 0;
+    bool fresh[kNumQuartetClasses] = {};   // the lists that this call made
+    // a list without its scratch serves nothing (one of an earlier build stays: a captured graph may read it)
+    auto refuse_list = [&](int k) {
+        plan.scr[k].list = JKTeamListDev{};
+        if (!fresh[k]) return;
+        h->drop_team_list(k);
+        h->team_list_state[k] = qcg_handle::ListState::refused;
+    };
     for (int k = 0; k < kNumQuartetClasses; ++k)
     {
         if (!want[k]) continue;
@@ -2337,23 +2374,31 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
         const int kmax = team_kmax(h, k);
         TeamShape& sh = plan.sh[k];
         sh = team_shape(h, k);
-        try
+        if (kmax > 1 && h->shard_world == 1)
         {
-            if (kmax > 1 && h->shard_world == 1) plan.scr[k].list = jk_team_list(h, k, sh.grid);
-        }
-        catch (const Error& e)
-        {
-            if (required || e.code != QCG_ERR_ALLOC) throw;
-            h->team_list[k] = JKTeamListDev{};
-            h->team_list_ready[k] = false;
-            continue;
+            if (!required && h->team_list_state[k] == qcg_handle::ListState::refused) continue;
+            fresh[k] = h->team_list_state[k] != qcg_handle::ListState::ready;
+            try
+            {
+                plan.scr[k].list = jk_team_list(h, k, sh.grid);
+            }
+            catch (const Error& e)
+            {
+                if (required || e.code != QCG_ERR_ALLOC) throw;
+                h->team_list_state[k] = qcg_handle::ListState::refused;
+                continue;
+            }
         }
         const long long ngroups = ((plan.scr[k].list.n ? plan.scr[k].list.total : ge - gb) + 31) / 32;
         sh.grid = (int)std::min<long long>(sh.grid, ngroups);
         sh.group_grid = (int)std::min<long long>(sh.group_grid, ngroups);
         need[k] = kmax == 1 ? std::min<long long>(ngroups, sh.group_grid * (sh.group_doubles / sh.jk_doubles)) * sh.jk_doubles
                             : sh.grid * (kmax * sh.slot_doubles + sh.jk_doubles);
-        if (need[k] * (long long)sizeof(double) > kTeamScratchMax) continue;
+        if (need[k] * (long long)sizeof(double) > kTeamScratchMax)
+        {
+            refuse_list(k);
+            continue;
+        }
         plan.on[k] = true;
         plan.scr[k].kmax = kmax;
         all += need[k];
@@ -2370,6 +2415,7 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
     catch (const Error& e)
     {
         if (required || e.code != QCG_ERR_ALLOC) throw;
+        for (int k = 0; k < kNumQuartetClasses; ++k) refuse_list(k);
         plan = JKTeamPlan{};
         return;
     }
@@ -2798,6 +2844,8 @@ int qcg_set_memory_limit(qcg_handle* h, long long bytes)
 {
     if (!h || bytes < 0) return QCG_ERR_ARG;
     h->mem_limit = bytes;
+    for (auto& s : h->team_list_state)
+        if (s == qcg_handle::ListState::refused) s = qcg_handle::ListState::none;
     return QCG_OK;
 }
 
@@ -3219,11 +3267,7 @@ int qcg_schwarz(qcg_handle* h, double thresh, double* Q)
                     h->d_witems[k] = nullptr;
                     h->nwitems[k] = 0;
                     h->witems_ready[k] = false;
-                    for (const void* p : {(const void*)h->team_list[k].offs, (const void*)h->team_list[k].entry,
-                                          (const void*)h->team_list[k].kets})
-                        if (p) h->release((void*)p);
-                    h->team_list[k] = JKTeamListDev{};
-                    h->team_list_ready[k] = false;
+                    h->drop_team_list(k);
                 }
                 h->screened = false;
             }
