@@ -137,7 +137,9 @@ const char* qcg_last_error(const qcg_handle* h);
 /* stream for all later work of this handle; NULL is the CUDA default (legacy) stream.  A new handle
  * starts on its own non-blocking stream. */
 int qcg_set_stream(qcg_handle* h, void* cuda_stream);
-int qcg_set_memory_limit(qcg_handle* h, long long bytes); /* cap on device bytes this handle allocates; 0 = none */
+/* cap on device bytes this handle allocates; 0 = none.  Calls for which the fastest form has no room run in another
+ * form (J/K builds, float batches); scratch kept for such forms makes room for what a call cannot do without. */
+int qcg_set_memory_limit(qcg_handle* h, long long bytes);
 int qcg_nbf(const qcg_handle* h, int* nbf);
 int qcg_nshell(const qcg_handle* h, int* nshell);
 /* per-function normalisation constants ns (1/sqrt of the self-overlap of the coefficient-scaled radial) */

@@ -213,21 +213,22 @@ public:
         pinned_.emplace(cap, p);
     }
     // Device scratch of the team kernels (a few MiB for a small molecule, up to GiB for contracted batches), at least
-    // `bytes`; *cap receives the capacity.  An idle buffer serves while it is not more than four times too large.
-    // Idle scratch is bounded by kScratchIdle per device; beyond it a returned buffer is freed.
+    // `bytes` and at most `budget` (>= bytes); *cap receives the capacity.  Capacities are powers of two from 1 MiB, so
+    // that the classes of one batch after another grow the scratch a few times at most and later handles find the same
+    // sizes idle -- or just `bytes` where the budget is smaller.  An idle buffer serves up to four times the power of
+    // two.  Idle scratch is bounded by kScratchIdle per device; beyond it a returned buffer is freed.
     static constexpr size_t kScratchIdle = (size_t)2 << 30;
-    void* scratch(int dev, size_t bytes, size_t* cap)
+    void* scratch(int dev, size_t bytes, size_t budget, size_t* cap)
     {
-        // capacities are powers of two from 1 MiB, so that the classes of one batch after another grow the scratch a few
-        // times at most and later handles find the same sizes idle
-        *cap = (size_t)1 << 20;
-        while (*cap < bytes) *cap <<= 1;
+        size_t pow2 = (size_t)1 << 20;
+        while (pow2 < bytes) pow2 <<= 1;
+        *cap = pow2 <= budget ? pow2 : bytes;
         std::vector<void*> drop;
         {
             std::lock_guard<std::mutex> g(mu_);
             auto& pd = per_[dev];
-            auto it = pd.scratch.lower_bound(*cap);
-            if (it != pd.scratch.end() && it->first / 4 <= *cap)
+            auto it = pd.scratch.lower_bound(bytes);
+            if (it != pd.scratch.end() && it->first <= budget && it->first / 4 <= pow2)
             {
                 void* p = it->second;
                 *cap = it->first;
@@ -446,51 +447,106 @@ struct qcg_handle
     int *d_order = nullptr, *d_hist = nullptr, *d_cursor = nullptr;
     BatchPlanDev* d_plan = nullptr;
 
-    // team-form ERI batches (eri_team.cu): per-CTA R cache and recurrence scratch (grow only), error word
-    // scratch of the team kernels: ERI batches, and J/K builds (whose address recorded graphs hold)
+    // Scratch of the team kernels: ERI batches, and J/K builds (whose address recorded graphs hold).  mem_used counts
+    // its capacity.
     struct Scratch
     {
         void* p = nullptr;
         size_t cap = 0;
-        long long counted = 0;   // bytes in mem_used: what was asked for, whatever the cache gave
+        bool captured = false;   // a graph that the caller captured holds the address: it stays until the handle goes
     };
     Scratch team_scr, jk_scr;
-    // at least `doubles` in s, for work queued on the handle's stream from now on.  A buffer that has to grow stays with
-    // the handle until it goes: work in flight, or a graph that the caller captured, may hold its address.  (Under a
-    // memory limit it goes back to the cache at once, after the work that may use it.)
     std::vector<Scratch> retired;
-    double* scratch(Scratch& s, long long doubles)
+    // between the planning of a build and the queueing of its launches: make_room takes nothing
+    bool scratch_in_use = false;
+    struct ScratchUse
+    {
+        qcg_handle* h;
+        explicit ScratchUse(qcg_handle* h_) : h(h_) { h->scratch_in_use = true; }
+        ~ScratchUse() { h->scratch_in_use = false; }
+    };
+    bool capturing()
+    {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) cudaGetLastError();
+        return st != cudaStreamCaptureStatusNone;
+    }
+    // At least `doubles` in s, for work queued on the handle's stream from now on.  A buffer that has to grow stays with
+    // the handle, because work in flight may use it; under a memory limit it goes back to the cache after that work,
+    // unless a captured graph holds its address.  need: the call cannot do without, so that other scratch makes room.
+    double* scratch(Scratch& s, long long doubles, bool need)
     {
         const size_t bytes = (size_t)doubles * sizeof(double);
-        if (bytes <= s.cap) return (double*)s.p;
-        if (s.p)
+        const bool cap = capturing();
+        if (bytes > s.cap)
         {
-            if (&s == &jk_scr) drop_graphs();
-            if (mem_limit > 0)
+            if (s.p)
             {
-                CK(cudaStreamSynchronize(stream));
-                give_scratch(s, true);
+                if (&s == &jk_scr) drop_graphs();
+                if (mem_limit > 0 && !s.captured && !cap)
+                {
+                    CK(cudaStreamSynchronize(stream));
+                    give_scratch(s, true);
+                }
+                else
+                {
+                    retired.push_back(s);
+                    s = Scratch{};
+                }
             }
-            else
-            {
-                retired.push_back(s);
-                s = Scratch{};
-            }
+            if (mem_limit > 0 && mem_used + (long long)bytes > mem_limit && !(need && make_room(bytes, &s == &jk_scr)))
+                throw Error{QCG_ERR_ALLOC, "device memory limit of " + std::to_string(mem_limit) + " bytes exceeded"};
+            const size_t budget = mem_limit > 0 ? (size_t)(mem_limit - mem_used) : ~(size_t)0;
+            s.p = ResourceCache::get().scratch(device, bytes, budget, &s.cap);
+            mem_used += (long long)s.cap;
         }
-        if (mem_limit > 0 && mem_used + (long long)bytes > mem_limit)
-            throw Error{QCG_ERR_ALLOC, "device memory limit of " + std::to_string(mem_limit) + " bytes exceeded"};
-        s.p = ResourceCache::get().scratch(device, bytes, &s.cap);
-        s.counted = (long long)bytes;
-        mem_used += s.counted;
+        s.captured |= cap;
         return (double*)s.p;
     }
     void give_scratch(Scratch& s, bool healthy)
     {
         if (!s.p) return;
-        mem_used -= s.counted;
+        mem_used -= (long long)s.cap;
         if (healthy) ResourceCache::get().give_scratch(device, s.p, s.cap);
         else cudaFree(s.p);
         s = Scratch{};
+    }
+    // Under the memory limit, room for `bytes` that a call cannot do without: the scratch, and the lists of the
+    // contracted J/K form unless keep_lists, go back where that is enough.  Later calls take the scratch again or run in
+    // another form.
+    bool make_room(size_t bytes, bool keep_lists = false)
+    {
+        if (scratch_in_use || capturing()) return false;
+        keep_lists |= jk_scr.captured;
+        long long have = 0;
+        for (const Scratch* s : {&team_scr, &jk_scr})
+            if (!s->captured) have += (long long)s->cap;
+        for (const Scratch& r : retired)
+            if (!r.captured) have += (long long)r.cap;
+        if (!keep_lists)
+            for (const JKTeamListDev& l : team_list)
+                for (const void* p : {(const void*)l.offs, (const void*)l.entry, (const void*)l.kets})
+                    have += bytes_of(p);
+        if (mem_used - have + (long long)bytes > mem_limit) return false;
+        CK(cudaStreamSynchronize(stream));
+        drop_graphs();
+        if (!keep_lists)
+            for (int k = 0; k < kNumQuartetClasses; ++k)
+                if (team_list[k].n)
+                {
+                    drop_team_list(k);
+                    team_list_state[k] = ListState::refused;
+                }
+        if (!team_scr.captured) give_scratch(team_scr, true);
+        if (!jk_scr.captured) give_scratch(jk_scr, true);
+        for (size_t i = 0; i < retired.size();)
+            if (retired[i].captured) ++i;
+            else
+            {
+                give_scratch(retired[i], true);
+                retired.erase(retired.begin() + i);
+            }
+        return true;
     }
     int* d_team_err = nullptr;
     TeamShape team_shapes[kNumQuartetClasses]{};
@@ -560,7 +616,7 @@ struct qcg_handle
     T* alloc(size_t count)
     {
         const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
-        if (mem_limit > 0 && mem_used + (long long)bytes > mem_limit)
+        if (mem_limit > 0 && mem_used + (long long)bytes > mem_limit && !make_room(bytes))
             throw Error{QCG_ERR_ALLOC, "device memory limit of " + std::to_string(mem_limit) + " bytes exceeded"};
         void* p = nullptr;
         if (bytes <= kSmallMax)
@@ -590,6 +646,14 @@ struct qcg_handle
         }
         mem_used += bytes;
         return (T*)p;
+    }
+    long long bytes_of(const void* p) const
+    {
+        const auto it = small_live.find(const_cast<void*>(p));
+        if (it != small_live.end()) return (long long)it->second;
+        for (const DevBuf& a : allocs)
+            if (a.p == p) return (long long)a.bytes;
+        return 0;
     }
     void release(void* p)
     {
@@ -2380,6 +2444,7 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
             fresh[k] = h->team_list_state[k] != qcg_handle::ListState::ready;
             try
             {
+                qcg_handle::ScratchUse use(h);   // a list makes no room for itself
                 plan.scr[k].list = jk_team_list(h, k, sh.grid);
             }
             catch (const Error& e)
@@ -2406,15 +2471,30 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
     }
     if (most == 0) return;
     plan.side = all * (long long)sizeof(double) <= kJKTeamSideMax;
-    const long long total = plan.side ? all : most;
     double* p = nullptr;
-    try
+    const auto allocate = [&](long long doubles) {
+        try
+        {
+            p = h->scratch(h->jk_scr, doubles, required);
+        }
+        catch (const Error& e)
+        {
+            if (e.code != QCG_ERR_ALLOC) throw;
+        }
+        return p != nullptr;
+    };
+    if (!allocate(plan.side ? all : most))
     {
-        p = h->scratch(h->jk_scr, total);
+        if (plan.side)
+        {
+            plan.side = false;   // one class's worth, shared
+            allocate(most);
+        }
     }
-    catch (const Error& e)
+    if (!p)
     {
-        if (required || e.code != QCG_ERR_ALLOC) throw;
+        if (required)
+            throw Error{QCG_ERR_ALLOC, "no room for the scratch of the team form"};
         for (int k = 0; k < kNumQuartetClasses; ++k) refuse_list(k);
         plan = JKTeamPlan{};
         return;
@@ -2498,10 +2578,9 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
                                                      : jk_mask | (unsigned)(QCG_JK_TEAM_CONTRACTED_MASK);
         team_want[k] = (mask >> k) & 1u;
     }
-    JKTeamPlan team;
-    jk_team_plan(h, team_want, jk_forced, team);
     // classes in the warp-shared form (FP64 band, one rank, not deterministic; the team form comes first);
-    // their work items are built here, before any capture.  The build's default applies to full builds of
+    // their work items are built here, before any capture, and before the team form's scratch where they are needed
+    // in any case.  The build's default applies to full builds of
     // uncontracted classes with at least kJKWarpMinQuartets quartets: under density screening a warp evaluates every
     // quartet that one of its lanes needs, where the thread-per-quartet form skips each one alone, and of a
     // contracted basis its few items of 256 kets run serial primitive loops (eight waters, 296 functions: (dp|ss)
@@ -2511,8 +2590,8 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     const unsigned warp_mask =
         warp_forced ? (unsigned)h->jk_warp_mask : jk_warp_mask_default(&warp_forced);
     bool warp_k[kNumQuartetClasses] = {};
-    for (int k = 0; k < kNumQuartetClasses; ++k)
-        if (((warp_mask >> k) & 1u) && !team.on[k] && h->work[k].total > 0 && h->shard_world == 1 &&
+    const auto warp_class = [&](int k) {
+        if (((warp_mask >> k) & 1u) && h->work[k].total > 0 && h->shard_world == 1 &&
             !(flags & QCG_JK_DETERMINISTIC) &&
             (warp_forced || (dmax == nullptr && dthr <= 0.0 && !split[k] && team_kmax(h, k) == 1 &&
                              h->work[k].total >= kJKWarpMinQuartets)))
@@ -2520,6 +2599,14 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
             warp_items(h, k);
             warp_k[k] = h->nwitems[k] > 0;
         }
+    };
+    for (int k = 0; k < kNumQuartetClasses; ++k)
+        if (!team_want[k]) warp_class(k);
+    JKTeamPlan team;
+    jk_team_plan(h, team_want, jk_forced, team);
+    qcg_handle::ScratchUse use(h);
+    for (int k = 0; k < kNumQuartetClasses; ++k)
+        if (team_want[k] && !team.on[k]) warp_class(k);
     // QCG_JK_DETERMINISTIC: J' and K' as integer accumulator pairs (the low words after the nn high ones),
     // every quartet in FP64
     const bool det = (flags & QCG_JK_DETERMINISTIC) != 0;
@@ -2665,8 +2752,8 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     }
 }
 
-// grouped visiting order of a batch (returns the device permutation)
-const int* batch_order(qcg_handle* h, const int* d_quartets, long long nq, int ctas)
+// the buffers of a batch's visiting order
+void ensure_sort_buffers(qcg_handle* h, long long nq)
 {
     require(nq <= 0x7fffffffLL, "at most 2^31-1 quartets per batch");
     if (nq > h->sort_cap)
@@ -2679,6 +2766,11 @@ const int* batch_order(qcg_handle* h, const int* d_quartets, long long nq, int c
         h->regrow(h->d_order, nq);
         h->sort_cap = nq;
     }
+}
+
+// grouped visiting order of a batch (returns the device permutation)
+const int* batch_order(qcg_handle* h, const int* d_quartets, long long nq, int ctas)
+{
     launch_pattern_sort(h->bs, (const int4*)d_quartets, nq, h->d_key, h->d_hist, h->d_cursor, h->d_order, ctas,
                         h->d_plan, h->stream, h->nsm);
     CK(cudaGetLastError());
@@ -2796,6 +2888,7 @@ int qcg_basis_create_batch(const int* shell_L, const int* shell_nprim, const dou
         h->bs.alpha = h->upload(plusd(h->alpha, {0.0}));
         h->bs.coef = h->upload(plusd(h->coef, {1.0}));
         h->d_f0 = h->upload(h->f0);
+        h->d_team_err = h->upload(std::vector<int>{0});
         h->mol_off.assign(nmol + 1, 0);
         for (int m = 0; m < nmol; ++m) h->mol_off[m + 1] = h->mol_off[m] + (long long)h->mol_nbf[m] * h->mol_nbf[m];
         h->packed = h->mol_off[nmol];
@@ -2933,11 +3026,6 @@ const TeamShape& team_shape(qcg_handle* h, int k)
 // the error word of the team kernels, read by the next check_team_error
 int* team_error_word(qcg_handle* h)
 {
-    if (!h->d_team_err)
-    {
-        h->d_team_err = h->alloc<int>(1);
-        CK(cudaMemsetAsync(h->d_team_err, 0, sizeof(int), h->stream));
-    }
     h->team_pending = true;
     return h->d_team_err;
 }
@@ -2945,14 +3033,14 @@ int* team_error_word(qcg_handle* h)
 // the team form's scratch for a batch of nq quartets of class k: at most one wave of CTAs, each with stage slots for the class's
 // longest primitive loop in this basis and its recurrence blocks.  False when that exceeds kTeamScratchMax bytes;
 // the batch then runs in the thread-per-quartet form.
-bool team_scratch(qcg_handle* h, int k, long long nq, TeamScratchDev& scr, TeamShape& sh)
+bool team_scratch(qcg_handle* h, int k, long long nq, TeamScratchDev& scr, TeamShape& sh, bool required = true)
 {
     const long long kmax = team_kmax(h, k);
     sh = team_shape(h, k);
     sh.grid = (int)std::min<long long>(sh.grid, nq);   // a group has at least one quartet
     const long long need = (long long)sh.grid * (kmax * sh.slot_doubles + sh.hrr_doubles);
     if (need * (long long)sizeof(double) > kTeamScratchMax) return false;
-    scr.rcache = h->scratch(h->team_scr, need);
+    scr.rcache = h->scratch(h->team_scr, need, required);
     scr.kmax = (int)kmax;
     scr.hrr = scr.rcache + (long long)sh.grid * kmax * sh.slot_doubles;
     scr.err = team_error_word(h);
@@ -2971,7 +3059,7 @@ void raise_team_error(qcg_handle* h, int e)
 }
 void check_team_error(qcg_handle* h)
 {
-    if (!h->d_team_err || !h->team_pending) return;
+    if (!h->team_pending) return;
     int e = 0;
     CK(cudaMemcpy(&e, h->d_team_err, sizeof(int), cudaMemcpyDeviceToHost));
     raise_team_error(h, e);
@@ -2981,7 +3069,7 @@ void check_team_error(qcg_handle* h)
 void queue_team_error(qcg_handle* h, int* pinned)
 {
     *pinned = 0;
-    if (h->d_team_err && h->team_pending)
+    if (h->team_pending)
         CK(cudaMemcpyAsync(pinned, h->d_team_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
 }
 
@@ -3016,7 +3104,7 @@ bool team_scratch_optional(qcg_handle* h, int k, long long nq, TeamScratchDev& s
 {
     try
     {
-        return team_scratch(h, k, nq, scr, sh);
+        return team_scratch(h, k, nq, scr, sh, false);
     }
     catch (const Error& e)
     {
@@ -3038,6 +3126,7 @@ void eri_batch_launch(qcg_handle* h, int k, const int* dq, long long m, T* dout)
     TeamShape sh{};
     sh.nsm = h->nsm;
     const bool ss_ket = k == 0 || k == 1 || k == 3 || k == 6 || k == 10 || k == 15;
+    ensure_sort_buffers(h, m);   // before the scratch, which may be optional
     const bool team = ((mask >> k) & 1u) &&
                       (ss_ket || (f64 ? team_scratch(h, k, m, scr, sh) : team_scratch_optional(h, k, m, scr, sh)));
     const int* order = batch_order(h, dq, m, team && !ss_ket ? sh.grid : h->nsm);

@@ -103,3 +103,83 @@ def test_builds_under_a_limit_that_holds_part_of_a_list(oracle_mod):
         # the room beyond the build's own buffers is still there: a new subset mask (one byte a shell pair, 484)
         if extra >= 512:
             eng.set_pair_subset(np.ones((len(sh), len(sh)), dtype=np.uint8))
+
+
+@pytest.mark.parametrize("idle", [0, 4800])
+def test_scratch_stays_within_the_limit(idle):
+    """A batch whose scratch is just above a power of two, and one that could take a larger idle buffer: what the
+    handle holds is within its limit (beside the slabs of 8 MiB that small buffers share)."""
+    import torch
+    sh = _pool(16, 1, 4760)
+    cls, nq, limit = (2, 2, 2, 2), 120, 88 << 20
+
+    def batch(eng, n):
+        q = torch.from_numpy(W.eri_class_batch(cls, n, 16, seed=1).astype(np.int32)).cuda()
+        out = torch.empty(n, 1296, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        eng.eri_batch_device(cls, q.data_ptr(), n, out.data_ptr())
+        torch.cuda.synchronize()
+        return out.cpu().numpy()
+
+    want = batch(api.Engine(sh), nq)
+    api.lib().qcg_release_cache()
+    eng = api.Engine(sh)
+    if idle:
+        batch(api.Engine(sh), idle)   # leaves its scratch, several times larger, in the cache
+    eng.set_memory_limit(limit)
+    assert np.array_equal(batch(eng, nq), want)
+    # with the cache's idle buffers freed, what the handle's end gives back is what it held
+    api.lib().qcg_release_cache()
+    before = torch.cuda.mem_get_info()[0]
+    del eng
+    api.lib().qcg_release_cache()
+    assert torch.cuda.mem_get_info()[0] - before <= limit + (16 << 20)
+
+
+def test_optional_scratch_makes_room(oracle_mod):
+    """What fits a limit by itself still fits after calls whose fastest form keeps scratch: batches and J/K builds in
+    turn, under limits from just their own buffers up to all the scratch."""
+    sh = [x for x in _contracted(W.water()) if len(x.exps) <= 3]
+    ob = oracle_mod.OracleBasis(sh)
+    D = _density(B.nbf(sh))
+    Jr, Kr = ob.jk_direct(D)[:2]
+    s, p = ([i for i, x in enumerate(sh) if x.L == L] for L in (0, 1))
+    rng = np.random.default_rng(2)
+    nq = 20
+    q = np.stack([rng.choice(p, nq), rng.choice(s, nq), rng.choice(p, nq), rng.choice(s, nq)], axis=1).astype(np.int32)
+    ref = ob.eri_batch(q).reshape(nq, -1)
+
+    def jk(eng):
+        J, K, _ = eng.fock_jk(D)
+        assert np.abs(J - Jr).max() <= FOCK_ABS and np.abs(K - Kr).max() <= FOCK_ABS
+
+    def batch(eng):
+        got = eng.eri_batch((1, 0, 1, 0), q, fp32=True)
+        assert np.abs(got - ref).max() <= 2e-5 * max(1.0, np.abs(ref).max())
+
+    def least(call):
+        lo, hi = 1, 1 << 26
+        while hi - lo > 64:
+            mid = (lo + hi) // 2
+            eng = api.Engine(sh)
+            eng.schwarz(1e-10)
+            eng.set_memory_limit(mid)
+            try:
+                call(eng)
+                hi = mid
+            except api.QcgError as e:
+                assert e.code == api.QCG_ERR_ALLOC
+                lo = mid
+        return hi
+
+    # what the screening and each call's own buffers take (a subset mask of at most 256 bytes measures the former)
+    assert len(sh) ** 2 <= 256
+    screening = least(lambda eng: eng.set_pair_subset(np.ones((len(sh), len(sh)), dtype=np.uint8))) - 256
+    both = least(jk) + least(batch) - screening + 256
+    for order in ((jk, batch), (batch, jk)):
+        for extra in range(0, 24 << 20, 96 << 10):
+            eng = api.Engine(sh)
+            eng.schwarz(1e-10)
+            eng.set_memory_limit(both + extra)
+            for call in order + order:
+                call(eng)
