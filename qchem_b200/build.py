@@ -131,10 +131,10 @@ def _jobs():
         key = _hash(parts + core + _headers(["eri_kernels.cuh", "eri_team.cuh", "eri_ss.cuh", "jk_group.cuh", "eri_team_iface.h", "team_sync.cuh", "smem_attr.h", "batch_plan.h"])
                     + FLAGS + defs)
         jobs.append((team_src, defs, os.path.join(BUILD, f"eri_team_{k}_{key}.o")))
-    extra = {"runtime.cu": _headers(["boys_table.h", "eri_team_iface.h", "batch_plan.h"]) + [_read(os.path.join(INCLUDE, "qchem_b200.h"))],
+    extra = {"runtime.cu": _headers(["boys_table.h", "eri_team_iface.h", "batch_plan.h", "device_malloc.h"]) + [_read(os.path.join(INCLUDE, "qchem_b200.h"))],
              "registry.cu": _headers(["eri_team_iface.h", "batch_plan.h"]),
              "fock_kernels.cu": _headers(["team_sync.cuh", "batch_plan.h"]),
-             "mlp.cu": [_read(os.path.join(INCLUDE, "qchem_b200.h"))] + _headers(["smem_attr.h", "team_sync.cuh"])}
+             "mlp.cu": [_read(os.path.join(INCLUDE, "qchem_b200.h"))] + _headers(["smem_attr.h", "team_sync.cuh", "device_malloc.h"])}
     for name in ("registry.cu", "fock_kernels.cu", "runtime.cu", "mlp.cu"):
         s = os.path.join(CSRC, name)
         defs = HOST_OMP + [f"-DQCG_TEAM_DEFAULT_MASK={_team_mask():#x}u",

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "../../include/qchem_b200.h"
+#include "device_malloc.h"
 #include "smem_attr.h"
 #include "team_sync.cuh"
 
@@ -483,10 +484,10 @@ struct qcg_mlp
         free_acts();
         X.resize(L() + 1, nullptr);
         Z.resize(L(), nullptr);
-        for (int l = 0; l <= L(); ++l) MCK(cudaMalloc(&X[l], (size_t)rows * w[l] * sizeof(float)));
-        for (int l = 0; l < L(); ++l) MCK(cudaMalloc(&Z[l], (size_t)rows * w[l + 1] * sizeof(float)));
-        MCK(cudaMalloc(&d_dA, (size_t)rows * maxw() * sizeof(float)));
-        MCK(cudaMalloc(&d_dB, (size_t)rows * maxw() * sizeof(float)));
+        for (int l = 0; l <= L(); ++l) MCK(qcg::device_malloc(&X[l], (size_t)rows * w[l] * sizeof(float)));
+        for (int l = 0; l < L(); ++l) MCK(qcg::device_malloc(&Z[l], (size_t)rows * w[l + 1] * sizeof(float)));
+        MCK(qcg::device_malloc(&d_dA, (size_t)rows * maxw() * sizeof(float)));
+        MCK(qcg::device_malloc(&d_dB, (size_t)rows * maxw() * sizeof(float)));
         cap_rows = rows;
     }
     ~qcg_mlp()
@@ -574,11 +575,11 @@ int qcg_mlp_create(int nlayers, const int* widths, unsigned long long seed, qcg_
             std::uniform_real_distribution<float> U(-bound, bound);
             for (size_t k = 0; k < (size_t)m->w[l + 1] * m->w[l]; ++k) h[m->woff[l] + k] = U(rng);
         }
-        MCK(cudaMalloc(&m->d_p, off * sizeof(float)));
-        MCK(cudaMalloc(&m->d_g, off * sizeof(float)));
-        MCK(cudaMalloc(&m->d_m, off * sizeof(float)));
-        MCK(cudaMalloc(&m->d_v, off * sizeof(float)));
-        MCK(cudaMalloc(&m->d_acc, 2 * sizeof(float)));
+        MCK(qcg::device_malloc(&m->d_p, off * sizeof(float)));
+        MCK(qcg::device_malloc(&m->d_g, off * sizeof(float)));
+        MCK(qcg::device_malloc(&m->d_m, off * sizeof(float)));
+        MCK(qcg::device_malloc(&m->d_v, off * sizeof(float)));
+        MCK(qcg::device_malloc(&m->d_acc, 2 * sizeof(float)));
         MCK(cudaMemcpy(m->d_p, h.data(), off * sizeof(float), cudaMemcpyHostToDevice));
         MCK(cudaMemset(m->d_g, 0, off * sizeof(float)));
         MCK(cudaMemset(m->d_m, 0, off * sizeof(float)));

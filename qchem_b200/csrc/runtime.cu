@@ -29,6 +29,7 @@
 #include "md_core.cuh"
 #include "qcg_internal.h"
 #include "boys_table.h"
+#include "device_malloc.h"
 
 namespace qcg {
 void launch_validate(const double* D, long long total, int n, const MolLayoutDev& ml, double tol, int* flag,
@@ -131,13 +132,33 @@ public:
             }
         }
         void* p = nullptr;
-        const cudaError_t e = cudaMalloc(&p, kSlab);
-        if (e != cudaSuccess)
-        {
-            cudaGetLastError();   // reported here; the call may go on in another form
-            throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
-        }
+        const cudaError_t e = device_malloc(dev, &p, kSlab);
+        if (e != cudaSuccess) throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
         return p;
+    }
+    // cudaMalloc on the current device `dev`; the idle scratch and slabs go when the device has no room beside them.  A
+    // failure is reported here alone: a call may go on in another form, and its launch check must not see it.
+    cudaError_t device_malloc(int dev, void** p, size_t bytes)
+    {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation)
+        {
+            cudaGetLastError();
+            std::vector<void*> drop;
+            {
+                std::lock_guard<std::mutex> g(mu_);
+                auto& pd = per_[dev];
+                drop.swap(pd.slabs);
+                for (auto& kv : pd.scratch) drop.push_back(kv.second);
+                pd.scratch.clear();
+                pd.scratch_idle = 0;
+            }
+            if (drop.empty()) return e;
+            for (void* q : drop) cudaFree(q);
+            e = cudaMalloc(p, bytes);
+        }
+        if (e != cudaSuccess) cudaGetLastError();
+        return e;
     }
     char* stage()
     {
@@ -223,7 +244,6 @@ public:
         size_t pow2 = (size_t)1 << 20;
         while (pow2 < bytes) pow2 <<= 1;
         *cap = pow2 <= budget ? pow2 : bytes;
-        std::vector<void*> drop;
         {
             std::lock_guard<std::mutex> g(mu_);
             auto& pd = per_[dev];
@@ -238,31 +258,13 @@ public:
             }
         }
         void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, *cap);
-        if (e == cudaErrorMemoryAllocation)
+        cudaError_t e = device_malloc(dev, &p, *cap);
+        if (e == cudaErrorMemoryAllocation && *cap > bytes)
         {
-            cudaGetLastError();
-            {
-                std::lock_guard<std::mutex> g(mu_);
-                auto& pd = per_[dev];
-                for (auto& kv : pd.scratch) drop.push_back(kv.second);
-                pd.scratch.clear();
-                pd.scratch_idle = 0;
-            }
-            for (void* q : drop) cudaFree(q);
-            e = cudaMalloc(&p, *cap);
-            if (e == cudaErrorMemoryAllocation)
-            {
-                cudaGetLastError();
-                *cap = bytes;
-                e = cudaMalloc(&p, *cap);
-            }
+            *cap = bytes;
+            e = device_malloc(dev, &p, *cap);
         }
-        if (e != cudaSuccess)
-        {
-            cudaGetLastError();
-            throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
-        }
+        if (e != cudaSuccess) throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
         return p;
     }
     void give_scratch(int dev, void* p, size_t cap)
@@ -349,6 +351,13 @@ struct PinnedArray
 };
 
 }   // namespace
+
+cudaError_t qcg::device_malloc(void** p, size_t bytes)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e != cudaSuccess ? e : ResourceCache::get().device_malloc(dev, p, bytes);
+}
 
 // arguments that identify a J/K build for graph replay
 struct QcgGraphKey
@@ -603,12 +612,8 @@ struct qcg_handle
     void* raw_alloc(size_t bytes)
     {
         void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e != cudaSuccess)
-        {
-            cudaGetLastError();   // reported here; the call may go on in another form
-            throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
-        }
+        const cudaError_t e = ResourceCache::get().device_malloc(device, &p, bytes);
+        if (e != cudaSuccess) throw Error{QCG_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
         return p;
     }
     // mem_used counts the bytes handed out (the limit applies to those, not to slab capacity)
@@ -1453,18 +1458,18 @@ struct GpuLinalg
         if (n <= cap) return;
         for (double** p : {&dA, &dB, &dC, &dW}) { cudaFree(*p); *p = nullptr; }
         const size_t nn = (size_t)n * n;
-        CK(cudaMalloc(&dA, nn * sizeof(double)));
-        CK(cudaMalloc(&dB, nn * sizeof(double)));
-        CK(cudaMalloc(&dC, nn * sizeof(double)));
-        CK(cudaMalloc(&dW, (size_t)n * sizeof(double)));
-        if (!dInfo) CK(cudaMalloc(&dInfo, sizeof(int)));
+        CK(device_malloc(&dA, nn * sizeof(double)));
+        CK(device_malloc(&dB, nn * sizeof(double)));
+        CK(device_malloc(&dC, nn * sizeof(double)));
+        CK(device_malloc(&dW, (size_t)n * sizeof(double)));
+        if (!dInfo) CK(device_malloc(&dInfo, sizeof(int)));
         int lw = 0;
         if (cusolverDnDsyevd_bufferSize(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, dA, n, dW, &lw) !=
             CUSOLVER_STATUS_SUCCESS)
             throw Error{QCG_ERR_CUDA, "cusolverDnDsyevd_bufferSize failed"};
         cudaFree(dWork);
         dWork = nullptr;
-        CK(cudaMalloc(&dWork, (size_t)std::max(lw, 1) * sizeof(double)));
+        CK(device_malloc(&dWork, (size_t)std::max(lw, 1) * sizeof(double)));
         lwork = lw;
         cap = n;
     }
@@ -3673,7 +3678,7 @@ struct SalcWork
             cudaFree(buf[i]);
             buf[i] = nullptr;
             cap[i] = 0;
-            CK(cudaMalloc(&buf[i], n * sizeof(double)));
+            CK(device_malloc(&buf[i], n * sizeof(double)));
             cap[i] = n;
         }
         return buf[i];
@@ -4178,7 +4183,7 @@ int measure_fma_peak(int reps, double* tflops, double* ms_per_launch, Launch lau
         int dev = 0, nsm = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        CK(cudaMalloc(&out, sizeof(T)));
+        CK(device_malloc(&out, sizeof(T)));
         CK(cudaEventCreate(&a));
         CK(cudaEventCreate(&b));
         const int blocks = nsm * 8, threads = 256, iters = 2048;
@@ -4223,7 +4228,7 @@ int qcg_selftest_bounded_wait(long long polls, int arrive, int* gave_up, double*
     int rc = QCG_OK;
     try
     {
-        CK(cudaMalloc(&err, sizeof(int)));
+        CK(device_malloc(&err, sizeof(int)));
         CK(cudaMemset(err, 0, sizeof(int)));
         CK(cudaEventCreate(&a));
         CK(cudaEventCreate(&b));

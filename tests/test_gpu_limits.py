@@ -183,3 +183,39 @@ def test_optional_scratch_makes_room(oracle_mod):
             eng.set_memory_limit(both + extra)
             for call in order + order:
                 call(eng)
+
+
+def test_idle_scratch_gives_way_to_other_allocations():
+    """With the device full but for less than the next call needs, the idle scratch of an earlier handle goes: a batch
+    with large host buffers and a network's activations both find room."""
+    import torch
+    sh = [B.Shell(2, (0.1 * i, 0.0, 0.3 * i), [0.3, 1.1, 4.0], [0.3, 0.5, 0.4]) for i in range(8)]
+    q = np.random.default_rng(0).integers(0, 8, size=(60000, 4)).astype(np.int32)   # 622 MB of integrals
+    want = api.Engine(sh).eri_batch((2, 2, 2, 2), q)   # the same batch: a smaller one may split its primitive loops
+    rows = 50000
+    x, y = torch.randn(rows, 29, device="cuda"), torch.empty(rows, 1225, device="cuda")
+    net = api.Mlp([29, 64, 1225])
+    net.forward(64, x.data_ptr(), y.data_ptr())
+    torch.cuda.synchronize()
+
+    def fill():
+        """idle scratch of 512 MiB and more, and the rest of the device taken but for about 400 MiB"""
+        eng = api.Engine(sh)
+        eng.eri_batch((2, 2, 2, 2), q[:20000])
+        del eng
+        torch.cuda.synchronize()
+        return torch.empty(torch.cuda.mem_get_info()[0] - (400 << 20), dtype=torch.uint8, device="cuda")
+
+    full = fill()
+    net.forward(rows, x.data_ptr(), y.data_ptr())   # four arrays of 245 MB
+    torch.cuda.synchronize()
+    del full, net
+    torch.cuda.empty_cache()
+    assert torch.isfinite(y).all().item()
+    eng = api.Engine(sh)
+    eng.eri_batch((2, 2, 2, 2), q[:20000])   # keeps its scratch, and buffers of 207 MB that the next call outgrows
+    full = fill()
+    got = eng.eri_batch((2, 2, 2, 2), q)
+    assert np.array_equal(got, want)
+    del full
+    torch.cuda.empty_cache()
