@@ -506,8 +506,10 @@ struct qcg_handle
             if (mem_limit > 0 && mem_used + (long long)bytes > mem_limit && !(need && make_room(bytes, &s == &jk_scr)))
                 throw Error{QCG_ERR_ALLOC, "device memory limit of " + std::to_string(mem_limit) + " bytes exceeded"};
             const size_t budget = mem_limit > 0 ? (size_t)(mem_limit - mem_used) : ~(size_t)0;
-            s.p = ResourceCache::get().scratch(device, bytes, budget, &s.cap);
-            mem_used += (long long)s.cap;
+            size_t got = 0;   // s stays empty where there is no room
+            s.p = ResourceCache::get().scratch(device, bytes, budget, &got);
+            s.cap = got;
+            mem_used += (long long)got;
         }
         s.captured |= cap;
         return (double*)s.p;

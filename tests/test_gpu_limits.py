@@ -219,3 +219,58 @@ def test_idle_scratch_gives_way_to_other_allocations():
     assert np.array_equal(got, want)
     del full
     torch.cuda.empty_cache()
+
+
+def _fill_device():
+    """every piece of device memory down to 2 MiB; the tensors that hold it"""
+    import torch
+    api.lib().qcg_release_cache()
+    torch.cuda.empty_cache()
+    full, size = [], torch.cuda.mem_get_info()[0]
+    while size >= 2 << 20:
+        try:
+            full.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            size //= 2
+    return full
+
+
+def test_calls_after_scratch_found_no_room(oracle_mod):
+    """A float batch and a J/K build on a full device, more than once, run in forms without scratch, a double batch is
+    refused each time; with room again all of them are right."""
+    import torch
+    sh = B.even_tempered(W.water_cluster(nx=2, ny=1, nz=1, seed=W.SEED0 + 3740))
+    ob = oracle_mod.OracleBasis(sh)
+    D = _density(B.nbf(sh))
+    Jr, Kr = ob.jk_direct(D)[:2]
+    d = [i for i, x in enumerate(sh) if x.L == 2]
+    q = np.random.default_rng(0).choice(d, size=(400, 4)).astype(np.int32)
+    ref = ob.eri_batch(q).reshape(400, -1)
+    eng = api.Engine(sh)
+    eng.schwarz(1e-10)
+
+    def float_batch():
+        assert np.abs(eng.eri_batch((2, 2, 2, 2), q, fp32=True) - ref).max() <= 2e-5 * max(1.0, np.abs(ref).max())
+
+    def build():
+        J, K, _ = eng.fock_jk(D)
+        assert np.abs(J - Jr).max() <= FOCK_ABS and np.abs(K - Kr).max() <= FOCK_ABS
+
+    # the calls' own buffers, and the code of the forms without scratch; host buffers of the double batch too
+    eng.eri_batch((2, 2, 0, 0), np.repeat(np.array([[d[0], d[0], 0, 0]], dtype=np.int32), 15000, axis=0))
+    small = api.Engine(sh)
+    small.schwarz(1e-10)
+    small.set_memory_limit(6 << 20)
+    small.fock_jk(D)
+    small.eri_batch((2, 2, 2, 2), q[:100], fp32=True)
+    full = _fill_device()
+    for _ in range(3):
+        float_batch()
+        build()
+        _refused(lambda: eng.eri_batch((2, 2, 2, 2), q))
+    del full
+    torch.cuda.empty_cache()
+    for _ in range(2):
+        float_batch()
+        build()
+        assert np.abs(eng.eri_batch((2, 2, 2, 2), q) - ref).max() <= ERI_ABS * max(1.0, np.abs(ref).max())
