@@ -48,9 +48,10 @@ enum qcg_status {
 #define QCG_JK_J_ONLY 2            /* reserved: both J and K are always built */
 #define QCG_JK_FP32 4              /* evaluate every quartet in FP32 (accumulation into J and K stays FP64) */
 /* accumulate J and K as exact 64-bit integer pairs (units of 2^-30 and 2^-70) instead of FP64 atomics, each
- * quartet's contribution rounded alone: the result is the same bit for bit from build to build, whatever order
- * the GPU's atomic updates take and whatever launch shapes the autotuner chose (for a given basis and shard);
- * each contribution is represented to 2^-71, and |J|, |K| must stay below 2^32.  Not recorded as a CUDA graph. */
+ * quartet's contribution rounded alone, in fixed pieces: the result is the same bit for bit from build to build,
+ * whatever order the GPU's atomic updates take, whatever launch shapes the autotuner chose and whatever memory is free
+ * (for a given basis, shard and set of kernel-form masks, with or without a memory limit; where the default forms find
+ * no memory the build returns QCG_ERR_ALLOC, and under a limit it takes forms without scratch); each contribution is represented to 2^-71, and |J|, |K| must stay below 2^32.  Not recorded as a CUDA graph. */
 #define QCG_JK_DETERMINISTIC 8
 
 typedef struct qcg_stats {

@@ -410,8 +410,9 @@ __global__ void __launch_bounds__(Cls::kJKWarps * 32, Cls::kJKBlocks)
                          team_pair(load_pp(P, ket.ppo[j])), bt, true);
     };
 
-    // a digestion task is a group, or with fewer groups than warps a part of its rows
-    const int parts = min(NCc, max(1, Cls::kJKWarps / ngrp)), rows = (NCc + parts - 1) / parts;
+    // a digestion task is a group, or with fewer groups than warps a part of its rows; in the deterministic mode, which
+    // rounds a task's K'(a d), K'(b d) and J'(a b), the parts are those of a full round whatever its groups
+    const int parts = min(NCc, max(1, Cls::kJKWarps / (DET ? NGRP : ngrp))), rows = (NCc + parts - 1) / parts;
     for (long long r = blockIdx.x; r < nround; r += gridDim.x)
     {
         for (int s = threadIdx.x >> 5; s < ngrp; s += Cls::kJKWarps) make(r, s);

@@ -426,18 +426,23 @@ struct qcg_handle
     int4* d_witems[kNumQuartetClasses] = {};
     long long nwitems[kNumQuartetClasses] = {};
     bool witems_ready[kNumQuartetClasses] = {};
-    // the contracted team form's order of each class (jk_team_list), built on first use after each screening; one that
-    // could not be had is not tried again until the next screening or another memory limit
+    // the contracted team form's order of each class (jk_team_list), for the default build and for the deterministic
+    // one, built on first use after each screening; one that could not be had is not tried again until the next
+    // screening or another memory limit
     enum class ListState { none, ready, refused };
-    JKTeamListDev team_list[kNumQuartetClasses] = {};
-    ListState team_list_state[kNumQuartetClasses] = {};
-    void drop_team_list(int k)
+    struct TeamList
     {
-        for (const void* p : {(const void*)team_list[k].offs, (const void*)team_list[k].entry,
-                              (const void*)team_list[k].kets})
+        JKTeamListDev dev{};
+        int kmax = 1;   // its longest loop
+        ListState state = ListState::none;
+    };
+    TeamList team_list[2][kNumQuartetClasses];
+    void drop_team_list(TeamList& l, ListState state)
+    {
+        for (const void* p : {(const void*)l.dev.offs, (const void*)l.dev.entry, (const void*)l.dev.kets})
             if (p) release((void*)p);
-        team_list[k] = JKTeamListDev{};
-        team_list_state[k] = ListState::none;
+        l = TeamList{};
+        l.state = state;
     }
     long long jk_warp_mask = -1;   // qcg_set_jk_warp_classes; -1: the process default
     double fp32_below = 0;   // qcg_set_fp32_bound: quartets with a smaller bound are evaluated in FP32
@@ -535,19 +540,17 @@ struct qcg_handle
         for (const Scratch& r : retired)
             if (!r.captured) have += (long long)r.cap;
         if (!keep_lists)
-            for (const JKTeamListDev& l : team_list)
-                for (const void* p : {(const void*)l.offs, (const void*)l.entry, (const void*)l.kets})
-                    have += bytes_of(p);
+            for (const auto& lists : team_list)
+                for (const TeamList& l : lists)
+                    for (const void* p : {(const void*)l.dev.offs, (const void*)l.dev.entry, (const void*)l.dev.kets})
+                        have += bytes_of(p);
         if (mem_used - have + (long long)bytes > mem_limit) return false;
         CK(cudaStreamSynchronize(stream));
         drop_graphs();
         if (!keep_lists)
-            for (int k = 0; k < kNumQuartetClasses; ++k)
-                if (team_list[k].n)
-                {
-                    drop_team_list(k);
-                    team_list_state[k] = ListState::refused;
-                }
+            for (auto& lists : team_list)
+                for (TeamList& l : lists)
+                    if (l.dev.n) drop_team_list(l, ListState::refused);
         if (!team_scr.captured) give_scratch(team_scr, true);
         if (!jk_scr.captured) give_scratch(jk_scr, true);
         for (size_t i = 0; i < retired.size();)
@@ -2311,6 +2314,9 @@ const TeamShape& team_shape(qcg_handle* h, int k);
 int* team_error_word(qcg_handle* h);
 // most scratch of one class in the team form
 constexpr long long kTeamScratchMax = 4LL << 30;
+// fewest CTAs for which a contracted class takes the team form: where the scratch does not go round for a whole wave,
+// as many CTAs run as it does
+constexpr long long kTeamMinCTAs = 64;
 // smallest quartet count of a class for the warp-shared form by default
 constexpr long long kJKWarpMinQuartets = 1LL << 20;
 // Classes from this many quartets on take the first side stream, one after another: each fills the GPU for
@@ -2318,7 +2324,10 @@ constexpr long long kJKWarpMinQuartets = 1LL << 20;
 // spread over the streams, 396 ms so; 456 functions: 40.5, 37.7).  Smaller ones fill each other's gaps (228
 // functions: 4.1 ms spread, 6.0 with the classes of 2^20 quartets alone).
 constexpr long long kJKAloneQuartets = 1LL << 24;
-// most scratch that lets the team classes of one build run side by side (they share one class's worth beyond it)
+// The team classes of one build run side by side, each with its own scratch, while the stages of their CTAs' whole
+// primitive loops (not cut into runs) come to no more than this; beyond it a class fills the GPU long enough, and they
+// share one class's worth and run one after another (a basis with contractions of six: four waters 1.10 ms side by
+// side, 0.96 so; eight 6.9 and 5.6; one water 0.65 side by side).
 constexpr long long kJKTeamSideMax = 2LL << 30;
 
 // The classes of a J/K build that run in the team form, their launch shapes and scratch.  side: every class has its
@@ -2335,14 +2344,18 @@ struct JKTeamPlan
 // kets come by their bounds, contraction lengths mixed, and a group of 32 runs its longest primitive loop for all
 // lanes.  Here the kets of a pair class are also listed by primitive-pair count (bounds descending within one), so
 // that a bra pair's screened kets are a run of each count's list; the runs are taken longest loop first.  A loop
-// longer than a CTA's average share of all loops (at least kTeamChain) is cut into runs of bra primitive pairs.
+// longer than a CTA's average share of all loops (at least kTeamChain) is cut into runs of bra primitive pairs -- in
+// the deterministic mode, where each run's contribution is rounded alone, one longer than kTeamChainDet, so that the
+// rounding depends on the quartet only (contractions of three stay whole).  Nor does a run need more stage slots than
+// `slots`, what the scratch has for each of `ctas` CTAs, unless a single bra primitive pair does.
 // Built once per screening, before any capture.  Split-valence basis: one water 416 -> 254 us, four 5.2 -> 3.3 ms,
 // eight 51.8 -> 41.3 ms.
-constexpr int kTeamChain = 9;
-const JKTeamListDev& jk_team_list(qcg_handle* h, int k, int ctas)
+constexpr int kTeamChain = 9, kTeamChainDet = 81;
+const qcg_handle::TeamList& jk_team_list(qcg_handle* h, int k, int ctas, long long slots, bool det)
 {
-    JKTeamListDev& list = h->team_list[k];
-    if (h->team_list_state[k] == qcg_handle::ListState::ready) return list;
+    qcg_handle::TeamList& tl = h->team_list[det][k];
+    JKTeamListDev& list = tl.dev;
+    if (tl.state == qcg_handle::ListState::ready) return tl;
     int X = 0;
     while ((X + 1) * (X + 2) / 2 <= k) ++X;
     const int Y = k - X * (X + 1) / 2;
@@ -2372,7 +2385,7 @@ const JKTeamListDev& jk_team_list(qcg_handle* h, int k, int ctas)
         j0 = j1;
     }
     const long long share = h->wh_cum[k].empty() ? 0 : h->wh_cum[k].back() / (32LL * ctas);
-    const long long most = std::max<long long>(share, kTeamChain);
+    const long long most = det ? kTeamChainDet : std::max<long long>(std::min(share, slots), kTeamChain);
     struct Run
     {
         long long loop, cnt;
@@ -2414,70 +2427,82 @@ const JKTeamListDev& jk_team_list(qcg_handle* h, int k, int ctas)
         }
         catch (...)
         {
-            h->drop_team_list(k);
+            h->drop_team_list(tl, qcg_handle::ListState::none);
             throw;
         }
         list.total = at.back();
         list.n = (int)runs.size();
+        tl.kmax = (int)runs.front().loop;
     }
-    h->team_list_state[k] = qcg_handle::ListState::ready;
-    return list;
+    tl.state = qcg_handle::ListState::ready;
+    return tl;
 }
 
-// want[k]: class k in the team form if its scratch can be had; required: the caller named the classes, so that a
-// failed allocation is an error rather than a reason for another form.
-void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool required, JKTeamPlan& plan)
+// want[k]: class k in the team form if its scratch can be had; required: the classes are the caller's choice, or the
+// build's in the deterministic mode, so that a failed allocation is an error rather than a reason for another form.
+void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool required, bool det, JKTeamPlan& plan)
 {
-    long long need[kNumQuartetClasses] = {}, all = 0, most = 0;
+    qcg_handle::TeamList* const lists = h->team_list[det];
+    long long need[kNumQuartetClasses] = {}, all = 0, most = 0, whole = 0;
     bool fresh[kNumQuartetClasses] = {};   // the lists that this call made
     // a list without its scratch serves nothing (one of an earlier build stays: a captured graph may read it)
     auto refuse_list = [&](int k) {
         plan.scr[k].list = JKTeamListDev{};
-        if (!fresh[k]) return;
-        h->drop_team_list(k);
-        h->team_list_state[k] = qcg_handle::ListState::refused;
+        if (fresh[k]) h->drop_team_list(lists[k], qcg_handle::ListState::refused);
     };
     for (int k = 0; k < kNumQuartetClasses; ++k)
     {
         if (!want[k]) continue;
         long long gb = 0, ge = 0;
         shard_range(h, k, gb, ge);
-        const int kmax = team_kmax(h, k);
+        int kmax = team_kmax(h, k);
         TeamShape& sh = plan.sh[k];
         sh = team_shape(h, k);
+        const auto cta_bytes = [&](long long slots) { return (slots * sh.slot_doubles + sh.jk_doubles) * (long long)sizeof(double); };
         if (kmax > 1 && h->shard_world == 1)
         {
-            if (!required && h->team_list_state[k] == qcg_handle::ListState::refused) continue;
-            fresh[k] = h->team_list_state[k] != qcg_handle::ListState::ready;
+            if (!required && lists[k].state == qcg_handle::ListState::refused) continue;
+            fresh[k] = lists[k].state != qcg_handle::ListState::ready;
             try
             {
                 qcg_handle::ScratchUse use(h);   // a list makes no room for itself
-                plan.scr[k].list = jk_team_list(h, k, sh.grid);
+                const long long slots = (kTeamScratchMax / sh.grid - cta_bytes(0)) / (cta_bytes(1) - cta_bytes(0));
+                const qcg_handle::TeamList& list = jk_team_list(h, k, sh.grid, slots, det);
+                plan.scr[k].list = list.dev;
+                if (list.dev.n) kmax = std::max(2, list.kmax);   // 1 stands for jk_group_kernel
             }
             catch (const Error& e)
             {
                 if (required || e.code != QCG_ERR_ALLOC) throw;
-                h->team_list_state[k] = qcg_handle::ListState::refused;
+                lists[k].state = qcg_handle::ListState::refused;
                 continue;
             }
         }
         const long long ngroups = ((plan.scr[k].list.n ? plan.scr[k].list.total : ge - gb) + 31) / 32;
-        sh.grid = (int)std::min<long long>(sh.grid, ngroups);
-        sh.group_grid = (int)std::min<long long>(sh.group_grid, ngroups);
-        need[k] = kmax == 1 ? std::min<long long>(ngroups, sh.group_grid * (sh.group_doubles / sh.jk_doubles)) * sh.jk_doubles
-                            : sh.grid * (kmax * sh.slot_doubles + sh.jk_doubles);
-        if (need[k] * (long long)sizeof(double) > kTeamScratchMax)
+        const bool groups = team_kmax(h, k) == 1;   // jk_group_kernel
+        if (!groups)
         {
-            refuse_list(k);
-            continue;
+            const long long ctas = kTeamScratchMax / cta_bytes(kmax);
+            if (ctas < std::min(kTeamMinCTAs, ngroups))
+            {
+                refuse_list(k);
+                continue;
+            }
+            const long long loops = std::min<long long>(sh.grid, ngroups) * cta_bytes(team_kmax(h, k));
+            if (loops <= kTeamScratchMax) whole += loops;
+            sh.grid = (int)std::min({(long long)sh.grid, ngroups, ctas});
         }
+        sh.group_grid = (int)std::min<long long>(sh.group_grid, ngroups);
+        need[k] = groups ? std::min<long long>(ngroups, sh.group_grid * (sh.group_doubles / sh.jk_doubles)) * sh.jk_doubles
+                            : sh.grid * (kmax * sh.slot_doubles + sh.jk_doubles);
         plan.on[k] = true;
         plan.scr[k].kmax = kmax;
+        if (groups) whole += need[k] * (long long)sizeof(double);
         all += need[k];
         most = std::max(most, need[k]);
     }
     if (most == 0) return;
-    plan.side = all * (long long)sizeof(double) <= kJKTeamSideMax;
+    plan.side = whole <= kJKTeamSideMax;
     double* p = nullptr;
     const auto allocate = [&](long long doubles) {
         try
@@ -2572,6 +2597,10 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     // whether the class is contracted in this basis (build.py has the two sets), not on the size: the uncontracted
     // set was faster from one water (197 -> 166 us) to sixteen (660 -> 528 ms), the contracted one likewise
     // (1.7 -> 0.42 ms, and 204 -> 57 ms for eight).
+    // QCG_JK_DETERMINISTIC: J' and K' as integer accumulator pairs (the low words after the nn high ones),
+    // every quartet in FP64
+    const bool det = (flags & QCG_JK_DETERMINISTIC) != 0;
+    require(!det || fp32_below <= 0, "the deterministic J/K build evaluates every quartet in FP64 (no FP32 band)");
     bool jk_forced = h->jk_team_mask >= 0;
     const unsigned jk_mask = jk_forced ? (unsigned)h->jk_team_mask : jk_team_mask_default(&jk_forced);
     bool team_want[kNumQuartetClasses] = {};
@@ -2583,7 +2612,8 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
         const unsigned mask = jk_forced                 ? jk_mask
                               : team_kmax(h, k) == 1 ? jk_mask | (unsigned)(QCG_JK_TEAM_PLAIN_MASK)
                                                      : jk_mask | (unsigned)(QCG_JK_TEAM_CONTRACTED_MASK);
-        team_want[k] = (mask >> k) & 1u;
+        // deterministic: the form must not depend on what memory is free, so that under a limit it is one without scratch
+        team_want[k] = ((mask >> k) & 1u) && (jk_forced || !det || h->mem_limit == 0);
     }
     // classes in the warp-shared form (FP64 band, one rank, not deterministic; the team form comes first);
     // their work items are built here, before any capture, and before the team form's scratch where they are needed
@@ -2610,14 +2640,10 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
     for (int k = 0; k < kNumQuartetClasses; ++k)
         if (!team_want[k]) warp_class(k);
     JKTeamPlan team;
-    jk_team_plan(h, team_want, jk_forced, team);
+    jk_team_plan(h, team_want, jk_forced || det, det, team);
     qcg_handle::ScratchUse use(h);
     for (int k = 0; k < kNumQuartetClasses; ++k)
         if (team_want[k] && !team.on[k]) warp_class(k);
-    // QCG_JK_DETERMINISTIC: J' and K' as integer accumulator pairs (the low words after the nn high ones),
-    // every quartet in FP64
-    const bool det = (flags & QCG_JK_DETERMINISTIC) != 0;
-    require(!det || fp32_below <= 0, "the deterministic J/K build evaluates every quartet in FP64 (no FP32 band)");
     const size_t nacc = det ? 2 * nn : nn;
     // side streams of this build: a molecule's few quartets are a dozen lone blocks per class, so every class gets a
     // stream (one water: 158 us on six streams, 139 on sixteen; contracted 235, 177); from a few hundred thousand
@@ -2944,8 +2970,9 @@ int qcg_set_memory_limit(qcg_handle* h, long long bytes)
 {
     if (!h || bytes < 0) return QCG_ERR_ARG;
     h->mem_limit = bytes;
-    for (auto& s : h->team_list_state)
-        if (s == qcg_handle::ListState::refused) s = qcg_handle::ListState::none;
+    for (auto& lists : h->team_list)
+        for (auto& l : lists)
+            if (l.state == qcg_handle::ListState::refused) l.state = qcg_handle::ListState::none;
     return QCG_OK;
 }
 
@@ -3363,7 +3390,7 @@ int qcg_schwarz(qcg_handle* h, double thresh, double* Q)
                     h->d_witems[k] = nullptr;
                     h->nwitems[k] = 0;
                     h->witems_ready[k] = false;
-                    h->drop_team_list(k);
+                    for (auto& lists : h->team_list) h->drop_team_list(lists[k], qcg_handle::ListState::none);
                 }
                 h->screened = false;
             }
