@@ -137,8 +137,17 @@ public:
         return p;
     }
     // cudaMalloc on the current device `dev`; the idle scratch and slabs go when the device has no room beside them.  A
-    // failure is reported here alone: a call may go on in another form, and its launch check must not see it.
+    // failure is reported here alone: a call may go on in another form, and its launch check must not see it.  Allowed
+    // while this thread captures a stream: the buffers stay with the handle, whose addresses a graph may hold.
     cudaError_t device_malloc(int dev, void** p, size_t bytes)
+    {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = malloc_beside_idle(dev, p, bytes);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        return e;
+    }
+    cudaError_t malloc_beside_idle(int dev, void** p, size_t bytes)
     {
         cudaError_t e = cudaMalloc(p, bytes);
         if (e == cudaErrorMemoryAllocation)
@@ -2459,7 +2468,10 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
         TeamShape& sh = plan.sh[k];
         sh = team_shape(h, k);
         const auto cta_bytes = [&](long long slots) { return (slots * sh.slot_doubles + sh.jk_doubles) * (long long)sizeof(double); };
-        if (kmax > 1 && h->shard_world == 1)
+        // a list that would be made in a caller's capture is left out: its upload would be recorded, to be replayed from
+        // a staging buffer with other contents
+        if (kmax > 1 && h->shard_world == 1 &&
+            (lists[k].state == qcg_handle::ListState::ready || !h->capturing()))
         {
             if (!required && lists[k].state == qcg_handle::ListState::refused) continue;
             fresh[k] = lists[k].state != qcg_handle::ListState::ready;
@@ -2633,6 +2645,7 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
             (warp_forced || (dmax == nullptr && dthr <= 0.0 && !split[k] && team_kmax(h, k) == 1 &&
                              h->work[k].total >= kJKWarpMinQuartets)))
         {
+            if (!h->witems_ready[k] && h->capturing()) return;   // its upload would be recorded (jk_team_plan)
             warp_items(h, k);
             warp_k[k] = h->nwitems[k] > 0;
         }
