@@ -81,8 +81,8 @@ typedef struct qcg_scf_params {
     int rebuild_every;        /* default 8 */
     int fp32_early;           /* 1: until the DIIS error first falls below fp32_switch, quartets whose density-
                                  weighted bound Q_ab Q_cd max|D| is below fp32_scale * (previous DIIS error) are
-                                 evaluated in FP32 (FP64 accumulation, FP64 Boys below T = 12), then a full FP64
-                                 rebuild; default 0 */
+                                 evaluated in FP32 (FP64 accumulation, FP64 Boys below T = 12) in the classes that
+                                 qcg_set_fp32_bound names, then a full FP64 rebuild; default 0 */
     double fp32_switch;       /* default 1e-5 */
     double fp32_scale;        /* <= 0 (default): 1e-4 / (3e-7 nbf^2), i.e. the worst-case FP32 error of a Fock
                                  element (nbf^2 quartets of relative error 3e-7) at 1e-4 of the DIIS error */
@@ -108,7 +108,8 @@ typedef struct qcg_scf_result {
     double fock_ms;           /* summed device time of the J/K builds */
     int full_builds;          /* J/K builds from the full density */
     int incremental_builds;   /* J/K builds from a density difference */
-    int fp32_builds;          /* J/K builds in which quartets below a bound were evaluated in FP32 */
+    int fp32_builds;          /* J/K builds that evaluated quartets below a bound in FP32 (those in classes of fewer
+                                 than 2^15 quartets: see qcg_set_fp32_bound) */
 } qcg_scf_result;
 
 /* ---- lifetime -------------------------------------------------------------------------------- */

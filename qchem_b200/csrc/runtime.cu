@@ -2562,9 +2562,10 @@ constexpr long long kFP32BandMaxQuartets = 1LL << 15;
 
 // fp32_below: quartets whose density-weighted bound Q_ab Q_cd max|D| (max over the six D blocks the
 // quartet digests) is below it may be evaluated in FP32 (FP64 accumulation), and are in the classes below
-// kFP32BandMaxQuartets; 0 = all FP64, HUGE_VAL = all FP32.  The weighting is what makes FP32 safe: the FP32 error of a quartet's contribution to J and K is
-// about 3e-7 of its bound.  dmax (the density maxima of dD) is computed here when the caller has none.
-void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flags, qcg_stats* stats,
+// kFP32BandMaxQuartets; 0 = all FP64, HUGE_VAL = all FP32.  The weighting is what makes FP32 safe: the FP32 error of a
+// quartet's contribution to J and K is about 3e-7 of its bound.  dmax (the density maxima of dD) is computed here when
+// the caller has none.  Returns whether any class ran an FP32 launch.
+bool jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flags, qcg_stats* stats,
                const double* dmax = nullptr, double dthr = 0.0, double fp32_below = 0.0)
 {
     require(h->screened, "qcg_schwarz must be called before qcg_fock_jk", QCG_ERR_STATE);
@@ -2796,6 +2797,7 @@ void jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
         stats->prim_quartets = h->work_prim_quartets;
         stats->flops = h->work_flops;
     }
+    return any_split || fp32_below >= HUGE_VAL;
 }
 
 // the buffers of a batch's visiting order
@@ -4006,7 +4008,7 @@ int qcg_rhf(qcg_handle* h, int natom, const double* Z, const double* R, int nele
             const bool full = !inc || inc_final || force_full || since_full >= prm.rebuild_every || exact_next;
             const double band = exact_next ? 0.0 : (fp32_phase ? fp32_scale * En_prev : prm.fp32_below);
             exact_next = false;
-            if (band > 0) ++n32;
+            bool ran32 = false;
             if (full)
             {
                 const double* Dup = D.data();
@@ -4022,15 +4024,16 @@ int qcg_rhf(qcg_handle* h, int natom, const double* Z, const double* R, int nele
                     const int e = qcg_autotune_jk(h, h->d_D, 1, nullptr, nullptr);
                     if (e != QCG_OK) throw Error{e, h->last_error};
                 }
-                jk_device(h, h->d_D, h->d_J, h->d_K, jk_flags, &st, nullptr, 0.0, band);
+                ran32 = jk_device(h, h->d_D, h->d_J, h->d_K, jk_flags, &st, nullptr, 0.0, band);
             }
             else
             {
                 for (size_t k = 0; k < nn; ++k) Dpin.p[k] = D[k] - Dprev[k];
                 CK(cudaMemcpyAsync(h->d_D, Dpin.p, nn * sizeof(double), cudaMemcpyHostToDevice, h->stream));
                 launch_block_max(h->d_D, h->d_f0, h->bs.L, h->nshell, n, d_dmax, h->stream, h->nsm);
-                jk_device(h, h->d_D, h->d_J, h->d_K, jk_flags, &st, d_dmax, prm.inc_thresh, band);
+                ran32 = jk_device(h, h->d_D, h->d_J, h->d_K, jk_flags, &st, d_dmax, prm.inc_thresh, band);
             }
+            n32 += ran32;
             const auto c1 = clk::now();
             CK(cudaMemcpyAsync(Jpin.p, h->d_J, nn * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
             CK(cudaMemcpyAsync(Kpin.p, h->d_K, nn * sizeof(double), cudaMemcpyDeviceToHost, h->stream));

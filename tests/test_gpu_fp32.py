@@ -111,3 +111,15 @@ def test_guess_density_from_a_converged_run():
     again = api.Engine(sh).rhf(mol, guess=ref["D"])
     assert again["converged"] and again["iterations"] <= 3
     assert abs(again["energy"] - ref["energy"]) <= E_TOL
+
+
+@pytest.mark.parametrize("atoms,shells,counted", [(2, 6, True), (4, 6, False)])
+def test_fp32_builds_counts_builds_with_fp32_quartets(atoms, shells, counted):
+    """An s basis has one class, of 3081 or 45150 quartets here: below 2^15 the SCF's early builds have an FP32 band, from
+    there on every quartet is FP64 and no build counts."""
+    mol = B.Molecule([1] * atoms, np.array([[0.0, 0.0, 1.6 * i] for i in range(atoms)]))
+    sh = [B.Shell(0, tuple(r), [0.12 * 2.3 ** k], [1.0], a) for a, r in enumerate(mol.R) for k in range(shells)]
+    plain = api.Engine(sh).rhf(mol)
+    early = api.Engine(sh).rhf(mol, fp32_early=True)
+    assert plain["converged"] and early["converged"] and abs(early["energy"] - plain["energy"]) <= E_TOL
+    assert (early["fp32_builds"] > 0) == counted
