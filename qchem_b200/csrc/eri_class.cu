@@ -127,6 +127,8 @@ constexpr size_t kLockSmem = (size_t)kLockThreads * Cls::kRSize * sizeof(Real);
 // lock step measured faster for every chunked class except FP64 (dd|dd), whose 169 KB per 128-thread
 // block leaves no room for a second block (ERI microbenchmark, 10^6 quartets per class); the FP32 form
 // needs half of that
+// float batches of the classes with an (ss) ket always run eri_ss_kernel
+#if QCG_PREC == 64 || !(QCG_CLASS == 0 || QCG_CLASS == 1 || QCG_CLASS == 3 || QCG_CLASS == 6 || QCG_CLASS == 10 || QCG_CLASS == 15)
 constexpr bool kUseLockstep = Cls::kChunked && (QCG_CLASS != 20 || QCG_PREC == 32);
 
 void QCG_NAME(launch_eri_batch)(const BasisDev& bs, const int4* q, const int* order, long long nq, Real* out,
@@ -159,6 +161,7 @@ void QCG_NAME(launch_eri_batch)(const BasisDev& bs, const int4* q, const int* or
         k<<<(unsigned)grid_for(nq, nsm), kThreads, kSmem, st>>>(bs, q, order, nq, out, boys);
     }
 }
+#endif
 
 namespace {
 // DET: the deterministic accumulation (JKWorkDev::det_lo, FP64 objects only)

@@ -70,11 +70,12 @@ const JKLauncher kJKLaunchers[kNumQuartetClasses] = {
     launch_jk_0,  launch_jk_1,  launch_jk_2,  launch_jk_3,  launch_jk_4,  launch_jk_5,  launch_jk_6,
     launch_jk_7,  launch_jk_8,  launch_jk_9,  launch_jk_10, launch_jk_11, launch_jk_12, launch_jk_13,
     launch_jk_14, launch_jk_15, launch_jk_16, launch_jk_17, launch_jk_18, launch_jk_19, launch_jk_20};
+// FP32 evaluation; the classes with an (ss) ket have none (eri_ss_kernel needs no scratch)
 const EriBatch32Launcher kEriBatch32Launchers[kNumQuartetClasses] = {
-    launch_eri_batch32_0,  launch_eri_batch32_1,  launch_eri_batch32_2,  launch_eri_batch32_3,  launch_eri_batch32_4,
-    launch_eri_batch32_5,  launch_eri_batch32_6,  launch_eri_batch32_7,  launch_eri_batch32_8,  launch_eri_batch32_9,
-    launch_eri_batch32_10, launch_eri_batch32_11, launch_eri_batch32_12, launch_eri_batch32_13, launch_eri_batch32_14,
-    launch_eri_batch32_15, launch_eri_batch32_16, launch_eri_batch32_17, launch_eri_batch32_18, launch_eri_batch32_19,
+    nullptr,  nullptr,  launch_eri_batch32_2,  nullptr,  launch_eri_batch32_4,
+    launch_eri_batch32_5,  nullptr,  launch_eri_batch32_7,  launch_eri_batch32_8,  launch_eri_batch32_9,
+    nullptr, launch_eri_batch32_11, launch_eri_batch32_12, launch_eri_batch32_13, launch_eri_batch32_14,
+    nullptr, launch_eri_batch32_16, launch_eri_batch32_17, launch_eri_batch32_18, launch_eri_batch32_19,
     launch_eri_batch32_20};
 const JKLauncher kJK32Launchers[kNumQuartetClasses] = {
     launch_jk32_0,  launch_jk32_1,  launch_jk32_2,  launch_jk32_3,  launch_jk32_4,  launch_jk32_5,  launch_jk32_6,

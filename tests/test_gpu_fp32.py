@@ -1,7 +1,8 @@
-"""The FP32 form of the ERI engine and of the J/K build, and the SCF schedule that uses it.
+"""Float ERI batches, the FP32 kernels that serve them without scratch, the FP32 form of the J/K build, and the SCF
+schedule that uses it.
 
-FP32 integrals are reported against the FP64 oracle and gated loosely (relative to the largest integral
-of the batch); what must hold exactly is the end result: an SCF that starts in FP32 reaches the plain
+Float batches are the FP64 integrals rounded once.  FP32 integrals are compared with the FP64 oracle loosely (relative to
+the largest integral of the batch); what must hold exactly is the end result: an SCF that starts in FP32 reaches the plain
 all-FP64 energy within 1e-8 Eh, because the build that confirms convergence is all-FP64.
 """
 import numpy as np
@@ -123,3 +124,42 @@ def test_fp32_builds_counts_builds_with_fp32_quartets(atoms, shells, counted):
     early = api.Engine(sh).rhf(mol, fp32_early=True)
     assert plain["converged"] and early["converged"] and abs(early["energy"] - plain["energy"]) <= E_TOL
     assert (early["fp32_builds"] > 0) == counted
+
+
+FP32_CLASSES = [k for k in range(21) if k not in (0, 1, 3, 6, 10, 15)]   # those with an (ss) ket need no scratch
+
+
+@pytest.mark.parametrize("k", range(21))
+def test_float_batch_is_the_fp64_value_rounded_once(k, pool_engines):
+    """The default float batch: within half a unit in the last place of a float, beside the 1e-12 bar of the FP64
+    integrals (of the larger of one and the batch's largest integral)."""
+    eng, ob = pool_engines
+    cls = W.quartet_classes()[k]
+    q = W.eri_class_batch(cls, 300, 512, seed=W.SEED0 + 4200 + k)
+    got, ref = eng.eri_batch(cls, q, fp32=True), ob.eri_batch(q).reshape(300, -1)
+    assert got.dtype == np.float32
+    assert np.all(np.abs(got.astype(np.float64) - ref) <= 1e-12 * max(1.0, np.abs(ref).max()) + 2.0 ** -24 * np.abs(ref))
+
+
+@pytest.mark.parametrize("k", FP32_CLASSES)
+def test_fp32_kernels_run_without_scratch(k, pool_engines):
+    """A handle with no room for the team form's scratch takes the FP32 kernels: within their bar of the oracle, and not
+    the rounded FP64 values (which shows that this route ran)."""
+    import torch
+    _, ob = pool_engines
+    cls = W.quartet_classes()[k]
+    nq = 1500
+    q = W.eri_class_batch(cls, nq, 512, seed=W.SEED0 + 4300 + k)
+    ref = ob.eri_batch(q).reshape(nq, -1)
+    d_q = torch.from_numpy(q.astype(np.int32)).cuda()
+    out = torch.empty(nq, ref.shape[1], dtype=torch.float32, device="cuda")
+    eng = api.Engine(W.shell_pool(512, seed=W.SEED0 + 4000))
+    ss = torch.zeros((nq, 4), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    eng.eri_batch_device((0, 0, 0, 0), ss.data_ptr(), nq, out.data_ptr(), fp32=True)   # the sort buffers
+    eng.set_memory_limit(1)
+    eng.eri_batch_device(cls, d_q.data_ptr(), nq, out.data_ptr(), fp32=True)
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    assert np.abs(got - ref).max() <= FP32_ERI_REL * np.abs(ref).max()
+    assert np.any(np.abs(got.astype(np.float64) - ref) > 1e-12 * max(1.0, np.abs(ref).max()) + 2.0 ** -24 * np.abs(ref))
