@@ -2323,9 +2323,14 @@ const TeamShape& team_shape(qcg_handle* h, int k);
 int* team_error_word(qcg_handle* h);
 // most scratch of one class in the team form
 constexpr long long kTeamScratchMax = 4LL << 30;
-// fewest CTAs for which a contracted class takes the team form: where the scratch does not go round for a whole wave,
-// as many CTAs run as it does
-constexpr long long kTeamMinCTAs = 64;
+// Whether a contracted class takes the team form on `ctas` CTAs, what its scratch has room for: where that is half a
+// wave, or a CTA for each group of 32 quartets.  (Contractions of eight, (ps|ps), whose wave is 592 CTAs, on 186: 3000
+// quartets 626 us against 4425 thread-per-quartet, 40 000 6105 against 5010.  Contractions of five, (dd|dd), 3000
+// quartets on 106 of 148: 1.8 ms against 42.7.)
+bool team_ctas_suffice(long long ctas, long long wave, long long groups)
+{
+    return ctas >= 1 && ctas >= std::min(wave / 2, groups);
+}
 // smallest quartet count of a class for the warp-shared form by default
 constexpr long long kJKWarpMinQuartets = 1LL << 20;
 // Classes from this many quartets on take the first side stream, one after another: each fills the GPU for
@@ -2495,7 +2500,7 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
         if (!groups)
         {
             const long long ctas = kTeamScratchMax / cta_bytes(kmax);
-            if (ctas < std::min(kTeamMinCTAs, ngroups))
+            if (!team_ctas_suffice(ctas, sh.grid, ngroups))
             {
                 refuse_list(k);
                 continue;
@@ -3060,9 +3065,9 @@ int team_kmax(qcg_handle* h, int k)
                 if (h->L[i] == l) mx = std::max(mx, h->nprim[i]);
             h->maxnp[l] = mx;
         }
-    int kmax = 1;
-    for (int l : Ls) kmax *= h->maxnp[l];
-    return kmax;
+    long long kmax = 1;
+    for (int l : Ls) kmax = std::min<long long>(kmax * h->maxnp[l], 0x7fffffff);
+    return (int)kmax;
 }
 
 // the team launch shape of class k (an occupancy query, made once per handle)
@@ -3079,17 +3084,18 @@ int* team_error_word(qcg_handle* h)
     return h->d_team_err;
 }
 
-// the team form's scratch for a batch of nq quartets of class k: at most one wave of CTAs, each with stage slots for the class's
-// longest primitive loop in this basis and its recurrence blocks.  False when that exceeds kTeamScratchMax bytes;
-// the batch then runs in the thread-per-quartet form.
+// the team form's scratch for a batch of nq quartets of class k: at most one wave of CTAs, each with stage slots for the
+// class's longest primitive loop in this basis and its recurrence blocks -- fewer CTAs where kTeamScratchMax bytes do
+// not go round for a wave ((dp|ps) with contractions of five, 40 000 quartets: 0.90 ms on 393 of 444 CTAs, 2.6
+// thread-per-quartet).  False where those would be too few; the batch then runs in the thread-per-quartet form.
 bool team_scratch(qcg_handle* h, int k, long long nq, TeamScratchDev& scr, TeamShape& sh, bool required = true)
 {
     const long long kmax = team_kmax(h, k);
     sh = team_shape(h, k);
-    sh.grid = (int)std::min<long long>(sh.grid, nq);   // a group has at least one quartet
-    const long long need = (long long)sh.grid * (kmax * sh.slot_doubles + sh.hrr_doubles);
-    if (need * (long long)sizeof(double) > kTeamScratchMax) return false;
-    scr.rcache = h->scratch(h->team_scr, need, required);
+    const long long per = kmax * sh.slot_doubles + sh.hrr_doubles, ctas = kTeamScratchMax / (long long)sizeof(double) / per;
+    if (!team_ctas_suffice(ctas, sh.grid, (nq + 31) / 32)) return false;
+    sh.grid = (int)std::min({(long long)sh.grid, nq, ctas});   // a group has at least one quartet
+    scr.rcache = h->scratch(h->team_scr, sh.grid * per, required);
     scr.kmax = (int)kmax;
     scr.hrr = scr.rcache + (long long)sh.grid * kmax * sh.slot_doubles;
     scr.err = team_error_word(h);

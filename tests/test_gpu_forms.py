@@ -153,3 +153,17 @@ def test_contracted_jk_shards_batch_and_memory_limit():
     tight.set_memory_limit(8 << 20)
     Jt, Kt, _ = tight.fock_jk(D)
     assert np.abs(Jt - J).max() <= FOCK_ABS and np.abs(Kt - K).max() <= FOCK_ABS
+
+
+@pytest.mark.parametrize("cls,most,nq", [((2, 1, 1, 0), 5, 3000), ((2, 2, 2, 2), 5, 220), ((1, 0, 1, 0), 8, 3000), ((2, 1, 2, 1), 6, 260)])
+def test_long_loops_on_fewer_ctas(cls, most, nq, engines):
+    """Contractions whose stage slots for a whole wave of CTAs would pass 4 GiB: as many CTAs as have room, each walking
+    more groups; and counts of a few groups, which need few CTAs."""
+    eng, ob = engines(most)
+    q = W.eri_class_batch(cls, nq, 96, seed=nq + most)
+    pick = np.random.default_rng(2).choice(nq, size=40, replace=False)
+    ref = ob.eri_batch(q[pick]).reshape(len(pick), -1)
+    for n in (nq, 63, 65):
+        got = eng.eri_batch(cls, q[:n])
+        use = pick < n
+        assert np.abs(got[pick[use]] - ref[use]).max(initial=0.0) <= ERI_ABS * max(1.0, np.abs(ref).max())
