@@ -242,10 +242,19 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         reinterpret_cast<int*>(&plan)[k] = reinterpret_cast<const int*>(scr.plan)[k];
     __syncthreads();
     const int ngroups = plan.group[256];
-    int b = 0;   // the group's bucket: groups come in increasing order
+    int b = -1;   // the group's bucket: the last one that starts no later, found by bisection (most are empty)
     for (int g = blockIdx.x; g < ngroups; g += gridDim.x)
     {
-        while (plan.group[b + 1] <= g) ++b;
+        if (b < 0 || plan.group[b + 1] <= g)
+        {
+            b = 0;
+            for (int hi = 256; hi - b > 1;)
+            {
+                const int mid = (b + hi) >> 1;
+                if (plan.group[mid] <= g) b = mid;
+                else hi = mid;
+            }
+        }
         // every warp reads the same quartets: lane l of every warp holds bra primitive pairs sub, sub + S, ... of its
         // quartet, S = 1 << lg
         const int lg = plan.lanes[b], sub = lane & ((1 << lg) - 1);

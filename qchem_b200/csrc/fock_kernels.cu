@@ -89,11 +89,14 @@ __device__ __forceinline__ int pattern_key(const BasisDev& bs, const int4 s)
 // 81 primitive quartets, a serial chain that alone outlasted the rest of a small batch) is split until it is.
 // Buckets go by decreasing loop length, so that the long loops start first and the short ones fill the last wave.
 // 32 quartets of each of 21 classes: 2.50 -> 0.95 ms; 3001 each 2.86 -> 1.93; 20 011 each 5.0 -> 4.7.
+// Every batch waits for this block: ranks by one 64-bit key, four compared per load, and sums by warp scans.  (Buckets
+// compared one by one and summed by each thread: 7-8 us a batch, 5 so.)
 __device__ int pattern_plan(const int* n, int ctas, BatchPlanDev* __restrict__ plan)
 {
-    __shared__ int w[256], rn[256], rg[256];
+    __shared__ alignas(16) int key[256];
+    __shared__ int rn[256], rg[256], before[256], wn[8], wg[8];
     __shared__ unsigned long long all;
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int kab = ((t >> 6) + 1) * (((t >> 4) & 3) + 1), kcd = (((t >> 2) & 3) + 1) * ((t & 3) + 1);
     if (t == 0) all = 0;
     __syncthreads();
@@ -103,29 +106,52 @@ __device__ int pattern_plan(const int* n, int ctas, BatchPlanDev* __restrict__ p
     const int most = max(share, kBatchChain);
     int l = 0;
     while (l < 4 && (1 << l) < kab && ((kab + (1 << l) - 1) >> l) * kcd > most) ++l;
-    w[t] = ((kab + (1 << l) - 1) >> l) * kcd;
+    // decreasing loop length, then bucket: distinct keys (loops have at most 256 primitive quartets here)
+    const int mine = (((kab + (1 << l) - 1) >> l) * kcd) << 8 | (255 - t);
+    key[t] = mine;
     __syncthreads();
     int rank = 0;
-    for (int u = 0; u < 256; ++u)
-        if (w[u] > w[t] || (w[u] == w[t] && u < t)) ++rank;
+#pragma unroll 8
+    for (int u = 0; u < 64; ++u)
+    {
+        const int4 k = reinterpret_cast<const int4*>(key)[u];
+        rank += (k.x > mine) + (k.y > mine) + (k.z > mine) + (k.w > mine);
+    }
     rn[rank] = n[t];
     rg[rank] = (int)((((long long)n[t] << l) + 31) >> 5);
-    __syncthreads();
-    int before = 0, groups = 0;
-    for (int r = 0; r < rank; ++r)
-    {
-        before += rn[r];
-        groups += rg[r];
-    }
-    plan->first[rank] = before;
-    plan->group[rank] = groups;
     plan->lanes[rank] = l;
-    if (rank == 255)
+    __syncthreads();
+    // thread t holds rank t: exclusive sums of the quartets and groups before it
+    int sn = rn[t], sg = rg[t];
+    for (int o = 1; o < 32; o <<= 1)
     {
-        plan->first[256] = before + rn[255];
-        plan->group[256] = groups + rg[255];
+        const int pn = __shfl_up_sync(0xffffffffu, sn, o), pg = __shfl_up_sync(0xffffffffu, sg, o);
+        if (lane >= o)
+        {
+            sn += pn;
+            sg += pg;
+        }
     }
-    return before;
+    if (lane == 31)
+    {
+        wn[warp] = sn;
+        wg[warp] = sg;
+    }
+    __syncthreads();
+    for (int u = 0; u < warp; ++u)
+    {
+        sn += wn[u];
+        sg += wg[u];
+    }
+    before[t] = plan->first[t] = sn - rn[t];
+    plan->group[t] = sg - rg[t];
+    if (t == 255)
+    {
+        plan->first[256] = sn;
+        plan->group[256] = sg;
+    }
+    __syncthreads();
+    return before[rank];
 }
 
 __global__ void pattern_key_kernel(BasisDev bs, const int4* __restrict__ quartets, long long nq,
