@@ -194,7 +194,7 @@ void launch_batch(const BasisDev& bs, const int4* q, const int* order, long long
     static std::atomic<unsigned long long> ready{0};
     ensure_smem(k, kSmem, ready);
     // one wave of CTAs, each walking groups of the plan; the scratch has room for sh.grid CTAs
-    k<<<(unsigned)sh.grid, kThreads, kSmem, st>>>(bs, q, order, out, boys, scr);
+    k<<<(unsigned)sh.grid, kThreads, kSmem, st>>>(bs, q, order, (int)nq, out, boys, scr);
 }
 #if QCG_SS_KET
 template <class OT, int SPLIT>

@@ -209,7 +209,7 @@ __device__ __forceinline__ bool team_contract(const double* __restrict__ rc, dou
 template <class Cls, class OT>
 __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     eri_batch_team_kernel(BasisDev bs, const int4* __restrict__ quartets, const int* __restrict__ order,
-                          OT* __restrict__ out, const double* __restrict__ boys_table, TeamScratchDev scr)
+                          const int nq, OT* __restrict__ out, const double* __restrict__ boys_table, TeamScratchDev scr)
 {
     constexpr int NW = Cls::kNW;
     constexpr int NF = Cls::kNF, NE = Cls::kNE;
@@ -238,8 +238,16 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
     TeamRing ring{full, done};
     __shared__ BatchPlanDev plan;
     __shared__ int lane_q[32];   // each lane's quartet, for the phases after the contraction; -1: none
-    for (int k = threadIdx.x; k < (int)(sizeof(BatchPlanDev) / sizeof(int)); k += blockDim.x)
-        reinterpret_cast<int*>(&plan)[k] = reinterpret_cast<const int*>(scr.plan)[k];
+    if (scr.plan)
+        for (int k = threadIdx.x; k < (int)(sizeof(BatchPlanDev) / sizeof(int)); k += blockDim.x)
+            reinterpret_cast<int*>(&plan)[k] = reinterpret_cast<const int*>(scr.plan)[k];
+    else   // an uncontracted class: one pattern, groups of 32 quartets as they come
+        for (int k = threadIdx.x; k < 257; k += blockDim.x)
+        {
+            plan.first[k] = k ? nq : 0;
+            plan.group[k] = k ? (nq + 31) >> 5 : 0;
+            if (k < 256) plan.lanes[k] = 0;
+        }
     __syncthreads();
     const int ngroups = plan.group[256];
     int b = -1;   // the group's bucket: the last one that starts no later, found by bisection (most are empty)
@@ -260,7 +268,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         const int lg = plan.lanes[b], sub = lane & ((1 << lg) - 1);
         const int gi = plan.first[b] + (g - plan.group[b]) * (32 >> lg) + (lane >> lg);
         const bool valid = gi < plan.first[b + 1];
-        const long long q = valid ? (long long)order[gi] : 0;
+        const long long q = valid ? (long long)(order ? order[gi] : gi) : 0;
         if (warp == 0) lane_q[lane] = valid && sub == 0 ? (int)q : -1;
         const int4 s = quartets[q];
         int ni = 0, nj = 0, nk = 0, nl = 0;

@@ -31,7 +31,7 @@ struct TeamScratchDev
     int kmax;
     double* hrr;
     int* err;
-    const BatchPlanDev* plan;   // ERI batches: the groups
+    const BatchPlanDev* plan;   // ERI batches: the groups; null (and no order) for an uncontracted class
     JKTeamListDev list;         // contracted J/K builds: the order of the quartets
 };
 

@@ -2808,7 +2808,6 @@ bool jk_device(qcg_handle* h, const double* dD, double* dJ, double* dK, int flag
 // the buffers of a batch's visiting order
 void ensure_sort_buffers(qcg_handle* h, long long nq)
 {
-    require(nq <= 0x7fffffffLL, "at most 2^31-1 quartets per batch");
     if (nq > h->sort_cap)
     {
         h->sort_cap = 0;
@@ -3176,16 +3175,25 @@ template <class T>
 void eri_batch_launch(qcg_handle* h, int k, const int* dq, long long m, T* dout)
 {
     constexpr bool f64 = std::is_same_v<T, double>;
+    require(m <= 0x7fffffffLL, "at most 2^31-1 quartets per batch");
     const unsigned mask = f64 ? (h->team_mask >= 0 ? (unsigned)h->team_mask : eri_team_mask()) : ~0u;
     TeamScratchDev scr{};
     TeamShape sh{};
     sh.nsm = h->nsm;
     const bool ss_ket = k == 0 || k == 1 || k == 3 || k == 6 || k == 10 || k == 15;
-    ensure_sort_buffers(h, m);   // before the scratch, which may be optional
+    // A class without contracted shells has one pattern and is not sorted: 10 000 quartets of (ps|ps) 44 -> 12 us,
+    // 250 000 of (pp|pp), whose sort waits on one counter, 570 -> 370 (490 before this form).
+    const bool plain = ((mask >> k) & 1u) && team_kmax(h, k) == 1;
+    if (!plain) ensure_sort_buffers(h, m);   // before the scratch, which may be optional
     const bool team = ((mask >> k) & 1u) &&
                       (ss_ket || (f64 ? team_scratch(h, k, m, scr, sh) : team_scratch_optional(h, k, m, scr, sh)));
-    const int* order = batch_order(h, dq, m, team && !ss_ket ? sh.grid : h->nsm);
-    scr.plan = h->d_plan;
+    const int* order = nullptr;
+    if (!plain || !team)
+    {
+        if (plain) ensure_sort_buffers(h, m);
+        order = batch_order(h, dq, m, team && !ss_ket ? sh.grid : h->nsm);
+        scr.plan = h->d_plan;
+    }
     const int4* q = (const int4*)dq;
     if constexpr (f64)
     {

@@ -167,3 +167,24 @@ def test_long_loops_on_fewer_ctas(cls, most, nq, engines):
         got = eng.eri_batch(cls, q[:n])
         use = pick < n
         assert np.abs(got[pick[use]] - ref[use]).max(initial=0.0) <= ERI_ABS * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("nq", [1, 31, 32, 33, 4097, 20001])
+@pytest.mark.parametrize("cls", [(0, 0, 0, 0), (2, 2, 0, 0), (1, 0, 1, 0), (2, 1, 1, 1), (2, 2, 2, 2)])
+def test_uncontracted_batches_are_not_sorted(cls, nq, fp32, oracle_mod, engines):
+    """Batches of classes without contracted shells run in the order they come, up to partial groups and CTAs with
+    several groups -- beside shells of another angular momentum that are contracted."""
+    rng = np.random.default_rng(11)
+    used = set(cls)
+    sh = [B.Shell(L, tuple(rng.uniform(0.0, 6.0, size=3)), list(np.exp(rng.uniform(np.log(0.05), np.log(50.0), size=k))),
+                  list(rng.uniform(0.1, 1.0, size=k)))
+          for L in range(3) for k in ([1] * 40 if L in used else [3] * 40)]
+    eng, ob = api.Engine(sh), oracle_mod.OracleBasis(sh)
+    q = W.eri_class_batch(cls, nq, 40, seed=nq)
+    pick = np.arange(nq) if nq < 100 else np.unique(np.concatenate([np.arange(40), np.arange(nq - 40, nq),
+                                                                    rng.integers(0, nq, size=120)]))
+    got, ref = eng.eri_batch(cls, q, fp32=fp32), ob.eri_batch(q[pick]).reshape(len(pick), -1)
+    assert np.all(np.isfinite(got))
+    tol = ERI_ABS * max(1.0, np.abs(ref).max()) + (2.0 ** -24 * np.abs(ref) if fp32 else 0.0)
+    assert np.all(np.abs(got[pick].astype(np.float64) - ref) <= tol)
