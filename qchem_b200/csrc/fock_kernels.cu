@@ -168,23 +168,23 @@ __global__ void pattern_key_kernel(BasisDev bs, const int4* __restrict__ quartet
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 256; i += blockDim.x)
-        if (h[i]) atomicAdd(&hist[i], h[i]);
+        if (h[i]) atomicAdd(&hist[i * kBucketStride], h[i]);
 }
 
 __global__ void pattern_scan_kernel(const int* __restrict__ hist, int* __restrict__ cursor, int ctas,
                                     BatchPlanDev* __restrict__ plan)
 {
     __shared__ int n[256];
-    n[threadIdx.x] = hist[threadIdx.x];
+    n[threadIdx.x] = hist[threadIdx.x * kBucketStride];
     __syncthreads();
-    cursor[threadIdx.x] = pattern_plan(n, ctas, plan);
+    cursor[threadIdx.x * kBucketStride] = pattern_plan(n, ctas, plan);
 }
 
 __global__ void pattern_scatter_kernel(const unsigned char* __restrict__ key, long long nq, int* __restrict__ cursor,
                                        int* __restrict__ order)
 {
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nq; q += (long long)gridDim.x * blockDim.x)
-        order[atomicAdd(&cursor[key[q]], 1)] = (int)q;
+        order[atomicAdd(&cursor[key[q] * kBucketStride], 1)] = (int)q;
 }
 
 // The three steps above by one block, for batches that one block sorts sooner than four launches start.
@@ -217,7 +217,7 @@ void launch_pattern_sort(const BasisDev& bs, const int4* quartets, long long nq,
         pattern_sort_small_kernel<<<1, 256, 0, st>>>(bs, quartets, (int)nq, order, ctas, plan);
         return;
     }
-    cudaMemsetAsync(hist, 0, 256 * sizeof(int), st);
+    cudaMemsetAsync(hist, 0, kBucketInts * sizeof(int), st);
     const long long blocks = std::min<long long>((nq + 255) / 256, (long long)nsm * 8);
     pattern_key_kernel<<<(unsigned)blocks, 256, 0, st>>>(bs, quartets, nq, key, hist);
     pattern_scan_kernel<<<1, 256, 0, st>>>(hist, cursor, ctas, plan);

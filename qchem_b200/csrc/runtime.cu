@@ -2811,8 +2811,8 @@ void ensure_sort_buffers(qcg_handle* h, long long nq)
     if (nq > h->sort_cap)
     {
         h->sort_cap = 0;
-        if (!h->d_hist) h->d_hist = h->alloc<int>(256);
-        if (!h->d_cursor) h->d_cursor = h->alloc<int>(256);
+        if (!h->d_hist) h->d_hist = h->alloc<int>(kBucketInts);
+        if (!h->d_cursor) h->d_cursor = h->alloc<int>(kBucketInts);
         if (!h->d_plan) h->d_plan = h->alloc<BatchPlanDev>(1);
         h->regrow(h->d_key, nq);
         h->regrow(h->d_order, nq);
