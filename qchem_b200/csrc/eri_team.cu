@@ -58,35 +58,38 @@ constexpr int team_pieces(int ncode, int nh, int ne)
     const int npass = (ncode + g - 1) / g;
     return (ncode + npass - 1) / npass;
 }
-// CTAs per SM to compile for: about twelve warps, as far as three stages each fit the shared memory, of which a
-// CTA may then use kSmemPerSM / m bytes less what it holds beside the stages
+// CTAs per SM to compile for: twelve warps or more, as far as the registers go round and three stages each fit the
+// shared memory, of which a CTA may then use kSmemPerSM / m bytes less what it holds beside the stages.  (Nine warps in
+// one CTA, the (pp|pp) and (ds|pp) classes, wait together between the phases of a group: 250 000 quartets of
+// contraction three 1068 and 1026 us, in two CTAs 853 and 799; of contraction two 612 and 562, 466 and 413.)
 constexpr int kSmemPerSM = 227 * 1024;
 constexpr int kSmemBeside = 2048 + (int)sizeof(BatchPlanDev) + (int)(kBoysRows * kBoysColumns * sizeof(double));
-constexpr int team_min_blocks(int ng, int stage)
+constexpr int team_min_blocks(int ng, int stage, int regs)
 {
-    const int fit = kSmemPerSM / (3 * stage * 32 * 8 + kSmemBeside), want = 12 / (3 * ng);
-    const int m = fit < want ? fit : want;
+    const int fit = kSmemPerSM / (3 * stage * 32 * 8 + kSmemBeside), want = (12 + 3 * ng - 1) / (3 * ng);
+    int m = fit < want ? fit : want;
+    while (m > 1 && warp_regs(ng * m) < regs) --m;
     return m < 1 ? 1 : m;
 }
 // stages per slot of the ring (team_contract): what three slots leave room for, eight at most
-constexpr int team_unroll(int ng, int stage)
+constexpr int team_unroll(int ng, int stage, int regs)
 {
-    const int u = (kSmemPerSM / team_min_blocks(ng, stage) - kSmemBeside) / (3 * stage * 32 * 8);
+    const int u = (kSmemPerSM / team_min_blocks(ng, stage, regs) - kSmemBeside) / (3 * stage * 32 * 8);
     return u < 1 ? 1 : (u > 8 ? 8 : u);
 }
 // Doubles of the stage space: three slots, and at least 18 primitive pairs (contractions of three) and the columns
 // of the bra recurrence that go out together.
-constexpr int team_stage_space(int ng, int stage)
+constexpr int team_stage_space(int ng, int stage, int regs)
 {
     const int ncd = ncart(kPairLA[kY]) * ncart(kPairLB[kY]), nab = ncart(kPairLA[kX]) * ncart(kPairLB[kX]);
-    const int columns = nab * (ncd < 3 * ng ? ncd : 3 * ng) * 33, slots = 3 * team_unroll(ng, stage) * stage * 32;
+    const int columns = nab * (ncd < 3 * ng ? ncd : 3 * ng) * 33, slots = 3 * team_unroll(ng, stage, regs) * stage * 32;
     int n = 18 * kTeamPairDoubles * 32;
     if (n < slots) n = slots;
     return n < columns ? columns : n;
 }
-constexpr size_t team_smem(int ng, int stage)
+constexpr size_t team_smem(int ng, int stage, int regs)
 {
-    return (size_t)(team_stage_space(ng, stage) + kBoysRows * kBoysColumns) * sizeof(double);
+    return (size_t)(team_stage_space(ng, stage, regs) + kBoysRows * kBoysColumns) * sizeof(double);
 }
 
 struct Cls
@@ -97,7 +100,8 @@ struct Cls
     static constexpr int kNCode = gen::QCG_CAT(kTeamNCode, QCG_CLASS);
     static constexpr int kKetStage = gen::QCG_CAT(kTeamKetStage, QCG_CLASS);
     static constexpr int kNG = team_pieces(kNCode, kNH, kNE), kNW = 3 * kNG;
-    static constexpr int kMinBlocks = team_min_blocks(kNG, kStage), kUnroll = team_unroll(kNG, kStage);
+    static constexpr int kRegs = 2 * (kNH + kNE) + kTemps;
+    static constexpr int kMinBlocks = team_min_blocks(kNG, kStage, kRegs), kUnroll = team_unroll(kNG, kStage, kRegs);
     // jk_group_kernel: eight warps (the digestion needs more registers than twelve leave), and up to eight groups of 32
     // quartets, one per warp, as far as their stages fit the shared memory
     static constexpr int kGroups = [] {
@@ -116,7 +120,7 @@ struct Cls
     using View = gen::QCG_CAT(TeamView, QCG_CLASS)<double>;
     static __device__ __forceinline__ constexpr int fslot(int jc) { return gen::QCG_CAT(team_fslot_, QCG_CLASS)(jc); }
     static __device__ __forceinline__ constexpr bool fixed(int jc) { return gen::QCG_CAT(team_ffixed_, QCG_CLASS)(jc); }
-    static constexpr int kStageSpace = team_stage_space(kNG, kStage), kPairSlots = kStageSpace / (32 * kTeamPairDoubles);
+    static constexpr int kStageSpace = team_stage_space(kNG, kStage, kRegs), kPairSlots = kStageSpace / (32 * kTeamPairDoubles);
     static __device__ __forceinline__ void produce(double* st, const TeamPair& ab, const TeamPair& cd,
                                                    const BoysColumns& bt, bool bra_e)
     {
@@ -158,7 +162,7 @@ struct Cls
 
 constexpr int kThreads = Cls::kNW * 32;
 constexpr int kNCD = ncart(Cls::LC) * ncart(Cls::LD);
-constexpr size_t kSmem = team_smem(Cls::kNG, Cls::kStage);   // the stages and the Boys columns
+constexpr size_t kSmem = team_smem(Cls::kNG, Cls::kStage, Cls::kRegs);   // the stages and the Boys columns
 constexpr size_t kGroupSmem =
     ((size_t)Cls::kGroups * Cls::kStage * 32 + kBoysRows * kBoysColumns) * sizeof(double);
 std::atomic<unsigned long long> g_smem_ready{0};
