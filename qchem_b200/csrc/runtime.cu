@@ -2360,11 +2360,12 @@ struct JKTeamPlan
 // that a bra pair's screened kets are a run of each count's list; the runs are taken longest loop first.  A loop
 // longer than a CTA's average share of all loops (at least kTeamChain) is cut into runs of bra primitive pairs -- in
 // the deterministic mode, where each run's contribution is rounded alone, one longer than kTeamChainDet, so that the
-// rounding depends on the quartet only (contractions of three stay whole).  Nor does a run need more stage slots than
+// rounding depends on the quartet only (split-valence basis, runs of at most 9, 18 and 81: one water 223, 247 and 290
+// us, four 5.6, 4.9 and 5.4 ms, eight 62.6, 57.8 and 56.1).  Nor does a run need more stage slots than
 // `slots`, what the scratch has for each of `ctas` CTAs, unless a single bra primitive pair does.
 // Built once per screening, before any capture.  Split-valence basis: one water 416 -> 254 us, four 5.2 -> 3.3 ms,
 // eight 51.8 -> 41.3 ms.
-constexpr int kTeamChain = 9, kTeamChainDet = 81;
+constexpr int kTeamChain = 9, kTeamChainDet = 18;
 const qcg_handle::TeamList& jk_team_list(qcg_handle* h, int k, int ctas, long long slots, bool det)
 {
     qcg_handle::TeamList& tl = h->team_list[det][k];

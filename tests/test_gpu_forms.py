@@ -40,15 +40,15 @@ def engines(oracle_mod):
     return get
 
 
+SMALL = [(0, 0, 0, 0), (2, 2, 0, 0), (1, 0, 1, 0), (2, 0, 1, 1), (2, 1, 2, 0), (2, 2, 2, 1)]
+
+
 @pytest.mark.parametrize("fp32", [False, True])
-@pytest.mark.parametrize("most", [1, 3, 5])
+@pytest.mark.parametrize("cls,most", [(c, m) for c in SMALL for m in (1, 3, 5) if m < 5 or sum(c) <= 4])
 @pytest.mark.parametrize("nq", [1, 33, 257])
-@pytest.mark.parametrize("cls", [(0, 0, 0, 0), (2, 2, 0, 0), (1, 0, 1, 0), (2, 0, 1, 1), (2, 1, 2, 0), (2, 2, 2, 1)])
 def test_small_batches(cls, nq, most, fp32, engines):
-    """every quartet of small batches, whose loops are split over lanes; contraction 5 goes beyond the pattern keys
-    (4) and, for (xx|ss), beyond the ket pairs kept in shared memory"""
-    if most == 5 and sum(cls) > 4:
-        pytest.skip("up to 625 primitive quartets: the light classes suffice")
+    """every quartet of small batches, whose loops are split over lanes; contraction 5 (up to 625 primitive quartets, in
+    the light classes) goes beyond the pattern keys (4) and, for (xx|ss), beyond the ket pairs kept in shared memory"""
     eng, ob = engines(most)
     q = W.eri_class_batch(cls, nq, 96, seed=nq + most)
     got, ref = eng.eri_batch(cls, q, fp32=fp32), ob.eri_batch(q).reshape(nq, -1)
