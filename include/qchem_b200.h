@@ -94,7 +94,8 @@ typedef struct qcg_scf_params {
     int deterministic;        /* 1: every J/K build with QCG_JK_DETERMINISTIC (exact integer accumulation), so
                                  that the trajectory, the iteration count and the energy repeat bit for bit from
                                  run to run -- near-degenerate SCFs otherwise follow the rounding of the FP64
-                                 atomics; each build costs about 1.9x; not with fp32_early or fp32_below > 0;
+                                 atomics; each build costs up to 2.4x (1.4x at 57
+                                 functions); not with fp32_early or fp32_below > 0;
                                  default 0 */
 } qcg_scf_params;
 

@@ -76,8 +76,8 @@ def _team_mask() -> int:
 
 # classes whose direct J/K build runs in the team form by default (QCG_JK_TEAM_MASK selects others at run time):
 # (dd|dd), (dd|dp), (dd|ds), (dd|pp), (dd|ps), (dp|dp).  On a B200, on the uncontracted 16-water build (912
-# functions), per class and serialised, against the thread-per-quartet kernel: (dd|dd) 1.35 vs 6.1 ms, (dd|dp) 10.8
-# vs 46, (dd|ds) 7.2 vs 22, (dd|pp) 12.6 vs 34, (dd|ps) 13.1 vs 34, (dp|dp) 26 vs 86.
+# functions), per class and serialised, against the thread-per-quartet kernel: (dd|dd) 1.6 vs 5.7 ms, (dd|dp) 9.4
+# vs 44, (dd|ds) 6.3 vs 21, (dd|pp) 10 vs 31, (dd|ps) 12.5 vs 32, (dp|dp) 20 vs 81.
 JK_TEAM_CLASSES = (14, 16, 17, 18, 19, 20)
 
 
@@ -85,11 +85,12 @@ def _jk_team_mask() -> int:
     return sum(1 << k for k in JK_TEAM_CLASSES)
 
 
-# ... and beside them, where the class is uncontracted in the basis (jk_group_kernel): (dp|pp) 54.8 ms against 110 in
-# the warp-shared form, (dp|ds) 35.9 against 77; on the classes with lighter quartets the warp-shared or
-# thread-per-quartet form is faster ((dp|ps) 39 vs 63 ms, (ps|ps) 46 vs 96).  Where it is contracted
+# ... and beside them, where the class is uncontracted in the basis (jk_group_kernel): (dp|pp) 39 ms against 105 in
+# the warp-shared form, (dp|ds) 28.5 against 74; on the classes with lighter quartets the warp-shared or
+# thread-per-quartet form is faster ((dp|ps) 36 vs 52 ms, (ps|ps) 24 vs 82).  Where it is contracted
 # (jk_team_kernel): every class whose ket pair is not (ss) -- eight waters in a split-valence basis of 296 functions
-# take 57 ms with this set, 62 with every class, 87 with the uncontracted set.  Both precede the warp-shared form.
+# take 36.5 ms with this set, 40.2 with every class, 118 with the uncontracted set, 174 without the form.  Both precede
+# the warp-shared form.
 JK_TEAM_PLAIN_CLASSES = (12, 13)
 JK_TEAM_CONTRACTED_CLASSES = (2, 4, 5, 7, 8, 9, 11, 12, 13)
 
@@ -98,12 +99,12 @@ def _mask(classes) -> int:
     return sum(1 << k for k in classes)
 
 
-# classes whose direct J/K build runs in the warp-shared form by default (QCG_JK_WARP_MASK selects others):
-# (ps|ss), (ps|ps), (pp|ss), (pp|ps), (ds|ss), (ds|ps), (ds|pp), (ds|ds), (dp|ss), (dp|ps), (dp|pp), (dp|ds).
-# Measured class by class on a B200 on the uncontracted 32-water build (half-warp sets), the warp-shared form
-# took 0.51-0.82x the thread-per-quartet kernel's time on these twelve ((ds|ps) 219 vs 428 ms, (dp|ds) 625
-# vs 872 ms, (dp|pp) 994 vs 1345 ms, where the team form took 1231 ms); on (ss|ss), (pp|pp) and (dd|ss) it
-# was level (1.00-1.02x), and those stay thread-per-quartet.
+# classes whose direct J/K build runs in the warp-shared form by default (QCG_JK_WARP_MASK selects others), in large
+# full builds of uncontracted bases: (ps|ss), (ps|ps), (pp|ss), (pp|ps), (ds|ss), (ds|ps), (ds|pp), (ds|ds), (dp|ss),
+# (dp|ps).  On the 16-water build, against the thread-per-quartet kernel: (ps|ps) 24 vs 43 ms, (ds|ps) 17.6 vs 36,
+# (dp|ps) 36 vs 50, (pp|ps) 34 vs 38, (pp|ss) 13.9 vs 14.3; (pp|pp) 18.6 vs 16.9 and (dd|ss) 3.4 vs 2.7 stay
+# thread-per-quartet, and so does (ss|ss), 6.6 vs 7.2.  (dp|pp) and (dp|ds) take it only where the scratch of
+# jk_group_kernel cannot be had: 105 vs 129 and 74 vs 84.
 JK_WARP_CLASSES = (1, 2, 3, 4, 6, 7, 8, 9, 10, 11, 12, 13)
 
 

@@ -798,6 +798,7 @@ def gen_class_team(LA, LB, LC, LD, idx):
     w("}")
     # one component at a time, Y and acc in the molecule's own frame
     w("// the ket step of component jf (slot order) and the bra step with every index in the molecule's frame")
+    # the ket and bra steps in the molecule's frame, for the host checks of the generated code (tests/host_md)
     w("template <class RT>")
     w(f"__device__ __forceinline__ void team_ket_{idx}(const int jf, const RT* __restrict__ st, RT (&Yf)[{NH}])")
     w("{")

@@ -169,8 +169,9 @@ __device__ __forceinline__ void team_digest(const JKWorkDev& w, const PairListDe
 // The digestion of jk_group_kernel: rows [ic0, ic1) of c components of this lane's quartet, every d component of each.
 // K'(a d) and K'(b d) stay in registers over the rows (kWholeRows: where they fit) and leave once per call, K'(a c)
 // and K'(b c) once per row: (dp|pp) updates J' and K' 63 times per quartet and lane where a call per row and an update
-// per column made 117.  The updates are what bounds the digestion: at 1.1e11 per second a group of (dp|pp) took 110k
-// of its CTA's 140k cycles.
+// per column made 117.  What bounds it is latency: with eight warps of 255 registers an SM issues in one cycle of five,
+// the warps waiting for loads of D and [e0|f0] (long scoreboard 3.7-4.3 cycles per issue) and, in (dp|ds), behind the
+// queue of updates (1.9); the updates run at 0.6-1.2e11 per second, where (pp|pp) thread-per-quartet reaches 1.9e11.
 template <class Cls, bool DET>
 struct RowSink
 {

@@ -2563,7 +2563,9 @@ void jk_team_plan(qcg_handle* h, const bool (&want)[kNumQuartetClasses], bool re
 
 // Classes from this many quartets on are evaluated in FP64 whatever the FP32 bound: their FP64 launch over every
 // quartet is faster than an FP64 and an FP32 launch that each pass over the list and skip the other's quartets
-// (four waters, 228 functions, bound 1e-7: 5.4 ms in two bands, 3.9 ms in one).
+// (four waters, 228 functions, bound 1e-7: 5.4 ms in two bands, 3.9 ms in one).  Below, two bands are no faster either
+// (bounds of 1e-9 to 1e-4: one water 147 us without a bound, 213-230 with; two 510 and 594-713; eight in a split-valence
+// basis 36.4 ms and 37.0-42.9), but cost a build at most some milliseconds, and the caller asked for FP32 evaluation.
 constexpr long long kFP32BandMaxQuartets = 1LL << 15;
 
 // fp32_below: quartets whose density-weighted bound Q_ab Q_cd max|D| (max over the six D blocks the
