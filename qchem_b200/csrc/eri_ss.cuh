@@ -4,8 +4,9 @@
 // most 36 integrals a quartet fits one thread: Y[h], the Hermite integrals summed over the ket primitives of one
 // bra primitive pair, and acc[e] = [e0|ss] stay in registers (70 + 62 for a (dd| bra), the bra contraction runs
 // once per bra primitive pair and the bra recurrence once per quartet.  (The direct form evaluated (ab|ss) per
-// primitive quartet and added it to the output block in memory: 250 000 quartets of (dd|ss) 883 us where this takes
-// 309, of (ss|ss) 265 and 208.)  What bounds it is the FP64 latency of the Boys function and the R recursion.
+// primitive quartet and added it to the output block in memory: 250 000 quartets of (dd|ss), contractions of one to
+// three, 1250 us where this takes 243, of (ss|ss) 334 and 143, sort included.)  What bounds it is the FP64 latency of the
+// Boys function and the R recursion: issue 33%, FP64 pipe 37% and 22%, eight and thirteen warps per SM.
 //
 // A warp takes 32 / SPLIT quartets, SPLIT neighbouring lanes sharing one: lane s of a quartet takes the bra
 // primitive pairs s, s + SPLIT, ..., and the lanes' acc are added by shuffles.  The ket primitive pairs of the

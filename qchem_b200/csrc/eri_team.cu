@@ -61,7 +61,8 @@ constexpr int team_pieces(int ncode, int nh, int ne)
 // CTAs per SM to compile for: twelve warps or more, as far as the registers go round and three stages each fit the
 // shared memory, of which a CTA may then use kSmemPerSM / m bytes less what it holds beside the stages.  (Nine warps in
 // one CTA, the (pp|pp) and (ds|pp) classes, wait together between the phases of a group: 250 000 quartets of
-// contraction three 1068 and 1026 us, in two CTAs 853 and 799; of contraction two 612 and 562, 466 and 413.)
+// contraction three 1068 and 1026 us, in two CTAs 853 and 799; of contraction two 612 and 562, 466 and 413.  With half the stages
+// per slot a lone group of long loops is slower: 32 quartets of contraction eight 96 and 87, 123 and 112.)
 constexpr int kSmemPerSM = 227 * 1024;
 constexpr int kSmemBeside = 2048 + (int)sizeof(BatchPlanDev) + (int)(kBoysRows * kBoysColumns * sizeof(double));
 constexpr int team_min_blocks(int ng, int stage, int regs)
