@@ -243,21 +243,21 @@ public:
         pinned_.emplace(cap, p);
     }
     // Device scratch of the team kernels (a few MiB for a small molecule, up to GiB for contracted batches), at least
-    // `bytes` and at most `budget` (>= bytes); *cap receives the capacity.  Capacities are powers of two from 1 MiB, so
+    // `bytes` and at most `room` (>= bytes); *cap receives the capacity.  Capacities are powers of two from 1 MiB, so
     // that the classes of one batch after another grow the scratch a few times at most and later handles find the same
-    // sizes idle -- or just `bytes` where the budget is smaller.  An idle buffer serves up to four times the power of
+    // sizes idle -- or just `bytes` where the room is smaller.  An idle buffer serves up to four times the power of
     // two.  Idle scratch is bounded by kScratchIdle per device; beyond it a returned buffer is freed.
     static constexpr size_t kScratchIdle = (size_t)2 << 30;
-    void* scratch(int dev, size_t bytes, size_t budget, size_t* cap)
+    void* scratch(int dev, size_t bytes, size_t room, size_t* cap)
     {
         size_t pow2 = (size_t)1 << 20;
         while (pow2 < bytes) pow2 <<= 1;
-        *cap = pow2 <= budget ? pow2 : bytes;
+        *cap = pow2 <= room ? pow2 : bytes;
         {
             std::lock_guard<std::mutex> g(mu_);
             auto& pd = per_[dev];
             auto it = pd.scratch.lower_bound(bytes);
-            if (it != pd.scratch.end() && it->first <= budget && it->first / 4 <= pow2)
+            if (it != pd.scratch.end() && it->first <= room && it->first / 4 <= pow2)
             {
                 void* p = it->second;
                 *cap = it->first;
@@ -519,9 +519,9 @@ struct qcg_handle
             }
             if (mem_limit > 0 && mem_used + (long long)bytes > mem_limit && !(need && make_room(bytes, &s == &jk_scr)))
                 throw Error{QCG_ERR_ALLOC, "device memory limit of " + std::to_string(mem_limit) + " bytes exceeded"};
-            const size_t budget = mem_limit > 0 ? (size_t)(mem_limit - mem_used) : ~(size_t)0;
+            const size_t room = mem_limit > 0 ? (size_t)(mem_limit - mem_used) : ~(size_t)0;
             size_t got = 0;   // s stays empty where there is no room
-            s.p = ResourceCache::get().scratch(device, bytes, budget, &got);
+            s.p = ResourceCache::get().scratch(device, bytes, room, &got);
             s.cap = got;
             mem_used += (long long)got;
         }
