@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         for (int k = threadIdx.x; k < 257; k += blockDim.x)
         {
             plan.first[k] = k ? nq : 0;
-            plan.group[k] = k ? (nq + 31) >> 5 : 0;
+            plan.group[k] = k ? (int)(((long long)nq + 31) >> 5) : 0;
             if (k < 256) plan.lanes[k] = 0;
         }
     __syncthreads();
@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(Cls::kNW * 32, Cls::kMinBlocks)
         // every warp reads the same quartets: lane l of every warp holds bra primitive pairs sub, sub + S, ... of its
         // quartet, S = 1 << lg
         const int lg = plan.lanes[b], sub = lane & ((1 << lg) - 1);
-        const int gi = plan.first[b] + (g - plan.group[b]) * (32 >> lg) + (lane >> lg);
+        // 64 bits: the last group of a batch of nearly 2^31 quartets reaches beyond it
+        const long long gi = plan.first[b] + (long long)(g - plan.group[b]) * (32 >> lg) + (lane >> lg);
         const bool valid = gi < plan.first[b + 1];
         const long long q = valid ? (long long)(order ? order[gi] : gi) : 0;
         if (warp == 0) lane_q[lane] = valid && sub == 0 ? (int)q : -1;
